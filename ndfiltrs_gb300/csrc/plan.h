@@ -185,6 +185,7 @@ struct Plan {
   int slide_rows = 0;        // output rows per chunk of the sliding moments kernel
   RobustArgs robust{};       // robust estimator parameters
   long long robust_threads = 0;  // threads of the scratch-backed robust kernel
+  int robust_width = 0;          // network width of the robust tile kernel (0: not used)
 
   // Host-buffer runs in overlapping row bands: built on a plan's third
   // host-buffer run (one-shot calls skip the setup), timed against the
