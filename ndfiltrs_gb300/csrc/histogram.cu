@@ -1,4 +1,4 @@
-// Sliding rank-histogram median and rank for rectangular 1-D/2-D windows
+// Rank-histogram median, rank and percentile for windows of rank 1 to 3
 // (method="histogram"; also the large-window path of "direct").
 //
 // Replaces order_statistic_into / Geometry::block / Histogram
@@ -16,19 +16,26 @@
 //    digits, warp match_any ranking for stability, digits on which every
 //    retained key agrees are skipped) through a per-block scratch slot in
 //    global memory (L2-resident); rank codes are u16 (support <= 65534);
-//  * sliding: each half-warp (16 lanes) owns a strip of output columns and
+//  * boxes: a warp selects for a patch of 32 outputs whose windows share one
+//    threshold rank (PatchWalk), at a few ranks and support rows per patch;
+//  * footprints: each half-warp (16 lanes) owns a strip of output columns and
 //    walks it in boustrophedon order, so a warp advances two windows per
-//    step; a vertical step removes one support row segment (kw codes) and
-//    adds another, spread over the 16 lanes with shared-memory atomics on the
-//    half-warp's private bitset; a selection scans 512 ranks per step from a
-//    tracked pivot (the previous window's order statistic) and ends with a
-//    5-step select in the final word. Tile widths are multiples of 32 columns,
-//    so every half-warp's columns lie inside the tile's support.
+//    step; a step removes and adds the ends of the footprint's runs, spread
+//    over the 16 lanes with shared-memory atomics on the half-warp's private
+//    bitset; a selection scans 512 ranks per step from a tracked pivot (the
+//    previous window's order statistic) and ends with a 5-step select in the
+//    final word. Tile widths are multiples of 32 columns, so every half-warp's
+//    columns lie inside the tile's support.
+// Walking every box window through a bitset of its own cost 238 warp
+// instructions per output at 65 x 65 whatever the window; patches took the
+// 65 x 65 median of a 4096^2 float32 star field from 6.59 to 3.07 ms and the
+// (9, 33, 33) median of a 64 x 512 x 512 cube from 61.2 to 33.0 ms.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <type_traits>
 
 #include "../../include/ndfiltrs_gb300.h"
 #include "common.cuh"
@@ -55,7 +62,9 @@ struct HistArgs {
   int cols_per_warp;        // columns walked by each half-warp segment
   int words;                // per-segment bit histogram: 32-bit words
   long long slot_bytes;     // scratch bytes per block slot
-  int digit_bits;           // radix digit width of the block sort (8 or 11)
+  int digit_bits;           // largest radix digit width of the block sort (8 to 11)
+  int patch_w;              // boxes: columns of a warp's patch of outputs (8 or 32)
+  unsigned int row_magic;   // ceil(2^32 / SW): row of an in-plane support index
   Reduce r;
   // Footprint windows: support-linear offsets (y * SW + x) of the taps
   // (nf), of the top and bottom ends of every vertical run of taps (nv
@@ -441,38 +450,6 @@ __device__ __forceinline__ void finish_update(SegHist& h, const StepDelta& d, bo
   __syncwarp();
 }
 
-// Remove the codes of one face and add those of another (n codes each,
-// `stride` apart, in shared memory).
-template <bool PROPAGATE>
-__device__ __forceinline__ void step(const uint16_t* codes, int remove_start, int add_start, int n,
-                                     int stride, SegHist& h) {
-  const int hl = seg_lane();
-  StepDelta d;
-  // The same trip count in every lane (lanes past the face's end update a
-  // dropped code, a no-op), so the loop never diverges.
-  const int iters = (n + kSeg - 1) / kSeg;
-  for (int it = 0, i = hl; it < iters; ++it, i += kSeg) {
-    const bool in = i < n;
-    const int rc = in ? codes[remove_start + i * stride] : (int)kOmitted;
-    const int ac = in ? codes[add_start + i * stride] : (int)kOmitted;
-    update<PROPAGATE>(h, rc, -1, d);
-    update<PROPAGATE>(h, ac, +1, d);
-  }
-  finish_update<PROPAGATE>(h, d, n <= 8 * 1024);
-}
-
-// Add every code of a kh x kw box (the first window of a segment's walk).
-template <bool PROPAGATE>
-__device__ __forceinline__ void add_box(const uint16_t* codes, int start, int kh, int kw, int SW,
-                                       SegHist& h) {
-  const int hl = seg_lane();
-  for (int ky = 0; ky < kh; ++ky) {
-    StepDelta d;
-    for (int i = hl; i < kw; i += kSeg) update<PROPAGATE>(h, codes[start + ky * SW + i], +1, d);
-    finish_update<PROPAGATE>(h, d, kw <= 8 * 1024);
-  }
-}
-
 // Footprint windows: remove the codes at rbase + rlist[i] and add those at
 // abase + alist[i] (n each).
 template <bool PROPAGATE>
@@ -625,16 +602,14 @@ struct OutPipe {
 };
 
 // A segment's boustrophedon walk over columns [c_begin, c_begin + ncols)
-// of its tile; columns at or beyond `tw_eff` are computed for convergence
-// but not stored. A window's origin is its top-left support position
-// o = row * SW + c. Rectangular windows (FP false) move whole support row or
-// column segments; footprint windows (FP true) move the run ends in `lists`:
-// down removes o + top[i] and adds o + SW + bottom[i], up removes
-// o + bottom[i] and adds o - SW + top[i], right removes o + left[i] and adds
-// o + 1 + right[i].
-template <typename T, bool PROPAGATE, bool FP>
+// of its tile (footprint windows); columns at or beyond `tw_eff` are computed
+// for convergence but not stored. A window's origin is its top-left support
+// position o = row * SW + c, and a step moves the run ends in `lists`: down
+// removes o + top[i] and adds o + SW + bottom[i], up removes o + bottom[i] and
+// adds o - SW + top[i], right removes o + left[i] and adds o + 1 + right[i].
+template <typename T, bool PROPAGATE>
 __device__ __forceinline__ void walk(const uint16_t* codes, const uint16_t* lists, int c_begin,
-                                     int ncols, int tw_eff, int th_eff, int kh, int kw, int SW,
+                                     int ncols, int tw_eff, int th_eff, int SW,
                                      long long y0, long long x0, const Geom3& g, const HistArgs& a,
                                      const typename KeyOf<T>::K* sorted, T* __restrict__ out,
                                      SegHist& h) {
@@ -642,10 +617,7 @@ __device__ __forceinline__ void walk(const uint16_t* codes, const uint16_t* list
   const uint16_t* bottom = top + a.nv;
   const uint16_t* left = bottom + a.nv;
   const uint16_t* right = left + a.nh;
-  if (FP)
-    add_taps<PROPAGATE>(codes, c_begin, lists, a.nf, h);
-  else
-    add_box<PROPAGATE>(codes, c_begin, kh, kw, SW, h);
+  add_taps<PROPAGATE>(codes, c_begin, lists, a.nf, h);
   OutPipe<T> pipe;
   int slot = 0;
   int row = 0;
@@ -662,31 +634,352 @@ __device__ __forceinline__ void walk(const uint16_t* codes, const uint16_t* list
       if (i + 1 < th_eff) {
         const int o = row * SW + c;
         if (dir > 0) {
-          if (FP)
-            step_lists<PROPAGATE>(codes, o, top, o + SW, bottom, a.nv, h);
-          else
-            step<PROPAGATE>(codes, o, o + kh * SW, kw, 1, h);
+          step_lists<PROPAGATE>(codes, o, top, o + SW, bottom, a.nv, h);
           ++row;
         } else {
-          if (FP)
-            step_lists<PROPAGATE>(codes, o, bottom, o - SW, top, a.nv, h);
-          else
-            step<PROPAGATE>(codes, o + (kh - 1) * SW, o - SW, kw, 1, h);
+          step_lists<PROPAGATE>(codes, o, bottom, o - SW, top, a.nv, h);
           --row;
         }
       }
     }
     if (j + 1 < ncols) {
       const int o = row * SW + c;
-      if (FP)
-        step_lists<PROPAGATE>(codes, o, left, o + 1, right, a.nh, h);
-      else
-        step<PROPAGATE>(codes, o, o + kw, kh, SW, h);
+      step_lists<PROPAGATE>(codes, o, left, o + 1, right, a.nh, h);
     }
     dir = -dir;
   }
   pipe.rotate(a, sorted, out);
   pipe.complete(a, out);
+}
+
+// ---------------------------------------------------------------------------
+// Box windows (1-D to 3-D): a warp selects for a patch of 32 outputs at once.
+//
+// The 32 windows of a patch overlap almost entirely, so their order statistics
+// lie close together among the tile's ranks. The warp keeps one threshold rank
+// t near them. Each lane knows how many samples of its window rank below t,
+// and reads its order statistic off the ranks around t, which every lane looks
+// through together:
+//  * counts: a support row becomes one bit per sample (code < t) by ballots;
+//    a lane's share of the row is a shifted, masked popcount. When the patch
+//    moves down by its height the rows that leave and enter are counted, or
+//    all rows when those are fewer;
+//  * ranks: lane i takes the sample of rank r + i and works out which of the
+//    32 windows hold it (a mask of lanes). The 32 x 32 bits are transposed in
+//    five shuffle stages, after which lane L has the word of the 32 ranks that
+//    its own window holds: a popcount advances its count and the word that
+//    reaches its order statistic is kept and searched once at the end.
+// The work per output is the rows' ballots over 32 outputs plus the rank
+// distance between the patch's least and largest result, instead of the
+// window's faces per output and a walk through a private bitset (16 lanes a
+// window). A patch of 8 x 4 outputs keeps that distance short on slopes; rows
+// of 32 x 1 serve single-row tiles and deep (3-D) windows, where counting rows
+// costs more than looking through ranks.
+
+// Bits [lo, lo + width) of a word; lo and width at least 0.
+__device__ __forceinline__ unsigned int bit_run(int lo, int width) {
+  unsigned int m;
+  asm("bmsk.clamp.b32 %0, %1, %2;" : "=r"(m) : "r"(lo), "r"(width));
+  return m;
+}
+
+// Transpose of the 32 x 32 bit matrix whose row i lane i holds: five exchanges
+// of halves. Moving the other lane's half into place is a byte permute for the
+// first two and a rotation for the rest; what a lane keeps follows from its
+// number, so the constants are made once.
+struct Transpose {
+  unsigned int bytes16, bytes8;    // __byte_perm selectors
+  unsigned int rot4, rot2, rot1;   // left rotations
+  unsigned int keep4, keep2, keep1;
+
+  __device__ __forceinline__ Transpose() {
+    const unsigned int lane = threadIdx.x & 31;
+    bytes16 = lane & 16 ? 0x3276u : 0x5410u;
+    bytes8 = lane & 8 ? 0x3715u : 0x6240u;
+    rot4 = lane & 4 ? 28 : 4;
+    rot2 = lane & 2 ? 30 : 2;
+    rot1 = lane & 1 ? 31 : 1;
+    keep4 = lane & 4 ? 0xF0F0F0F0u : 0x0F0F0F0Fu;
+    keep2 = lane & 2 ? 0xCCCCCCCCu : 0x33333333u;
+    keep1 = lane & 1 ? 0xAAAAAAAAu : 0x55555555u;
+  }
+  __device__ __forceinline__ static unsigned int swap(unsigned int x, int j, unsigned int rot, unsigned int keep) {
+    const unsigned int y = __shfl_xor_sync(kFull, x, j);
+    return (x & keep) | (__funnelshift_l(y, y, rot) & ~keep);
+  }
+  __device__ __forceinline__ unsigned int operator()(unsigned int x) const {
+    x = __byte_perm(x, __shfl_xor_sync(kFull, x, 16), bytes16);
+    x = __byte_perm(x, __shfl_xor_sync(kFull, x, 8), bytes8);
+    x = swap(x, 4, rot4, keep4);
+    x = swap(x, 2, rot2, keep2);
+    return swap(x, 1, rot1, keep1);
+  }
+};
+
+template <typename T, int PW, bool DROPS>
+struct PatchWalk {
+  using K = typename KeyOf<T>::K;
+  static constexpr int PH = 32 / PW;
+
+  const HistArgs& a;
+  const uint16_t* codes;  // rank of each support sample (or a dropped code)
+  const uint16_t* place;  // in-plane support index of each rank (65535 up to 32 before and after)
+  const K* sorted;
+  int lx, ly;             // the lane's output within the patch
+  int px, py;             // the patch's first column and row in the tile
+  int t;                  // threshold rank
+  int below, dropped;     // the lane's window: samples of rank below t, dropped samples
+  Transpose transpose;
+
+  // Add to the lane's counts those of two support rows (its kw columns from
+  // px + lx), negated for the first if FLIP; `first` and `second` say whether
+  // the rows lie in (or leave and enter) the lane's window. `row` is the first
+  // one's start, the second lies `apart` codes further.
+  template <bool FLIP>
+  __device__ __forceinline__ void add_rows(const uint16_t* row, int apart, bool first, bool second) {
+    const uint16_t* at = row + px + (threadIdx.x & 31);
+    int u = at[0], v = at[apart];
+    unsigned int a0 = __ballot_sync(kFull, u < t), b0 = __ballot_sync(kFull, v < t), c0 = 0, d0 = 0;
+    if (DROPS) {
+      c0 = __ballot_sync(kFull, u >= (int)kPropagated);
+      d0 = __ballot_sync(kFull, v >= (int)kPropagated);
+    }
+    int na = 0, nb = 0, nc = 0, nd = 0;
+    int left = a.g.kw;
+#pragma unroll 1
+    for (; left >= 32; left -= 32) {
+      at += 32;
+      u = at[0];
+      v = at[apart];
+      const unsigned int a1 = __ballot_sync(kFull, u < t), b1 = __ballot_sync(kFull, v < t);
+      na += __popc(__funnelshift_r(a0, a1, lx));
+      nb += __popc(__funnelshift_r(b0, b1, lx));
+      a0 = a1;
+      b0 = b1;
+      if (DROPS) {
+        const unsigned int c1 = __ballot_sync(kFull, u >= (int)kPropagated);
+        const unsigned int d1 = __ballot_sync(kFull, v >= (int)kPropagated);
+        nc += __popc(__funnelshift_r(c0, c1, lx));
+        nd += __popc(__funnelshift_r(d0, d1, lx));
+        c0 = c1;
+        d0 = d1;
+      }
+    }
+    if (left > 0) {
+      const unsigned int mask = (1u << left) - 1u;
+      unsigned int a1 = 0, b1 = 0, c1 = 0, d1 = 0;
+      if (left + PW - 1 > 32) {
+        u = at[32];
+        v = at[apart + 32];
+        a1 = __ballot_sync(kFull, u < t);
+        b1 = __ballot_sync(kFull, v < t);
+        if (DROPS) {
+          c1 = __ballot_sync(kFull, u >= (int)kPropagated);
+          d1 = __ballot_sync(kFull, v >= (int)kPropagated);
+        }
+      }
+      na += __popc(__funnelshift_r(a0, a1, lx) & mask);
+      nb += __popc(__funnelshift_r(b0, b1, lx) & mask);
+      if (DROPS) {
+        nc += __popc(__funnelshift_r(c0, c1, lx) & mask);
+        nd += __popc(__funnelshift_r(d0, d1, lx) & mask);
+      }
+    }
+    below += (second ? nb : 0) + (first ? (FLIP ? -na : na) : 0);
+    if (DROPS) dropped += (second ? nd : 0) + (first ? (FLIP ? -nc : nc) : 0);
+  }
+
+  // Count the whole windows, two rows at a time (the row after the last is
+  // read but lies in no window; it ends within the places that follow).
+  __device__ __forceinline__ void count_all() {
+    below = dropped = 0;
+    for (int z = 0; z < a.g.kd; ++z) {
+      const uint16_t* row = codes + z * a.plane + py * a.SW;
+      for (int q = 0; q < a.g.kh + PH - 1; q += 2, row += 2 * a.SW)
+        add_rows<false>(row, a.SW, (unsigned)(q - ly) < (unsigned)a.g.kh, (unsigned)(q + 1 - ly) < (unsigned)a.g.kh);
+    }
+  }
+
+  // Move the windows down by the patch height.
+  __device__ __forceinline__ void move_down() {
+    for (int z = 0; z < a.g.kd; ++z) {
+      const uint16_t* row = codes + z * a.plane + py * a.SW;
+#pragma unroll 1
+      for (int q = 0; q < 2 * PH - 1; ++q, row += a.SW) {
+        const bool mine = PH == 1 || (unsigned)(q - ly) < (unsigned)PH;
+        add_rows<true>(row, a.g.kh * a.SW, mine, mine);
+      }
+    }
+    py += PH;
+  }
+
+  // Which of the ranks [start, start + 32) the lane's window holds (bit i:
+  // rank start + i). Ranks outside the support are in no window.
+  __device__ __forceinline__ unsigned int ranks_in(int start) const {
+    const unsigned int e = place[start + (int)(threadIdx.x & 31)];
+    const int sy = (int)__umulhi(e, a.row_magic);
+    const int dx = (int)e - sy * a.SW - px, dy = sy - py;
+    const bool in = (unsigned)dx < (unsigned)(a.g.kw + PW - 1) && (unsigned)dy < (unsigned)(a.g.kh + PH - 1);
+    if (!__any_sync(kFull, in)) return 0u;
+    unsigned int lanes = 0;
+    if (in) {
+      // Columns dx - kw + 1 .. dx and rows dy - kh + 1 .. dy of the patch.
+      const int cl = max(dx - a.g.kw + 1, 0), ch = min(dx, PW - 1);
+      lanes = bit_run(cl, ch - cl + 1);
+      if (PH > 1) {
+        lanes *= PW == 8 ? 0x01010101u : PW == 16 ? 0x00010001u : 1u;
+        const int rl = max(dy - a.g.kh + 1, 0), rh = min(dy, PH - 1);
+        lanes &= bit_run(rl * PW, (rh - rl + 1) * PW);
+      }
+    }
+    return transpose(lanes);
+  }
+
+  // Move the threshold to rank `to` (the counts follow).
+  __device__ __forceinline__ void move_threshold(int to) {
+    const int lo = min(t, to), hi = max(t, to);
+    int count = 0;
+    for (int start = lo; start < hi; start += 32) count += __popc(ranks_in(start) & bit_run(0, hi - start));
+    below += to > t ? count : -count;
+    t = to;
+  }
+
+  // The patch's order statistics: which ranks, and whether there is a value.
+  // Lanes outside the image (`live` false) ask for nothing.
+  __device__ __forceinline__ Ranks select(bool live) {
+    const Reduce& r = a.r;
+    Ranks o;
+    const int volume = a.g.kd * a.g.kh * a.g.kw;
+    o.n = volume - dropped;
+    o.valid = live && !((!r.omit && dropped > 0) || (r.omit && o.n < r.min_count) || o.n == 0);
+    int k1 = 0, k2;
+    switch (r.kind) {
+      case kRank:
+      case kRankHistogram:
+        o.valid = o.valid && r.param < o.n;
+        k1 = o.valid ? (int)r.param : 0;
+        break;
+      case kMin:
+        break;
+      case kMax:
+        k1 = o.n - 1;
+        break;
+      case kPercentile:
+        if (r.q_is_max) {
+          k1 = o.n - 1;
+        } else {
+          const PctSplit ps = pct_split(r, max(o.n, 1));
+          k1 = ps.lower;
+          o.two = ps.upper != ps.lower;
+        }
+        break;
+      default:
+        o.two = (o.n & 1) == 0;
+        k1 = o.two ? o.n / 2 - 1 : o.n / 2;
+    }
+    k2 = k1 + (o.two ? 1 : 0);
+    // The word that holds order statistic k starts at rank s and has it as
+    // its k'-th set bit.
+    int s1 = 0, s2 = 0, i1 = 0, i2 = 0;
+    unsigned int w1 = 0, w2 = 0;
+    const bool pairs = __any_sync(kFull, o.two);
+    // Lanes without a value wait for nothing and find nothing.
+    k1 = o.valid ? k1 : -1;
+    k2 = o.valid ? k2 : -1;
+    const int least = o.valid ? k1 : INT_MAX;
+    auto look = [&](int start, int base, unsigned int word, int count) {
+      if ((unsigned)(k1 - base) < (unsigned)count) {
+        s1 = start;
+        i1 = k1 - base;
+        w1 = word;
+      }
+      if (pairs && (unsigned)(k2 - base) < (unsigned)count) {
+        s2 = start;
+        i2 = k2 - base;
+        w2 = word;
+      }
+    };
+    int base = below;
+    for (int start = t; __any_sync(kFull, k2 >= base) && start < a.S; start += 32) {
+      const unsigned int word = ranks_in(start);
+      const int count = __popc(word);
+      look(start, base, word, count);
+      base += count;
+    }
+    base = below;
+    for (int start = t; __any_sync(kFull, least < base) && start > 0;) {
+      start -= 32;
+      const unsigned int word = ranks_in(start);
+      const int count = __popc(word);
+      base -= count;
+      look(start, base, word, count);
+    }
+    o.lo = s1 + select_in_word32(w1, i1);
+    o.hi = o.two ? s2 + select_in_word32(w2, i2) : o.lo;
+    return o;
+  }
+
+  // Walk patches down the tile's rows [row0, row1) of the columns from px.
+  __device__ __forceinline__ void walk(int row0, int row1, int tw_eff, int th_eff, T* __restrict__ out,
+                                       long long at0) {
+    // Counting whole windows costs kh + PH - 1 rows a plane, moving them
+    // 2 (2 PH - 1).
+    const bool recount = a.g.kh + PH - 1 <= 2 * (2 * PH - 1);
+    py = row0;
+    Ranks held;
+    K kl = 0, kh = 0;
+    long long held_at = -1;
+    for (;;) {
+      if (py == row0 || recount) count_all();
+      const bool live = px + lx < tw_eff && py + ly < th_eff;
+      const Ranks o = select(live);
+      // The previous patch's keys have arrived by now.
+      if (held_at >= 0) out[held_at] = canonical(hist_value<T>(held, a, kl, kh));
+      held = o;
+      held_at = live ? at0 + (long long)(py + ly) * a.g.W + px + lx : -1;
+      if (o.valid) {
+        kl = sorted[o.lo];
+        kh = o.two ? sorted[o.hi] : kl;
+      }
+      const int next = py + PH;
+      const int least = __reduce_min_sync(kFull, o.valid ? o.lo : INT_MAX);
+      const int most = __reduce_max_sync(kFull, o.valid ? o.hi : -1);
+      if (next >= row1) {
+        if (most >= 0) t = (least + most) >> 1;
+        break;
+      }
+      if (recount) {
+        if (most >= 0) t = (least + most) >> 1;
+        py = next;
+      } else {
+        if (most >= 0 && (t < least || t > most)) move_threshold((least + most) >> 1);
+        move_down();
+      }
+    }
+    if (held_at >= 0) out[held_at] = canonical(hist_value<T>(held, a, kl, kh));
+  }
+};
+
+// Every patch column of a tile: columns of patches split into runs of rows so
+// that the block's warps all have work.
+template <typename T, int PW, bool DROPS>
+__device__ __forceinline__ void walk_patches(const HistArgs& a, const uint16_t* codes, const uint16_t* place,
+                                             const typename KeyOf<T>::K* sorted, int nret, int tw_eff,
+                                             int th_eff, T* __restrict__ out, long long at0) {
+  constexpr int PH = 32 / PW;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int columns = (tw_eff + PW - 1) / PW, rows = (th_eff + PH - 1) / PH;
+  const int runs = min(rows, max(1, kHWarps / columns));
+  PatchWalk<T, PW, DROPS> p{a, codes, place, sorted, lane % PW, lane / PW, 0, 0, 0, 0, 0};
+  const Reduce& r = a.r;
+  p.t = r.kind == kMin ? 0 : r.kind == kMax ? nret : r.kind == kPercentile ? (int)(nret * r.q_fraction) : nret / 2;
+  if (r.kind == kRank || r.kind == kRankHistogram)
+    p.t = (int)min((long long)nret, r.param * nret / max(1, a.g.kd * a.g.kh * a.g.kw));
+  for (int item = warp; item < columns * runs; item += kHWarps) {
+    const int run = item / columns;
+    p.px = (item - run * columns) * PW;
+    p.walk(rows * run / runs * PH, rows * (run + 1) / runs * PH, tw_eff, th_eff, out, at0);
+  }
 }
 
 // One output tile (index `tile` of the plan's tile list) of the sliding
@@ -702,18 +995,19 @@ __device__ __forceinline__ void histogram_tile(const T* __restrict__ in, T* __re
   __shared__ int red_sent[kHWarps];
   const Geom3& g = a.g;
   const int S = a.S;
-  // Shared memory: rank codes [S] u16 | footprint lists (FP) | decode table
+  // Shared memory. Footprints: rank codes [S] u16 | run lists | decode table
   // [S] keys (SDEC) | work (radix tables during the sort, half-warp
-  // histograms while sliding).
+  // histograms while sliding). Boxes: rank codes [S + 32] u16 (patches read up
+  // to 32 codes past a row's end) | places of the ranks [32 + S + 32] u16 (no
+  // window holds the outer ones) | decode table (SDEC); the radix tables use the same bytes before those are written.
   uint16_t* codes_s = reinterpret_cast<uint16_t*>(smem);
-  const long long list_bytes = FP ? align16((long long)(a.nf + 2 * a.nv + 2 * a.nh) * 2) : 0;
-  uint16_t* lists_s = reinterpret_cast<uint16_t*>(smem + align16((long long)a.S * 2));
-  K* decode_s = reinterpret_cast<K*>(smem + align16((long long)a.S * 2) + list_bytes);
+  const long long list_bytes = FP ? align16((long long)(a.nf + 2 * a.nv + 2 * a.nh) * 2) : align16((long long)(a.S + 64) * 2);
+  const long long code_bytes = align16((long long)(FP ? a.S : a.S + 32) * 2);
+  uint16_t* lists_s = reinterpret_cast<uint16_t*>(smem + code_bytes);
+  uint16_t* place_s = lists_s + 32;
+  K* decode_s = reinterpret_cast<K*>(smem + code_bytes + list_bytes);
   unsigned int* work = reinterpret_cast<unsigned int*>(
-      smem + align16((long long)a.S * 2) + list_bytes + (SDEC ? align16((long long)a.S * sizeof(K)) : 0));
-  const int nd = 1 << a.digit_bits;
-  unsigned int* table = work;
-  unsigned int* totals = work + kHWarps * nd;
+      FP ? smem + code_bytes + list_bytes + (SDEC ? align16((long long)a.S * sizeof(K)) : 0) : smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   Slot<K> slot = slot_at<K>(scratch_slot, S);
   const unsigned long long keep = keep_policy();
@@ -723,20 +1017,33 @@ __device__ __forceinline__ void histogram_tile(const T* __restrict__ in, T* __re
   const long long tyx = tile - z * a.tiles_yx;
   const long long y0 = (tyx / a.tiles_x) * a.TH;
   const long long x0 = (tyx % a.tiles_x) * a.TW;
-  // Gather the support as keys (payload = support index), mapping each
-  // coordinate through the boundary modes.
+  // Gather the support as keys (payload = support index): each coordinate is
+  // mapped through its axis's boundary mode once, into a table in the shared
+  // memory that the sort's counters use afterwards; rows go to warps.
   K k_and = kSent, k_or = 0;
   int sent = 0;
-  for (int e = threadIdx.x; e < S; e += blockDim.x) {
-    const int sz = e / a.plane;
-    const int ep = e - sz * a.plane;
-    const int sy = ep / a.SW;
-    const int sx = ep - sy * a.SW;
-    long long mz, my, mx;
-    const bool inside = map_index(z + sz - g.az, g.D, g.mz, &mz) &&
-                        map_index(y0 + sy - g.ay, g.H, g.my, &my) &&
-                        map_index(x0 + sx - g.ax, g.W, g.mx, &mx);
-    const K key = inside ? sample_key<T>(__ldcs(in + (mz * g.H + my) * g.W + mx), drop_inf) : outside;
+  // (A single row maps its columns as it goes: a table of 64-bit offsets for
+  // it would not fit. For two rows or more the tables take at most the 4 S
+  // bytes that both layouts have there.)
+  const int rows = g.kd * a.SH;
+  long long* row_map = reinterpret_cast<long long*>(work);
+  long long* column_map = row_map + a.SH + g.kd;
+  auto column = [&](int sx) -> long long {
+    long long m;
+    return map_index(x0 + sx - g.ax, g.W, g.mx, &m) ? m : -1;
+  };
+  for (int i = threadIdx.x; i < a.SH + g.kd + (rows > 1 ? a.SW : 0); i += blockDim.x) {
+    long long m;
+    if (i < a.SH)
+      row_map[i] = map_index(y0 + i - g.ay, g.H, g.my, &m) ? m * g.W : -1;
+    else if (i < a.SH + g.kd)
+      row_map[i] = map_index(z + (i - a.SH) - g.az, g.D, g.mz, &m) ? m * g.H * g.W : -1;
+    else
+      column_map[i - a.SH - g.kd] = column(i - a.SH - g.kd);
+  }
+  __syncthreads();
+  auto take = [&](int e, bool inside, const T* src) {
+    const K key = inside ? sample_key<T>(__ldcs(src), drop_inf) : outside;
     st_keep(slot.keys_a + e, key, keep);
     st_keep(slot.pay_a + e, (uint16_t)e, keep);
     if (key != kSent) {
@@ -744,6 +1051,25 @@ __device__ __forceinline__ void histogram_tile(const T* __restrict__ in, T* __re
       k_or |= key;
     } else {
       ++sent;
+    }
+  };
+  if (rows == 1) {
+    const bool inside = row_map[0] >= 0 && row_map[1] >= 0;
+    const T* src = in + (inside ? row_map[0] + row_map[1] : 0);
+    for (int sx = threadIdx.x; sx < a.SW; sx += blockDim.x) {
+      const long long ox = column(sx);
+      take(sx, inside && ox >= 0, src + ox);
+    }
+  } else {
+    for (int row = warp; row < rows; row += kHWarps) {
+      const int sz = g.kd > 1 ? row / a.SH : 0;
+      const long long oy = row_map[row - sz * a.SH], oz = row_map[a.SH + sz];
+      const bool inside = oy >= 0 && oz >= 0;
+      const T* src = in + (inside ? oy + oz : 0);
+      for (int sx = lane; sx < a.SW; sx += 32) {
+        const long long ox = column_map[sx];
+        take(row * a.SW + sx, inside && ox >= 0, src + ox);
+      }
     }
   }
   for (int o = 16; o >= 1; o >>= 1) {
@@ -778,9 +1104,13 @@ __device__ __forceinline__ void histogram_tile(const T* __restrict__ in, T* __re
     const int bits = (int)sizeof(K) * 8;
     const int lo = sizeof(K) == 8 ? __ffsll((long long)varying) - 1 : __ffs((int)varying) - 1;
     const int hi = bits - 1 - (sizeof(K) == 8 ? __clzll((long long)varying) : __clz((int)varying));
+    // The fewest passes, with the smallest digits that still cover the bits.
+    const int passes = (hi - lo + a.digit_bits) / a.digit_bits;
+    const int digits = max(5, (hi - lo + passes) / passes);
+    const int nd = 1 << digits;
     const K mask = (K)(nd - 1);
-    for (int shift = lo; shift <= hi; shift += a.digit_bits) {
-      radix_pass(src_k, src_p, dst_k, dst_p, S, table, totals, nd,
+    for (int shift = lo; shift <= hi; shift += digits) {
+      radix_pass(src_k, src_p, dst_k, dst_p, S, work, work + kHWarps * nd, nd,
                  [shift, mask](K key) { return (unsigned int)((key >> shift) & mask); }, keep);
       K* tk = src_k;
       src_k = dst_k;
@@ -793,37 +1123,56 @@ __device__ __forceinline__ void histogram_tile(const T* __restrict__ in, T* __re
   const uint16_t dropped = a.r.omit ? kOmitted : kPropagated;
   for (int pos = threadIdx.x; pos < S; pos += blockDim.x) {
     const K key = ld_keep(src_k + pos, keep);
-    codes_s[ld_keep(src_p + pos, keep)] = key == kSent ? dropped : (uint16_t)pos;
+    const uint16_t at = ld_keep(src_p + pos, keep);
+    codes_s[at] = key == kSent ? dropped : (uint16_t)pos;
+    // A dropped sample (its key can tie with the largest retained one's sorted
+    // bits) lies in no window: place 65535 is below the support's last row.
+    if (!FP) place_s[pos] = key == kSent ? (uint16_t)0xFFFF : (uint16_t)(g.kd > 1 ? at % a.plane : at);
     if (SDEC) decode_s[pos] = key;
   }
+  if (!FP && threadIdx.x < 64) lists_s[threadIdx.x < 32 ? (int)threadIdx.x : S + (int)threadIdx.x] = 0xFFFF;
   __syncthreads();
   const K* sorted = SDEC ? decode_s : src_k;
-
-  // Slide: each half-warp walks its columns in boustrophedon order.
   const int th_eff = (int)min((long long)a.TH, g.H - y0);
   const int tw_eff = (int)min((long long)a.TW, g.W - x0);
-  const int seg = threadIdx.x / kSeg;
-  SegHist h;
-  h.words = work + seg * a.words;
-  h.nwords = a.words;
-  h.m = 0;
-  h.lt = 0;
-  h.count = 0;
-  h.nan = 0;
-  for (int i = seg_lane(); i < a.words; i += kSeg) h.words[i] = 0u;
-  __syncwarp();
-  const int kh = g.kh, kw = g.kw, SW = a.SW;
-  // Both halves of a warp have columns iff the warp's first column is in
-  // the tile's valid width; whole warps beyond it sit out.
-  const int warp_first = (threadIdx.x / 32) * 2 * a.cols_per_warp;
   T* plane_out = out + z * g.H * g.W;
-  if (warp_first < tw_eff) {
-    if (!a.r.omit)
-      walk<T, true, FP>(codes_s, lists_s, seg * a.cols_per_warp, a.cols_per_warp, tw_eff, th_eff, kh,
-                        kw, SW, y0, x0, g, a, sorted, plane_out, h);
+  if constexpr (!FP) {
+    const long long at0 = y0 * g.W + x0;
+    auto walk_all = [&](auto width, auto drops) {
+      walk_patches<T, decltype(width)::value, decltype(drops)::value>(a, codes_s, place_s, sorted, S - sent, tw_eff,
+                                                                      th_eff, plane_out, at0);
+    };
+    using Yes = std::true_type;
+    using No = std::false_type;
+    using P8 = std::integral_constant<int, 8>;
+    using P32 = std::integral_constant<int, 32>;
+    if (a.patch_w == 8)
+      sent > 0 ? walk_all(P8{}, Yes{}) : walk_all(P8{}, No{});
     else
-      walk<T, false, FP>(codes_s, lists_s, seg * a.cols_per_warp, a.cols_per_warp, tw_eff, th_eff, kh,
-                         kw, SW, y0, x0, g, a, sorted, plane_out, h);
+      sent > 0 ? walk_all(P32{}, Yes{}) : walk_all(P32{}, No{});
+  } else {
+    // Slide: each half-warp walks its columns in boustrophedon order.
+    const int seg = threadIdx.x / kSeg;
+    SegHist h;
+    h.words = work + seg * a.words;
+    h.nwords = a.words;
+    h.m = 0;
+    h.lt = 0;
+    h.count = 0;
+    h.nan = 0;
+    for (int i = seg_lane(); i < a.words; i += kSeg) h.words[i] = 0u;
+    __syncwarp();
+    // Both halves of a warp have columns iff the warp's first column is in
+    // the tile's valid width; whole warps beyond it sit out.
+    const int warp_first = (threadIdx.x / 32) * 2 * a.cols_per_warp;
+    if (warp_first < tw_eff) {
+      if (!a.r.omit)
+        walk<T, true>(codes_s, lists_s, seg * a.cols_per_warp, a.cols_per_warp, tw_eff, th_eff, a.SW, y0, x0, g, a,
+                      sorted, plane_out, h);
+      else
+        walk<T, false>(codes_s, lists_s, seg * a.cols_per_warp, a.cols_per_warp, tw_eff, th_eff, a.SW, y0, x0, g, a,
+                       sorted, plane_out, h);
+    }
   }
   __syncthreads();
 }
@@ -837,7 +1186,7 @@ __device__ __forceinline__ void load_lists(const HistArgs& a, unsigned char* sme
 }
 
 template <typename T, bool SDEC, bool FP>
-__global__ void __launch_bounds__(kHThreads, 1)
+__global__ void __launch_bounds__(kHThreads, FP ? 1 : 2)
     histogram_kernel(const T* __restrict__ in, T* __restrict__ out, const __grid_constant__ HistArgs a,
                      unsigned char* scratch) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -859,7 +1208,7 @@ struct HistTask {
 };
 
 template <bool SDEC, bool FP>
-__global__ void __launch_bounds__(kHThreads, 1)
+__global__ void __launch_bounds__(kHThreads, FP ? 1 : 2)
     histogram_family_kernel(const HistTask* __restrict__ tasks, int ntasks, long long total_tiles,
                             unsigned char* scratch, long long slot_bytes) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -910,7 +1259,7 @@ struct Runs {
   int entries() const { return footprint ? nf + 2 * nv + 2 * nh : 0; }
 };
 
-// Bytes of the work region (the sort's 8-bit-digit tables, or the
+// Footprints: bytes of the work region (the sort's 8-bit-digit tables, or the
 // segments' bit histograms while sliding, whichever is larger).
 size_t work_bytes_for(int S) {
   const size_t sort = (size_t)sort_table_words(256) * 4;
@@ -918,15 +1267,21 @@ size_t work_bytes_for(int S) {
   return std::max(sort, hist);
 }
 
-// The sort uses 11-bit digits (three passes cover 32 varying bits) when
-// their tables fit in the work region, else 8-bit digits.
-int digit_bits_for(int S) { return work_bytes_for(S) >= (size_t)sort_table_words(2048) * 4 ? 11 : 8; }
+size_t smem_bytes_for(int S, bool sdec, size_t key_bytes, const Runs& runs) {
+  const size_t codes = (size_t)align16((long long)(runs.footprint ? S : S + 32) * 2);
+  const size_t lists = (size_t)align16((long long)(runs.footprint ? runs.entries() : S + 64) * 2);
+  const size_t decode = sdec ? (size_t)align16((long long)S * (long long)key_bytes) : 0;
+  if (runs.footprint) return codes + lists + decode + work_bytes_for(S);
+  return std::max(codes + lists + decode, (size_t)sort_table_words(256) * 4);
+}
 
-size_t smem_bytes_for(int S, bool sdec, size_t key_bytes, int list_entries) {
-  size_t codes = (size_t)align16((long long)S * 2);
-  size_t lists = (size_t)align16((long long)list_entries * 2);
-  size_t decode = sdec ? (size_t)align16((long long)S * (long long)key_bytes) : 0;
-  return codes + lists + decode + work_bytes_for(S);
+// The sort takes digits of up to 11 bits (three passes cover 32 varying bits)
+// as far as their tables fit in the bytes they share.
+int digit_bits_for(int S, bool sdec, size_t key_bytes, const Runs& runs) {
+  const size_t room = runs.footprint ? work_bytes_for(S) : smem_bytes_for(S, sdec, key_bytes, runs);
+  int bits = 8;
+  while (bits < 11 && (size_t)sort_table_words(2 << bits) * 4 <= room) ++bits;
+  return bits;
 }
 
 // Count the taps and the vertical and horizontal runs (within each plane)
@@ -946,35 +1301,62 @@ Runs count_runs(const std::vector<uint8_t>& mask, int kd, int kh, int kw) {
   return r;
 }
 
-// Pick the output tile by a cost model in units of one histogram update per
-// output: vertical steps (2 kw), the first window of each warp's walk, the
-// column moves, the block sort (about 8 units per support sample) and a
-// global decode when the sorted keys do not fit in shared memory.
-// The tile of a sliding-histogram plan: by the cost model, or the given
-// tw x th when it fits (an autotuner candidate; 0 when it does not).
+// The patch width of a box window's tile of height th: rows of 32 outputs
+// where a tile has single rows or a window has planes (counting the 2 PH - 1
+// rows that a patch of height PH leaves and enters per plane costs more there
+// than looking through the ranks that a wider patch spreads over).
+int patch_width(const Geom3& g, int th) { return th % 4 != 0 || g.kd > 1 ? 32 : 8; }
+
+// Work per output of a box window's tile in warp instructions: the block sort
+// of the support, the rows counted per patch, and the ranks looked through,
+// which grow with the support over the window and with the spread of the
+// patch's order statistics (that of windows shifted across the patch, for
+// independent samples).
+double box_cost(const Geom3& g, int tw, int th, double S, bool sdec) {
+  const int pw = patch_width(g, th), ph = 32 / pw;
+  const double outputs = (double)tw * th, volume = (double)g.kd * g.kh * g.kw;
+  const double words = (g.kw + pw - 1 + 31) / 32;
+  const double row = 8.0 * words + 8.0;
+  const double all = (double)g.kd * (g.kh + ph - 1), moved = (double)g.kd * 2 * (2 * ph - 1);
+  const double columns = tw / pw, runs = std::max(1.0, kHWarps / columns);
+  const double steps = std::max(1.0, th / ph / runs);
+  const double rows = std::min(all, moved + all / steps) * row;
+  const double moves = std::min(std::sqrt(0.5 * g.kd * ((double)g.kh * (pw - 1) + (double)g.kw * (ph - 1))),
+                                1.5 * std::sqrt(0.25 * volume) * 2.0);
+  const double ranks = std::min(S, 1.6 * moves * S / volume);
+  const double idle = std::max(1.0, kHWarps / (columns * std::min(runs, (double)th / ph)));
+  return 6.0 * S / outputs + idle * (rows + 45.0 * (ranks / 32.0 + 2.0) + 120.0) / 32.0 + (sdec ? 0.0 : 0.5);
+}
+
+// Pick the output tile by a cost model: for boxes box_cost; for footprints in
+// units of one histogram update per output: vertical steps, the first window
+// of each segment's walk, the column moves, the block sort (about 8 units per
+// support sample) and a global decode when the sorted keys do not fit in
+// shared memory. Or the given tw x th when it fits (an autotuner candidate; 0
+// when it does not).
 HistChoice choose_tile(const Geom3& g, size_t key_bytes, const Runs& runs = Runs{}, int force_tw = 0,
                        int force_th = 0) {
   HistChoice best;
   if ((long long)g.kw > kMaxSupport || (long long)g.kh > kMaxSupport || (long long)g.kd > kMaxSupport)
     return best;
-  // Windows deeper than one plane walk their (kd-plane) faces through the
-  // run lists.
-  if (g.kd > 1 && !runs.footprint) return best;
   double best_cost = 1e300;
   auto consider = [&](int tw, int th) {
     long long S = (long long)g.kd * (tw + g.kw - 1) * (th + g.kh - 1);
     if (S > kMaxSupport) return;
     for (int sdec = 1; sdec >= 0; --sdec) {
-      size_t smem = smem_bytes_for((int)S, sdec != 0, key_bytes, runs.entries());
+      size_t smem = smem_bytes_for((int)S, sdec != 0, key_bytes, runs);
       if (smem > kSmemBudget) continue;
-      const double cpw = (tw + kSegs - 1) / kSegs;
-      const double outputs = (double)tw * th;
-      const double vertical = runs.footprint ? runs.nv : g.kw;
-      const double horizontal = runs.footprint ? runs.nh : g.kh;
-      const double taps = runs.footprint ? runs.nf : (double)g.kh * g.kw;
-      double cost = 2.0 * vertical + taps / (cpw * th) + 2.0 * horizontal / th +
-                    8.0 * (double)S / outputs + (sdec ? 0.0 : 12.0);
-      if (smem * 2 <= kSmemBudget) cost *= 0.9;  // two resident blocks per SM
+      double cost;
+      if (runs.footprint) {
+        const double cpw = (tw + kSegs - 1) / kSegs;
+        const double outputs = (double)tw * th;
+        cost = 2.0 * runs.nv + runs.nf / (cpw * th) + 2.0 * runs.nh / th + 8.0 * (double)S / outputs +
+               (sdec ? 0.0 : 12.0);
+        if (smem * 2 <= kSmemBudget) cost *= 0.9;  // two resident blocks per SM
+      } else {
+        cost = box_cost(g, tw, th, (double)S, sdec != 0);
+        if (smem * 2 <= kSmemBudget) cost *= 0.8;  // two resident blocks per SM
+      }
       if (cost < best_cost) {
         best_cost = cost;
         best.TW = tw;
@@ -982,7 +1364,7 @@ HistChoice choose_tile(const Geom3& g, size_t key_bytes, const Runs& runs = Runs
         best.sdec = sdec != 0;
         best.smem = smem;
       }
-      return;
+      if (runs.footprint) return;
     }
   };
   if (force_tw > 0) {
@@ -1004,7 +1386,7 @@ HistChoice choose_tile(const Geom3& g, size_t key_bytes, const Runs& runs = Runs
   return best;
 }
 
-HistArgs make_args_core(const Geom3& g, int TW, int TH, int dtype, const Reduce& r) {
+HistArgs make_args_core(const Geom3& g, int TW, int TH, int dtype, bool sdec, const Runs& runs, const Reduce& r) {
   HistArgs a{};
   a.g = g;
   a.TW = TW;
@@ -1019,43 +1401,29 @@ HistArgs make_args_core(const Geom3& g, int TW, int TH, int dtype, const Reduce&
   a.cols_per_warp = (a.TW + kSegs - 1) / kSegs;  // columns per half-warp segment
   a.words = (a.S + 31) / 32;
   a.slot_bytes = dtype == 0 ? slot_bytes_for<uint32_t>(a.S) : slot_bytes_for<unsigned long long>(a.S);
-  a.digit_bits = digit_bits_for(a.S);
+  a.digit_bits = digit_bits_for(a.S, sdec, dtype == 0 ? 4 : 8, runs);
+  a.patch_w = patch_width(g, TH);
+  a.row_magic = (unsigned int)(((1ull << 32) + a.SW - 1) / (unsigned long long)a.SW);
   a.r = r;
   a.lists = nullptr;
-  a.nf = a.g.kh * a.g.kw;
-  a.nv = a.g.kw;
-  a.nh = a.g.kh;
+  a.nf = runs.nf;
+  a.nv = runs.nv;
+  a.nh = runs.nh;
   return a;
 }
 
+Runs plan_runs(const Plan& p) {
+  Runs runs;
+  runs.footprint = p.hist_footprint;
+  runs.nf = p.hist_nf;
+  runs.nv = p.hist_nv;
+  runs.nh = p.hist_nh;
+  return runs;
+}
+
 HistArgs make_args(const Plan& p) {
-  HistArgs a{};
-  a.g = p.tile.g;
-  a.TW = p.hist_block_w;
-  a.TH = p.hist_block_h;
-  a.SW = a.TW + a.g.kw - 1;
-  a.SH = a.TH + a.g.kh - 1;
-  a.plane = a.SW * a.SH;
-  a.S = a.g.kd * a.plane;
-  a.tiles_x = (a.g.W + a.TW - 1) / a.TW;
-  a.tiles_yx = a.tiles_x * ((a.g.H + a.TH - 1) / a.TH);
-  a.tiles = a.tiles_yx * a.g.D;
-  a.cols_per_warp = (a.TW + kSegs - 1) / kSegs;  // columns per half-warp segment
-  a.words = (a.S + 31) / 32;
-  a.slot_bytes = p.dtype == 0 ? slot_bytes_for<uint32_t>(a.S) : slot_bytes_for<unsigned long long>(a.S);
-  a.digit_bits = digit_bits_for(a.S);
-  a.r = p.r;
-  if (p.hist_footprint) {
-    a.lists = p.d_hist_lists;
-    a.nf = p.hist_nf;
-    a.nv = p.hist_nv;
-    a.nh = p.hist_nh;
-  } else {
-    a.lists = nullptr;
-    a.nf = a.g.kh * a.g.kw;
-    a.nv = a.g.kw;
-    a.nh = a.g.kh;
-  }
+  HistArgs a = make_args_core(p.tile.g, p.hist_block_w, p.hist_block_h, p.dtype, p.hist_sdec, plan_runs(p), p.r);
+  if (p.hist_footprint) a.lists = p.d_hist_lists;
   return a;
 }
 
@@ -1103,11 +1471,10 @@ std::vector<uint8_t> footprint_mask(const Plan& p) {
   return mask;
 }
 
-// Run lists for footprint windows and for every window deeper than one
-// plane (a 3-D box is walked as a footprint); none for 1-D/2-D boxes.
+// Run lists for footprint windows; none for boxes.
 Runs runs_of(const Plan& p) {
   const Geom3& g = p.tile.g;
-  if (p.footprint.empty() && g.kd == 1) return Runs{};
+  if (p.footprint.empty()) return Runs{};
   if ((long long)g.kd * g.kh * g.kw > (1ll << 24)) return Runs{};  // too large to list
   return count_runs(footprint_mask(p), g.kd, g.kh, g.kw);
 }
@@ -1172,7 +1539,7 @@ void histogram_configure(Plan& p, int tw, int th) {
 
 size_t histogram_smem(const Plan& p) {
   HistArgs a = make_args(p);
-  return smem_bytes_for(a.S, p.hist_sdec, p.dtype == 0 ? 4 : 8, (int)p.hist_lists.size());
+  return smem_bytes_for(a.S, p.hist_sdec, p.dtype == 0 ? 4 : 8, plan_runs(p));
 }
 
 // Scratch slots for the block sort: one per resident block (occupancy x
@@ -1394,7 +1761,7 @@ extern "C" int ndf_histogram_filter_noalloc(const void* d_in, void* d_out, int32
   r.cval = dtype == NDF_FLOAT32 ? (double)(float)cval : cval;
   HistChoice c = choose_tile(g, dtype == 0 ? 4 : 8);
   if (c.TW == 0) return noalloc_fail(NDF_ERR_UNSUPPORTED, "window too large for the histogram kernel");
-  HistArgs a = make_args_core(g, c.TW, c.TH, dtype, r);
+  HistArgs a = make_args_core(g, c.TW, c.TH, dtype, c.sdec, Runs{}, r);
   if ((size_t)a.slot_bytes > kNoAllocScratchBytes)
     return noalloc_fail(NDF_ERR_MEMORY,
                         "the window's sort slot exceeds the 16 MiB allocation-free scratch");
@@ -1406,7 +1773,7 @@ extern "C" int ndf_histogram_filter_noalloc(const void* d_in, void* d_out, int32
     cudaGetLastError();
     return noalloc_fail(NDF_ERR_NO_DEVICE, "no usable CUDA device");
   }
-  const size_t smem = smem_bytes_for(a.S, c.sdec, dtype == 0 ? 4 : 8, 0);
+  const size_t smem = smem_bytes_for(a.S, c.sdec, dtype == 0 ? 4 : 8, Runs{});
   if (smem > (size_t)optin) return noalloc_fail(NDF_ERR_UNSUPPORTED, "window too large for shared memory");
   void* scratch = nullptr;
   e = noalloc_scratch(device, &scratch);
