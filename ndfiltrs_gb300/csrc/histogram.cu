@@ -11,11 +11,11 @@
 // does not matter.
 //
 // GB300 design:
-//  * one thread block per output tile (persistent grid over tiles);
-//  * ranking: a block-level LSD radix sort of the support's keys (8-bit
-//    digits, warp match_any ranking for stability, digits on which every
-//    retained key agrees are skipped) through a per-block scratch slot in
-//    global memory (L2-resident); rank codes are u16 (support <= 65534);
+//  * one thread block per output tile (a persistent grid where slots are used);
+//  * ranking: a block-level LSD radix sort of the support's keys over the bits
+//    on which the retained ones differ, in shared memory where it fits (boxes)
+//    or through a per-block scratch slot in global memory (L2-resident); rank
+//    codes are u16 (support <= 65534);
 //  * boxes: a warp selects for a patch of 32 outputs whose windows share one
 //    threshold rank (PatchWalk), at a few ranks and support rows per patch;
 //  * footprints: each half-warp (16 lanes) owns a strip of output columns and
@@ -29,7 +29,8 @@
 // Walking every box window through a bitset of its own cost 238 warp
 // instructions per output at 65 x 65 whatever the window; patches took the
 // 65 x 65 median of a 4096^2 float32 star field from 6.59 to 3.07 ms and the
-// (9, 33, 33) median of a 64 x 512 x 512 cube from 61.2 to 33.0 ms.
+// (9, 33, 33) median of a 64 x 512 x 512 cube from 61.2 to 33.0 ms; sorting a box's
+// support in shared memory, and sharing it among four planes, to 2.42 and 15 ms.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -56,15 +57,17 @@ constexpr int kMaxSupport = 65534;
 
 struct HistArgs {
   Geom3 g;
-  int TW, TH, SW, SH, S;
-  int plane;                // SH * SW: one support plane (the support is kd planes)
+  int TW, TH, TZ, SW, SH, SZ, S;
+  int plane;                // SH * SW: one support plane (the support is SZ of them)
   long long tiles_x, tiles_yx, tiles;
   int cols_per_warp;        // columns walked by each half-warp segment
   int words;                // per-segment bit histogram: 32-bit words
-  long long slot_bytes;     // scratch bytes per block slot
+  long long slot_bytes;     // scratch bytes per block slot (sorts through a slot)
   int digit_bits;           // largest radix digit width of the block sort (8 to 11)
   int patch_w;              // boxes: columns of a warp's patch of outputs (8 or 32)
+  int in_smem;              // boxes: the support is sorted in shared memory (else through a slot)
   unsigned int row_magic;   // ceil(2^32 / SW): row of an in-plane support index
+  unsigned int plane_magic; // ceil(2^32 / plane): plane of a support index
   Reduce r;
   // Footprint windows: support-linear offsets (y * SW + x) of the taps
   // (nf), of the top and bottom ends of every vertical run of taps (nv
@@ -84,6 +87,12 @@ struct Slot {
 };
 
 __host__ __device__ inline long long align16(long long v) { return (v + 15) & ~15ll; }
+
+// Bytes of a box tile's axis maps: 64-bit offsets of its rows, planes and
+// columns (not for a single row).
+__host__ __device__ inline long long box_map_bytes(int SH, int SZ, int SW) {
+  return align16(8ll * (SH + SZ + (SH * SZ > 1 ? SW : 0)));
+}
 
 template <typename K>
 __host__ __device__ inline long long slot_bytes_for(int S) {
@@ -535,19 +544,15 @@ __device__ __forceinline__ Ranks hist_ranks(SegHist& h, const HistArgs& a) {
   }
 }
 
-// The statistic of a window from its ranks' keys (kl = sorted[lo],
-// kh = sorted[hi]).
+// The statistic of a window from the samples of its ranks lo and hi.
 template <typename T>
-__device__ __forceinline__ T hist_value(const Ranks& o, const HistArgs& a, typename KeyOf<T>::K kl,
-                                        typename KeyOf<T>::K kh) {
-  using KO = KeyOf<T>;
+__device__ __forceinline__ T hist_value(const Ranks& o, const HistArgs& a, T vlo, T vhi) {
   if (!o.valid) return nan_of(T());
-  const T vlo = KO::value(kl);
   switch (a.r.kind) {
     case kPercentile: {
       if (a.r.q_is_max) return vlo;
       const PctSplit ps = pct_split(a.r, max(o.n, 1));
-      return pct_value<T>(ps, vlo, o.two ? KO::value(kh) : vlo);
+      return pct_value<T>(ps, vlo, o.two ? vhi : vlo);
     }
     case kRank:
     case kRankHistogram:
@@ -557,9 +562,9 @@ __device__ __forceinline__ T hist_value(const Ranks& o, const HistArgs& a, typen
     default:
       if (!o.two) return vlo;
       if constexpr (sizeof(T) == 4) {
-        return midpoint_f32(vlo, KO::value(kh));
+        return midpoint_f32(vlo, vhi);
       } else {
-        return midpoint(vlo, KO::value(kh));
+        return midpoint(vlo, vhi);
       }
   }
 }
@@ -585,7 +590,7 @@ struct OutPipe {
     }
   }
   __device__ __forceinline__ void complete(const HistArgs& a, T* __restrict__ out) {
-    if (held_at >= 0) out[held_at] = canonical(hist_value<T>(held, a, kl, kh));
+    if (held_at >= 0) out[held_at] = canonical(hist_value<T>(held, a, KeyOf<T>::value(kl), KeyOf<T>::value(kh)));
     held_at = -1;
   }
   // Complete the held batch, then load the parked one's keys and hold it.
@@ -653,6 +658,253 @@ __device__ __forceinline__ void walk(const uint16_t* codes, const uint16_t* list
 }
 
 // ---------------------------------------------------------------------------
+// A tile's support: its samples in the array, each axis mapped through its
+// boundary mode once per tile. (A single row maps its columns as it goes: a
+// table for it would not fit.)
+template <typename T>
+struct Support {
+  using K = typename KeyOf<T>::K;
+  const HistArgs& a;
+  const T* in;
+  long long* row_map;     // SH row offsets, then SZ plane offsets (-1: outside)
+  long long* column_map;  // SW column offsets
+  long long x0;
+  T outside;
+
+  __device__ __forceinline__ long long column(int sx) const {
+    long long m;
+    return map_index(x0 + sx - a.g.ax, a.g.W, a.g.mx, &m) ? m : -1;
+  }
+  __device__ __forceinline__ bool line() const { return a.SZ * a.SH == 1; }
+
+  // Fill the tables (the caller synchronizes).
+  __device__ __forceinline__ void build(long long z0, long long y0) {
+    const Geom3& g = a.g;
+    const int lines = a.SH + a.SZ;
+    for (int i = threadIdx.x; i < lines + (line() ? 0 : a.SW); i += blockDim.x) {
+      long long m;
+      if (i < a.SH)
+        row_map[i] = map_index(y0 + i - g.ay, g.H, g.my, &m) ? m * g.W : -1;
+      else if (i < lines)
+        row_map[i] = map_index(z0 + (i - a.SH) - g.az, g.D, g.mz, &m) ? m * g.H * g.W : -1;
+      else
+        column_map[i - lines] = column(i - lines);
+    }
+  }
+
+  // f(support index, key) for every sample, rows to warps.
+  template <typename F>
+  __device__ __forceinline__ void each(F&& f) const {
+    const bool drop_inf = a.r.drop_inf;
+    const K out_key = sample_key<T>(outside, drop_inf);
+    if (line()) {
+      const bool inside = row_map[0] >= 0 && row_map[1] >= 0;
+      const T* src = in + (inside ? row_map[0] + row_map[1] : 0);
+      for (int sx = threadIdx.x; sx < a.SW; sx += blockDim.x) {
+        const long long ox = column(sx);
+        f(sx, inside && ox >= 0 ? sample_key<T>(__ldg(src + ox), drop_inf) : out_key);
+      }
+      return;
+    }
+    const int lane = threadIdx.x & 31, rows = a.SZ * a.SH;
+    for (int row = threadIdx.x >> 5; row < rows; row += kHWarps) {
+      const int sz = a.SZ > 1 ? row / a.SH : 0;
+      const long long oy = row_map[row - sz * a.SH], oz = row_map[a.SH + sz];
+      const bool inside = oy >= 0 && oz >= 0;
+      const T* src = in + (inside ? oy + oz : 0);
+      const int e = row * a.SW;
+#pragma unroll 4
+      for (int sx = lane; sx < a.SW; sx += 32) {
+        const long long ox = column_map[sx];
+        f(e + sx, inside && ox >= 0 ? sample_key<T>(__ldg(src + ox), drop_inf) : out_key);
+      }
+    }
+  }
+
+  __device__ __forceinline__ T value(unsigned int e) const {
+    unsigned int sz = 0;
+    if (a.SZ > 1) {
+      sz = __umulhi(e, a.plane_magic);
+      e -= sz * a.plane;
+    }
+    const unsigned int sy = __umulhi(e, a.row_magic);
+    const int sx = (int)(e - sy * a.SW);
+    const long long oy = row_map[sy], oz = row_map[a.SH + sz];
+    const long long ox = line() ? column(sx) : column_map[sx];
+    return oy >= 0 && oz >= 0 && ox >= 0 ? __ldg(in + oy + oz + ox) : outside;
+  }
+};
+
+// The bits on which the support's retained keys differ (AND and OR over the
+// block) and the number of dropped samples.
+template <typename K>
+struct KeyBits {
+  K varying;
+  int sent;
+};
+
+template <typename K>
+__device__ __forceinline__ KeyBits<K> block_bits(K k_and, K k_or, int sent, int S) {
+  __shared__ K red_and[kHWarps], red_or[kHWarps];
+  __shared__ int red_sent[kHWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int o = 16; o >= 1; o >>= 1) {
+    k_and &= __shfl_xor_sync(0xffffffffu, k_and, o);
+    k_or |= __shfl_xor_sync(0xffffffffu, k_or, o);
+    sent += __shfl_xor_sync(0xffffffffu, sent, o);
+  }
+  if (lane == 0) {
+    red_and[warp] = k_and;
+    red_or[warp] = k_or;
+    red_sent[warp] = sent;
+  }
+  __syncthreads();
+  k_and = ~K(0);
+  k_or = 0;
+  sent = 0;
+  for (int w = 0; w < kHWarps; ++w) {
+    k_and &= red_and[w];
+    k_or |= red_or[w];
+    sent += red_sent[w];
+  }
+  return {sent == S ? K(0) : (K)(k_and ^ k_or), sent};
+}
+
+template <typename K>
+__device__ __forceinline__ int lowest_set(K v) {
+  return (sizeof(K) == 8 ? __ffsll((long long)v) : __ffs((int)v)) - 1;
+}
+template <typename K>
+__device__ __forceinline__ int highest_set(K v) {
+  return (int)sizeof(K) * 8 - 1 - (sizeof(K) == 8 ? __clzll((long long)v) : __clz((int)v));
+}
+
+// ---------------------------------------------------------------------------
+// Block sort of a support within shared memory (boxes).
+//
+// Sorting keys and payloads through a slot in global memory scatters a key and
+// a payload per sample and pass, a 32-byte sector each: 1.7 of the 3.1 ms of a
+// 65 x 65 median of 4096^2 went there, at 21% issue. Here the samples' order (16-bit
+// indices) ping-pongs between the two arrays that the walk needs anyway, and
+// only the 16 key bits that the next digits come from lie beside them; they are
+// taken from the array again (it is in L2) when those are used up. A key is
+// never moved, so a sample costs 6 bytes of shared memory whatever its type.
+// Per pass of four bits each thread counts the digits of a run of consecutive
+// samples in sixteen counters of its own, one scan over (digit, thread) makes
+// them first positions, and the thread places its samples in order: no atomics
+// and no search for equal digits within a warp, which made wide digits dear
+// (ranking 8-bit digits with match_any kept that pipe 61% busy and took 1.9 ms
+// of a 65 x 65 median of 4096^2, with ballots 1.5 ms at 149 warp instructions per
+// 32 samples and pass). Counters of the digits d and d + 8 share a word in the
+// thread's bank; a run has twice an odd number of samples, so that the runs'
+// words lie in different banks too.
+// Returns with the sorted order in `order` (S indices).
+constexpr int kDigitBits = 4;
+constexpr int kCounterWords = (1 << kDigitBits) / 2 * kHThreads;
+
+template <typename T>
+__device__ void sort_in_smem(const Support<T>& sup, uint16_t* other, uint16_t* order, uint16_t* seg,
+                             unsigned int* table, typename KeyOf<T>::K varying) {
+  using K = typename KeyOf<T>::K;
+  __shared__ unsigned int warp_sum[kHWarps];
+  const HistArgs& a = sup.a;
+  const int S = a.S, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (varying == 0) {
+    for (int i = tid; i < S; i += blockDim.x) order[i] = (uint16_t)i;
+    __syncthreads();
+    return;
+  }
+  // The last pass writes `order`.
+  const int lo = lowest_set(varying), nbits = highest_set(varying) - lo + 1;
+  const int passes = (nbits + kDigitBits - 1) / kDigitBits;
+  constexpr int kPerFill = 16 / kDigitBits;
+  constexpr int kRake = kCounterWords / kHThreads;  // 8
+  const int run = 2 * (((S + 2 * kHThreads - 1) / (2 * kHThreads)) | 1);
+  const int begin = min(S, tid * run), end = min(S, begin + run);
+  uint16_t* counters = reinterpret_cast<uint16_t*>(table + tid);
+  auto counter = [&](unsigned int d) -> uint16_t& { return counters[(d & 7) * 2 * kHThreads + (d >> 3)]; };
+  for (int pass = 0; pass < passes; ++pass) {
+    const int in_seg = pass % kPerFill;
+    if (in_seg == 0) {
+      const int shift = lo + pass * kDigitBits;
+      sup.each([&](int e, K key) { seg[e] = (uint16_t)(key >> shift); });
+    }
+    const int shift = in_seg * kDigitBits;
+    const bool to_order = ((passes - 1 - pass) & 1) == 0;
+    const uint16_t* src = to_order ? other : order;
+    uint16_t* dst = to_order ? order : other;
+#pragma unroll
+    for (int j = 0; j < kRake; ++j) table[j * kHThreads + tid] = 0;
+    __syncthreads();
+    // Two samples at a time: i and i + 1 (runs start at even places).
+    auto samples = [&](int i) -> unsigned int {
+      return pass == 0 ? (unsigned int)i | (unsigned int)(i + 1) << 16 : *reinterpret_cast<const unsigned int*>(src + i);
+    };
+    auto digit = [&](unsigned int e) -> unsigned int { return (unsigned int)(seg[e] >> shift) & 15u; };
+#pragma unroll 2
+    for (int i = begin; i + 1 < end; i += 2) {
+      const unsigned int e = samples(i);
+      const unsigned int d0 = digit(e & 0xFFFFu), d1 = digit(e >> 16);
+      ++counter(d0);
+      ++counter(d1);
+    }
+    if ((end - begin) & 1) ++counter(digit(samples(end - 1) & 0xFFFFu));
+    __syncthreads();
+    // Exclusive scan in the order (digit, thread); thread r rakes the words
+    // 8 r to 8 r + 7. The low halves (digits 0 to 7) come before all high ones.
+    uint4* mine = reinterpret_cast<uint4*>(table + tid * kRake);
+    uint4 u = mine[0], v = mine[1];
+    const unsigned int c[kRake] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+    unsigned int sum = 0;
+#pragma unroll
+    for (int j = 0; j < kRake; ++j) sum += c[j];
+    unsigned int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned int up = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += up;
+    }
+    if (lane == 31) warp_sum[warp] = incl;
+    __syncthreads();
+    unsigned int base = incl - sum, total = 0;
+#pragma unroll
+    for (int w = 0; w < kHWarps; ++w) {
+      const unsigned int t = warp_sum[w];
+      base += w < warp ? t : 0;
+      total += t;
+    }
+    base += total << 16;
+    unsigned int p[kRake];
+#pragma unroll
+    for (int j = 0; j < kRake; ++j) {
+      p[j] = base;
+      base += c[j];
+    }
+    mine[0] = make_uint4(p[0], p[1], p[2], p[3]);
+    mine[1] = make_uint4(p[4], p[5], p[6], p[7]);
+    __syncthreads();
+#pragma unroll 2
+    for (int i = begin; i + 1 < end; i += 2) {
+      const unsigned int e = samples(i);
+      const unsigned int d0 = digit(e & 0xFFFFu), d1 = digit(e >> 16);
+      uint16_t& c0 = counter(d0);
+      const uint16_t at0 = c0;
+      c0 = at0 + 1;
+      uint16_t& c1 = counter(d1);
+      const uint16_t at1 = c1;
+      c1 = at1 + 1;
+      dst[at0] = (uint16_t)e;
+      dst[at1] = (uint16_t)(e >> 16);
+    }
+    if ((end - begin) & 1) {
+      const unsigned int e = samples(end - 1) & 0xFFFFu;
+      dst[counter(digit(e))] = (uint16_t)e;
+    }
+    __syncthreads();
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Box windows (1-D to 3-D): a warp selects for a patch of 32 outputs at once.
 //
 // The 32 windows of a patch overlap almost entirely, so their order statistics
@@ -672,9 +924,10 @@ __device__ __forceinline__ void walk(const uint16_t* codes, const uint16_t* list
 // The work per output is the rows' ballots over 32 outputs plus the rank
 // distance between the patch's least and largest result, instead of the
 // window's faces per output and a walk through a private bitset (16 lanes a
-// window). A patch of 8 x 4 outputs keeps that distance short on slopes; rows
-// of 32 x 1 serve single-row tiles and deep (3-D) windows, where counting rows
-// costs more than looking through ranks.
+// window). A patch of 8 x 4 outputs keeps that distance short on slopes (rows
+// of 32 x 1 serve single-row tiles). Deep (3-D) windows take patches of 8 columns
+// in 4 planes and move them down by a row: of each plane one row leaves and one
+// enters, where 8 x 4 in a plane would count 14.
 
 // Bits [lo, lo + width) of a word; lo and width at least 0.
 __device__ __forceinline__ unsigned int bit_run(int lo, int width) {
@@ -716,17 +969,18 @@ struct Transpose {
   }
 };
 
-template <typename T, int PW, bool DROPS>
+// PW columns by 32 / PW rows (or planes, if DEEP) of outputs.
+template <typename T, int PW, bool DEEP, bool DROPS>
 struct PatchWalk {
-  using K = typename KeyOf<T>::K;
-  static constexpr int PH = 32 / PW;
+  static constexpr int PZ = DEEP ? 32 / PW : 1;
+  static constexpr int PH = DEEP ? 1 : 32 / PW;
 
   const HistArgs& a;
   const uint16_t* codes;  // rank of each support sample (or a dropped code)
-  const uint16_t* place;  // in-plane support index of each rank (65535 up to 32 before and after)
-  const K* sorted;
-  int lx, ly;             // the lane's output within the patch
-  int px, py;             // the patch's first column and row in the tile
+  const uint16_t* place;  // support index of each rank (65535 up to 32 before and after)
+  const Support<T>& sup;
+  int lx, ly, lz;         // the lane's output within the patch
+  int px, py, pz;         // the patch's first column, row and plane in the tile
   int t;                  // threshold rank
   int below, dropped;     // the lane's window: samples of rank below t, dropped samples
   Transpose transpose;
@@ -789,24 +1043,34 @@ struct PatchWalk {
     if (DROPS) dropped += (second ? nd : 0) + (first ? (FLIP ? -nc : nc) : 0);
   }
 
+  // Whether the lane's window holds plane pz + dz of the support.
+  __device__ __forceinline__ bool in_depth(int dz) const { return !DEEP || (unsigned)(dz - lz) < (unsigned)a.g.kd; }
+
+  // Support planes that the patch's windows reach (tiles of fewer planes than a
+  // patch end earlier; the lanes beyond have no output).
+  __device__ __forceinline__ int depth() const { return DEEP ? min(a.g.kd + PZ - 1, a.SZ - pz) : 1; }
+
   // Count the whole windows, two rows at a time (the row after the last is
   // read but lies in no window; it ends within the places that follow).
   __device__ __forceinline__ void count_all() {
     below = dropped = 0;
-    for (int z = 0; z < a.g.kd; ++z) {
-      const uint16_t* row = codes + z * a.plane + py * a.SW;
+    for (int dz = 0; dz < depth(); ++dz) {
+      const uint16_t* row = codes + (pz + dz) * a.plane + py * a.SW;
+      const bool deep = in_depth(dz);
       for (int q = 0; q < a.g.kh + PH - 1; q += 2, row += 2 * a.SW)
-        add_rows<false>(row, a.SW, (unsigned)(q - ly) < (unsigned)a.g.kh, (unsigned)(q + 1 - ly) < (unsigned)a.g.kh);
+        add_rows<false>(row, a.SW, deep && (unsigned)(q - ly) < (unsigned)a.g.kh,
+                        deep && (unsigned)(q + 1 - ly) < (unsigned)a.g.kh);
     }
   }
 
   // Move the windows down by the patch height.
   __device__ __forceinline__ void move_down() {
-    for (int z = 0; z < a.g.kd; ++z) {
-      const uint16_t* row = codes + z * a.plane + py * a.SW;
+    for (int dz = 0; dz < depth(); ++dz) {
+      const uint16_t* row = codes + (pz + dz) * a.plane + py * a.SW;
+      const bool deep = in_depth(dz);
 #pragma unroll 1
       for (int q = 0; q < 2 * PH - 1; ++q, row += a.SW) {
-        const bool mine = PH == 1 || (unsigned)(q - ly) < (unsigned)PH;
+        const bool mine = deep && (PH == 1 || (unsigned)(q - ly) < (unsigned)PH);
         add_rows<true>(row, a.g.kh * a.SW, mine, mine);
       }
     }
@@ -816,19 +1080,30 @@ struct PatchWalk {
   // Which of the ranks [start, start + 32) the lane's window holds (bit i:
   // rank start + i). Ranks outside the support are in no window.
   __device__ __forceinline__ unsigned int ranks_in(int start) const {
-    const unsigned int e = place[start + (int)(threadIdx.x & 31)];
+    unsigned int e = place[start + (int)(threadIdx.x & 31)];
+    int dz = 0;
+    if (DEEP) {
+      // (The planes end below 65535, so its plane is in no window.)
+      const int sz = (int)__umulhi(e, a.plane_magic);
+      e -= sz * a.plane;
+      dz = sz - pz;
+    }
     const int sy = (int)__umulhi(e, a.row_magic);
     const int dx = (int)e - sy * a.SW - px, dy = sy - py;
-    const bool in = (unsigned)dx < (unsigned)(a.g.kw + PW - 1) && (unsigned)dy < (unsigned)(a.g.kh + PH - 1);
+    bool in = (unsigned)dx < (unsigned)(a.g.kw + PW - 1) && (unsigned)dy < (unsigned)(a.g.kh + PH - 1);
+    if (DEEP) in = in && (unsigned)dz < (unsigned)(a.g.kd + PZ - 1);
     if (!__any_sync(kFull, in)) return 0u;
     unsigned int lanes = 0;
     if (in) {
-      // Columns dx - kw + 1 .. dx and rows dy - kh + 1 .. dy of the patch.
+      // Columns dx - kw + 1 .. dx and rows dy - kh + 1 .. dy (planes, if deep)
+      // of the patch.
       const int cl = max(dx - a.g.kw + 1, 0), ch = min(dx, PW - 1);
       lanes = bit_run(cl, ch - cl + 1);
-      if (PH > 1) {
-        lanes *= PW == 8 ? 0x01010101u : PW == 16 ? 0x00010001u : 1u;
-        const int rl = max(dy - a.g.kh + 1, 0), rh = min(dy, PH - 1);
+      if (PW < 32) {
+        static_assert(PW == 8 || PW == 32, "column masks are repeated per byte");
+        lanes *= 0x01010101u;
+        const int d = DEEP ? dz : dy, k = DEEP ? a.g.kd : a.g.kh;
+        const int rl = max(d - k + 1, 0), rh = min(d, 32 / PW - 1);
         lanes &= bit_run(rl * PW, (rh - rl + 1) * PW);
       }
     }
@@ -920,26 +1195,26 @@ struct PatchWalk {
   }
 
   // Walk patches down the tile's rows [row0, row1) of the columns from px.
-  __device__ __forceinline__ void walk(int row0, int row1, int tw_eff, int th_eff, T* __restrict__ out,
-                                       long long at0) {
+  __device__ __forceinline__ void walk(int row0, int row1, int tw_eff, int th_eff, int tz_eff,
+                                       T* __restrict__ out) {
     // Counting whole windows costs kh + PH - 1 rows a plane, moving them
     // 2 (2 PH - 1).
     const bool recount = a.g.kh + PH - 1 <= 2 * (2 * PH - 1);
     py = row0;
     Ranks held;
-    K kl = 0, kh = 0;
+    T vl = 0, vh = 0;
     long long held_at = -1;
     for (;;) {
       if (py == row0 || recount) count_all();
-      const bool live = px + lx < tw_eff && py + ly < th_eff;
+      const bool live = px + lx < tw_eff && py + ly < th_eff && pz + lz < tz_eff;
       const Ranks o = select(live);
-      // The previous patch's keys have arrived by now.
-      if (held_at >= 0) out[held_at] = canonical(hist_value<T>(held, a, kl, kh));
+      // The previous patch's samples have arrived by now.
+      if (held_at >= 0) out[held_at] = canonical(hist_value<T>(held, a, vl, vh));
       held = o;
-      held_at = live ? at0 + (long long)(py + ly) * a.g.W + px + lx : -1;
+      held_at = live ? ((long long)(pz + lz) * a.g.H + py + ly) * a.g.W + px + lx : -1;
       if (o.valid) {
-        kl = sorted[o.lo];
-        kh = o.two ? sorted[o.hi] : kl;
+        vl = sup.value(place[o.lo]);
+        vh = o.two ? sup.value(place[o.hi]) : vl;
       }
       const int next = py + PH;
       const int least = __reduce_min_sync(kFull, o.valid ? o.lo : INT_MAX);
@@ -956,29 +1231,31 @@ struct PatchWalk {
         move_down();
       }
     }
-    if (held_at >= 0) out[held_at] = canonical(hist_value<T>(held, a, kl, kh));
+    if (held_at >= 0) out[held_at] = canonical(hist_value<T>(held, a, vl, vh));
   }
 };
 
 // Every patch column of a tile: columns of patches split into runs of rows so
-// that the block's warps all have work.
-template <typename T, int PW, bool DROPS>
+// that the block's warps all have work. `out` is the tile's first output.
+template <typename T, int PW, bool DEEP, bool DROPS>
 __device__ __forceinline__ void walk_patches(const HistArgs& a, const uint16_t* codes, const uint16_t* place,
-                                             const typename KeyOf<T>::K* sorted, int nret, int tw_eff,
-                                             int th_eff, T* __restrict__ out, long long at0) {
-  constexpr int PH = 32 / PW;
+                                             const Support<T>& sup, int nret, int tw_eff, int th_eff, int tz_eff,
+                                             T* __restrict__ out) {
+  using Walk = PatchWalk<T, PW, DEEP, DROPS>;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int columns = (tw_eff + PW - 1) / PW, rows = (th_eff + PH - 1) / PH;
+  const int across = (tw_eff + PW - 1) / PW, columns = across * ((tz_eff + Walk::PZ - 1) / Walk::PZ);
+  const int rows = (th_eff + Walk::PH - 1) / Walk::PH;
   const int runs = min(rows, max(1, kHWarps / columns));
-  PatchWalk<T, PW, DROPS> p{a, codes, place, sorted, lane % PW, lane / PW, 0, 0, 0, 0, 0};
+  Walk p{a, codes, place, sup, lane % PW, DEEP ? 0 : lane / PW, DEEP ? lane / PW : 0, 0, 0, 0, 0, 0, 0};
   const Reduce& r = a.r;
   p.t = r.kind == kMin ? 0 : r.kind == kMax ? nret : r.kind == kPercentile ? (int)(nret * r.q_fraction) : nret / 2;
   if (r.kind == kRank || r.kind == kRankHistogram)
     p.t = (int)min((long long)nret, r.param * nret / max(1, a.g.kd * a.g.kh * a.g.kw));
   for (int item = warp; item < columns * runs; item += kHWarps) {
-    const int run = item / columns;
-    p.px = (item - run * columns) * PW;
-    p.walk(rows * run / runs * PH, rows * (run + 1) / runs * PH, tw_eff, th_eff, out, at0);
+    const int run = item / columns, column = item - run * columns, deep = column / across;
+    p.px = (column - deep * across) * PW;
+    p.pz = deep * Walk::PZ;
+    p.walk(rows * run / runs * Walk::PH, rows * (run + 1) / runs * Walk::PH, tw_eff, th_eff, tz_eff, out);
   }
 }
 
@@ -991,61 +1268,38 @@ __device__ __forceinline__ void histogram_tile(const T* __restrict__ in, T* __re
                                                long long tile, unsigned char* scratch_slot, unsigned char* smem) {
   using K = typename KeyOf<T>::K;
   const K kSent = KeyOf<T>::kSentinel;
-  __shared__ K red_and[kHWarps], red_or[kHWarps];
-  __shared__ int red_sent[kHWarps];
   const Geom3& g = a.g;
   const int S = a.S;
   // Shared memory. Footprints: rank codes [S] u16 | run lists | decode table
-  // [S] keys (SDEC) | work (radix tables during the sort, half-warp
-  // histograms while sliding). Boxes: rank codes [S + 32] u16 (patches read up
-  // to 32 codes past a row's end) | places of the ranks [32 + S + 32] u16 (no
-  // window holds the outer ones) | decode table (SDEC); the radix tables use the same bytes before those are written.
-  uint16_t* codes_s = reinterpret_cast<uint16_t*>(smem);
-  const long long list_bytes = FP ? align16((long long)(a.nf + 2 * a.nv + 2 * a.nh) * 2) : align16((long long)(a.S + 64) * 2);
-  const long long code_bytes = align16((long long)(FP ? a.S : a.S + 32) * 2);
-  uint16_t* lists_s = reinterpret_cast<uint16_t*>(smem + code_bytes);
-  uint16_t* place_s = lists_s + 32;
-  K* decode_s = reinterpret_cast<K*>(smem + code_bytes + list_bytes);
-  unsigned int* work = reinterpret_cast<unsigned int*>(
-      FP ? smem + code_bytes + list_bytes + (SDEC ? align16((long long)a.S * sizeof(K)) : 0) : smem);
+  // [S] keys (SDEC) | work (the axis maps while gathering, radix tables during
+  // the sort, half-warp histograms while sliding). Boxes: axis maps | rank codes
+  // [S + 64] u16 (patches read up to 32 codes past a row's end, and the row
+  // after the last) | places of the ranks [32 + S + 32] u16 (no window holds
+  // the outer ones) | key bits [S] u16 and counters of the sort in shared
+  // memory. A sort through a slot has its counters where the codes come.
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  Slot<K> slot = slot_at<K>(scratch_slot, S);
-  const unsigned long long keep = keep_policy();
-  const bool drop_inf = a.r.drop_inf;
-  const K outside = sample_key<T>((T)a.r.cval, drop_inf);
-  const long long z = tile / a.tiles_yx;
-  const long long tyx = tile - z * a.tiles_yx;
+  const long long map_bytes = FP ? 0 : box_map_bytes(a.SH, a.SZ, a.SW);
+  uint16_t* codes_s = reinterpret_cast<uint16_t*>(smem + map_bytes);
+  const long long code_bytes = align16((long long)(FP ? a.S : a.S + 64) * 2);
+  const long long list_bytes = FP ? align16((long long)(a.nf + 2 * a.nv + 2 * a.nh) * 2) : code_bytes;
+  uint16_t* lists_s = reinterpret_cast<uint16_t*>(smem + map_bytes + code_bytes);
+  uint16_t* place_s = lists_s + 32;
+  unsigned char* rest = smem + map_bytes + code_bytes + list_bytes;
+  K* decode_s = reinterpret_cast<K*>(rest);
+  unsigned int* work = reinterpret_cast<unsigned int*>(
+      FP ? rest + (SDEC ? align16((long long)a.S * sizeof(K)) : 0) : smem + map_bytes);
+  const long long tz = tile / a.tiles_yx, z = tz * a.TZ;
+  const long long tyx = tile - tz * a.tiles_yx;
   const long long y0 = (tyx / a.tiles_x) * a.TH;
   const long long x0 = (tyx % a.tiles_x) * a.TW;
-  // Gather the support as keys (payload = support index): each coordinate is
-  // mapped through its axis's boundary mode once, into a table in the shared
-  // memory that the sort's counters use afterwards; rows go to warps.
+  long long* maps = reinterpret_cast<long long*>(FP ? reinterpret_cast<unsigned char*>(work) : smem);
+  Support<T> sup{a, in, maps, maps + a.SH + a.SZ, x0, (T)a.r.cval};
+  sup.build(z, y0);
+  __syncthreads();
+  const uint16_t dropped = a.r.omit ? kOmitted : kPropagated;
   K k_and = kSent, k_or = 0;
   int sent = 0;
-  // (A single row maps its columns as it goes: a table of 64-bit offsets for
-  // it would not fit. For two rows or more the tables take at most the 4 S
-  // bytes that both layouts have there.)
-  const int rows = g.kd * a.SH;
-  long long* row_map = reinterpret_cast<long long*>(work);
-  long long* column_map = row_map + a.SH + g.kd;
-  auto column = [&](int sx) -> long long {
-    long long m;
-    return map_index(x0 + sx - g.ax, g.W, g.mx, &m) ? m : -1;
-  };
-  for (int i = threadIdx.x; i < a.SH + g.kd + (rows > 1 ? a.SW : 0); i += blockDim.x) {
-    long long m;
-    if (i < a.SH)
-      row_map[i] = map_index(y0 + i - g.ay, g.H, g.my, &m) ? m * g.W : -1;
-    else if (i < a.SH + g.kd)
-      row_map[i] = map_index(z + (i - a.SH) - g.az, g.D, g.mz, &m) ? m * g.H * g.W : -1;
-    else
-      column_map[i - a.SH - g.kd] = column(i - a.SH - g.kd);
-  }
-  __syncthreads();
-  auto take = [&](int e, bool inside, const T* src) {
-    const K key = inside ? sample_key<T>(__ldcs(src), drop_inf) : outside;
-    st_keep(slot.keys_a + e, key, keep);
-    st_keep(slot.pay_a + e, (uint16_t)e, keep);
+  auto note = [&](K key) {
     if (key != kSent) {
       k_and &= key;
       k_or |= key;
@@ -1053,103 +1307,92 @@ __device__ __forceinline__ void histogram_tile(const T* __restrict__ in, T* __re
       ++sent;
     }
   };
-  if (rows == 1) {
-    const bool inside = row_map[0] >= 0 && row_map[1] >= 0;
-    const T* src = in + (inside ? row_map[0] + row_map[1] : 0);
-    for (int sx = threadIdx.x; sx < a.SW; sx += blockDim.x) {
-      const long long ox = column(sx);
-      take(sx, inside && ox >= 0, src + ox);
+  const K* sorted = nullptr;
+  if (!FP && a.in_smem) {
+    sup.each([&](int, K key) { note(key); });
+    const KeyBits<K> bits = block_bits<K>(k_and, k_or, sent, S);
+    sent = bits.sent;
+    uint16_t* seg = reinterpret_cast<uint16_t*>(rest);
+    unsigned int* table = reinterpret_cast<unsigned int*>(rest + align16((long long)S * 2));
+    sort_in_smem<T>(sup, codes_s, place_s, seg, table, bits.varying);
+    if (sent > 0) {
+      sup.each([&](int e, K key) { seg[e] = key == kSent ? 1 : 0; });
+      __syncthreads();
+    }
+    for (int r = threadIdx.x; r < S; r += blockDim.x) {
+      // A dropped sample (its key can tie with the largest retained one's
+      // sorted bits) lies in no window: place 65535 is below the last row.
+      const uint16_t e = place_s[r];
+      const bool drop = sent > 0 && seg[e] != 0;
+      codes_s[e] = drop ? dropped : (uint16_t)r;
+      if (drop) place_s[r] = 0xFFFF;
     }
   } else {
-    for (int row = warp; row < rows; row += kHWarps) {
-      const int sz = g.kd > 1 ? row / a.SH : 0;
-      const long long oy = row_map[row - sz * a.SH], oz = row_map[a.SH + sz];
-      const bool inside = oy >= 0 && oz >= 0;
-      const T* src = in + (inside ? oy + oz : 0);
-      for (int sx = lane; sx < a.SW; sx += 32) {
-        const long long ox = column_map[sx];
-        take(row * a.SW + sx, inside && ox >= 0, src + ox);
+    Slot<K> slot = slot_at<K>(scratch_slot, S);
+    const unsigned long long keep = keep_policy();
+    sup.each([&](int e, K key) {
+      st_keep(slot.keys_a + e, key, keep);
+      st_keep(slot.pay_a + e, (uint16_t)e, keep);
+      note(key);
+    });
+    const KeyBits<K> bits = block_bits<K>(k_and, k_or, sent, S);
+    sent = bits.sent;
+    // Sort keys (LSD over the bits on which the retained keys differ). The
+    // dropped samples' all-ones keys take part like any other key: an LSD
+    // sort orders the retained keys among themselves whatever lies between
+    // them, and a dropped sample's position is never set in a histogram.
+    K* src_k = slot.keys_a;
+    K* dst_k = slot.keys_b;
+    uint16_t* src_p = slot.pay_a;
+    uint16_t* dst_p = slot.pay_b;
+    if (bits.varying != 0) {
+      const int lo = lowest_set(bits.varying), hi = highest_set(bits.varying);
+      // The fewest passes, with the smallest digits that still cover the bits.
+      const int passes = (hi - lo + a.digit_bits) / a.digit_bits;
+      const int digits = max(5, (hi - lo + passes) / passes);
+      const int nd = 1 << digits;
+      const K mask = (K)(nd - 1);
+      for (int shift = lo; shift <= hi; shift += digits) {
+        radix_pass(src_k, src_p, dst_k, dst_p, S, work, work + kHWarps * nd, nd,
+                   [shift, mask](K key) { return (unsigned int)((key >> shift) & mask); }, keep);
+        K* tk = src_k;
+        src_k = dst_k;
+        dst_k = tk;
+        uint16_t* tp = src_p;
+        src_p = dst_p;
+        dst_p = tp;
       }
     }
-  }
-  for (int o = 16; o >= 1; o >>= 1) {
-    k_and &= __shfl_xor_sync(0xffffffffu, k_and, o);
-    k_or |= __shfl_xor_sync(0xffffffffu, k_or, o);
-    sent += __shfl_xor_sync(0xffffffffu, sent, o);
-  }
-  if (lane == 0) {
-    red_and[warp] = k_and;
-    red_or[warp] = k_or;
-    red_sent[warp] = sent;
-  }
-  __syncthreads();
-  k_and = kSent;
-  k_or = 0;
-  sent = 0;
-  for (int w = 0; w < kHWarps; ++w) {
-    k_and &= red_and[w];
-    k_or |= red_or[w];
-    sent += red_sent[w];
-  }
-  // Sort keys (LSD over the bits on which the retained keys differ). The
-  // dropped samples' all-ones keys take part like any other key: an LSD
-  // sort orders the retained keys among themselves whatever lies between
-  // them, and a dropped sample's position is never set in a histogram.
-  K* src_k = slot.keys_a;
-  K* dst_k = slot.keys_b;
-  uint16_t* src_p = slot.pay_a;
-  uint16_t* dst_p = slot.pay_b;
-  const K varying = sent == S ? K(0) : (k_and ^ k_or);
-  if (varying != 0) {
-    const int bits = (int)sizeof(K) * 8;
-    const int lo = sizeof(K) == 8 ? __ffsll((long long)varying) - 1 : __ffs((int)varying) - 1;
-    const int hi = bits - 1 - (sizeof(K) == 8 ? __clzll((long long)varying) : __clz((int)varying));
-    // The fewest passes, with the smallest digits that still cover the bits.
-    const int passes = (hi - lo + a.digit_bits) / a.digit_bits;
-    const int digits = max(5, (hi - lo + passes) / passes);
-    const int nd = 1 << digits;
-    const K mask = (K)(nd - 1);
-    for (int shift = lo; shift <= hi; shift += digits) {
-      radix_pass(src_k, src_p, dst_k, dst_p, S, work, work + kHWarps * nd, nd,
-                 [shift, mask](K key) { return (unsigned int)((key >> shift) & mask); }, keep);
-      K* tk = src_k;
-      src_k = dst_k;
-      dst_k = tk;
-      uint16_t* tp = src_p;
-      src_p = dst_p;
-      dst_p = tp;
+    for (int pos = threadIdx.x; pos < S; pos += blockDim.x) {
+      const K key = ld_keep(src_k + pos, keep);
+      const uint16_t at = ld_keep(src_p + pos, keep);
+      codes_s[at] = key == kSent ? dropped : (uint16_t)pos;
+      if (!FP) place_s[pos] = key == kSent ? (uint16_t)0xFFFF : at;
+      if (SDEC) decode_s[pos] = key;
     }
-  }
-  const uint16_t dropped = a.r.omit ? kOmitted : kPropagated;
-  for (int pos = threadIdx.x; pos < S; pos += blockDim.x) {
-    const K key = ld_keep(src_k + pos, keep);
-    const uint16_t at = ld_keep(src_p + pos, keep);
-    codes_s[at] = key == kSent ? dropped : (uint16_t)pos;
-    // A dropped sample (its key can tie with the largest retained one's sorted
-    // bits) lies in no window: place 65535 is below the support's last row.
-    if (!FP) place_s[pos] = key == kSent ? (uint16_t)0xFFFF : (uint16_t)(g.kd > 1 ? at % a.plane : at);
-    if (SDEC) decode_s[pos] = key;
+    sorted = SDEC ? decode_s : src_k;
   }
   if (!FP && threadIdx.x < 64) lists_s[threadIdx.x < 32 ? (int)threadIdx.x : S + (int)threadIdx.x] = 0xFFFF;
   __syncthreads();
-  const K* sorted = SDEC ? decode_s : src_k;
   const int th_eff = (int)min((long long)a.TH, g.H - y0);
   const int tw_eff = (int)min((long long)a.TW, g.W - x0);
   T* plane_out = out + z * g.H * g.W;
   if constexpr (!FP) {
-    const long long at0 = y0 * g.W + x0;
-    auto walk_all = [&](auto width, auto drops) {
-      walk_patches<T, decltype(width)::value, decltype(drops)::value>(a, codes_s, place_s, sorted, S - sent, tw_eff,
-                                                                      th_eff, plane_out, at0);
+    const int tz_eff = (int)min((long long)a.TZ, g.D - z);
+    auto walk_all = [&](auto width, auto deep, auto drops) {
+      walk_patches<T, decltype(width)::value, decltype(deep)::value, decltype(drops)::value>(
+          a, codes_s, place_s, sup, S - sent, tw_eff, th_eff, tz_eff, plane_out + y0 * g.W + x0);
     };
     using Yes = std::true_type;
     using No = std::false_type;
     using P8 = std::integral_constant<int, 8>;
     using P32 = std::integral_constant<int, 32>;
-    if (a.patch_w == 8)
-      sent > 0 ? walk_all(P8{}, Yes{}) : walk_all(P8{}, No{});
+    if (g.kd > 1)
+      sent > 0 ? walk_all(P8{}, Yes{}, Yes{}) : walk_all(P8{}, Yes{}, No{});
+    else if (a.patch_w == 8)
+      sent > 0 ? walk_all(P8{}, No{}, Yes{}) : walk_all(P8{}, No{}, No{});
     else
-      sent > 0 ? walk_all(P32{}, Yes{}) : walk_all(P32{}, No{});
+      sent > 0 ? walk_all(P32{}, No{}, Yes{}) : walk_all(P32{}, No{}, No{});
   } else {
     // Slide: each half-warp walks its columns in boustrophedon order.
     const int seg = threadIdx.x / kSeg;
@@ -1245,12 +1488,14 @@ __global__ void __launch_bounds__(kHThreads, FP ? 1 : 2)
 }
 
 struct HistChoice {
-  int TW = 0, TH = 0;
-  bool sdec = false;
+  int TW = 0, TH = 0, TZ = 1;
+  bool sdec = false;     // footprints: sorted keys in shared memory
+  bool in_smem = false;  // boxes: sorted in shared memory
   size_t smem = 0;
 };
 
 constexpr size_t kSmemBudget = 225 * 1024;
+constexpr size_t kSmemPair = 113 * 1024 - 640;  // two blocks per SM (with 1 KB and the static variables each)
 
 // Run-list entries of a footprint window (0 for a rectangular one).
 struct Runs {
@@ -1267,18 +1512,24 @@ size_t work_bytes_for(int S) {
   return std::max(sort, hist);
 }
 
-size_t smem_bytes_for(int S, bool sdec, size_t key_bytes, const Runs& runs) {
-  const size_t codes = (size_t)align16((long long)(runs.footprint ? S : S + 32) * 2);
-  const size_t lists = (size_t)align16((long long)(runs.footprint ? runs.entries() : S + 64) * 2);
+size_t footprint_smem(int S, bool sdec, size_t key_bytes, const Runs& runs) {
+  const size_t codes = (size_t)align16((long long)S * 2);
+  const size_t lists = (size_t)align16((long long)runs.entries() * 2);
   const size_t decode = sdec ? (size_t)align16((long long)S * (long long)key_bytes) : 0;
-  if (runs.footprint) return codes + lists + decode + work_bytes_for(S);
-  return std::max(codes + lists + decode, (size_t)sort_table_words(256) * 4);
+  return codes + lists + decode + work_bytes_for(S);
 }
 
-// The sort takes digits of up to 11 bits (three passes cover 32 varying bits)
-// as far as their tables fit in the bytes they share.
-int digit_bits_for(int S, bool sdec, size_t key_bytes, const Runs& runs) {
-  const size_t room = runs.footprint ? work_bytes_for(S) : smem_bytes_for(S, sdec, key_bytes, runs);
+size_t box_smem(const Geom3& g, int tw, int th, int tz, bool in_smem) {
+  const int SH = th + g.kh - 1, SW = tw + g.kw - 1, SZ = tz + g.kd - 1;
+  const long long S = (long long)SZ * SH * SW;
+  const size_t maps = (size_t)box_map_bytes(SH, SZ, SW), codes = 2 * (size_t)align16((S + 64) * 2);
+  if (in_smem) return maps + codes + (size_t)align16(S * 2) + (size_t)kCounterWords * 4;
+  return maps + std::max(codes, (size_t)sort_table_words(256) * 4);
+}
+
+// Sorts through a slot take digits of up to 11 bits (three passes cover 32
+// varying bits) as far as their tables fit in the bytes they share.
+int slot_digit_bits(size_t room) {
   int bits = 8;
   while (bits < 11 && (size_t)sort_table_words(2 << bits) * 4 <= room) ++bits;
   return bits;
@@ -1302,30 +1553,36 @@ Runs count_runs(const std::vector<uint8_t>& mask, int kd, int kh, int kw) {
 }
 
 // The patch width of a box window's tile of height th: rows of 32 outputs
-// where a tile has single rows or a window has planes (counting the 2 PH - 1
-// rows that a patch of height PH leaves and enters per plane costs more there
-// than looking through the ranks that a wider patch spreads over).
-int patch_width(const Geom3& g, int th) { return th % 4 != 0 || g.kd > 1 ? 32 : 8; }
+// where a tile has single rows, else 8 columns.
+int patch_width(const Geom3& g, int th) { return th % 4 != 0 && g.kd == 1 ? 32 : 8; }
 
-// Work per output of a box window's tile in warp instructions: the block sort
-// of the support, the rows counted per patch, and the ranks looked through,
-// which grow with the support over the window and with the spread of the
-// patch's order statistics (that of windows shifted across the patch, for
-// independent samples).
-double box_cost(const Geom3& g, int tw, int th, double S, bool sdec) {
-  const int pw = patch_width(g, th), ph = 32 / pw;
-  const double outputs = (double)tw * th, volume = (double)g.kd * g.kh * g.kw;
+// Work per output of a box window's tile in warp instructions (measured on
+// windows from 13 x 13 to 129 x 129 and 9 x 33 x 33): the block sort of the
+// support (13 per sample in shared memory, 29 through a slot, and a share of the
+// passes' scans and barriers per tile), pairs of rows
+// counted per patch, and the ranks looked through, which grow with the support
+// over the window and with the spread of the patch's order statistics (that of
+// windows shifted across the patch, for independent samples, and 1% of the
+// support for a slope).
+double box_cost(const Geom3& g, int tw, int th, int tz, double S, bool in_smem) {
+  const int pw = patch_width(g, th), lines = 32 / pw;
+  const bool deep = g.kd > 1;
+  const int ph = deep ? 1 : lines, pz = deep ? lines : 1;
+  const double outputs = (double)tw * th * tz, volume = (double)g.kd * g.kh * g.kw;
   const double words = (g.kw + pw - 1 + 31) / 32;
-  const double row = 8.0 * words + 8.0;
-  const double all = (double)g.kd * (g.kh + ph - 1), moved = (double)g.kd * 2 * (2 * ph - 1);
-  const double columns = tw / pw, runs = std::max(1.0, kHWarps / columns);
-  const double steps = std::max(1.0, th / ph / runs);
-  const double rows = std::min(all, moved + all / steps) * row;
-  const double moves = std::min(std::sqrt(0.5 * g.kd * ((double)g.kh * (pw - 1) + (double)g.kw * (ph - 1))),
-                                1.5 * std::sqrt(0.25 * volume) * 2.0);
-  const double ranks = std::min(S, 1.6 * moves * S / volume);
-  const double idle = std::max(1.0, kHWarps / (columns * std::min(runs, (double)th / ph)));
-  return 6.0 * S / outputs + idle * (rows + 45.0 * (ranks / 32.0 + 2.0) + 120.0) / 32.0 + (sdec ? 0.0 : 0.5);
+  const double pair = 20.0 * words + 25.0;
+  const double planes = g.kd + pz - 1;
+  const double all = planes * (g.kh + ph - 1) / 2, moved = planes * (2 * ph - 1);
+  const double columns = (double)(tw / pw) * ((tz + pz - 1) / pz), steps_all = std::max(1, th / ph);
+  const double runs = std::min(steps_all, std::max(1.0, kHWarps / columns));
+  const double steps = std::max(1.0, steps_all / runs);
+  const double pairs = std::min(all, moved + all / steps);
+  const double shifted = deep ? (double)g.kh * g.kw * (pz - 1) : (double)g.kw * (ph - 1);
+  const double moves = std::min(std::sqrt(0.5 * ((double)g.kd * g.kh * (pw - 1) + shifted)), 1.5 * std::sqrt(volume));
+  const double ranks = std::min(S, 1.6 * moves * S / volume + 0.01 * S);
+  const double idle = std::max(1.0, kHWarps / (columns * runs));
+  const double patches = outputs / 32.0 * (deep ? (double)pz * ((tz + pz - 1) / pz) / tz : 1.0);
+  return ((in_smem ? 13.0 : 29.0) * S + 12000.0 + idle * patches * (pairs * pair + 65.0 * (ranks / 32.0 + 2.0) + 250.0)) / outputs;
 }
 
 // Pick the output tile by a cost model: for boxes box_cost; for footprints in
@@ -1340,31 +1597,42 @@ HistChoice choose_tile(const Geom3& g, size_t key_bytes, const Runs& runs = Runs
   if ((long long)g.kw > kMaxSupport || (long long)g.kh > kMaxSupport || (long long)g.kd > kMaxSupport)
     return best;
   double best_cost = 1e300;
-  auto consider = [&](int tw, int th) {
-    long long S = (long long)g.kd * (tw + g.kw - 1) * (th + g.kh - 1);
+  auto consider = [&](int tw, int th, int tz = 1) {
+    long long S = (long long)(g.kd + tz - 1) * (tw + g.kw - 1) * (th + g.kh - 1);
     if (S > kMaxSupport) return;
-    for (int sdec = 1; sdec >= 0; --sdec) {
-      size_t smem = smem_bytes_for((int)S, sdec != 0, key_bytes, runs);
-      if (smem > kSmemBudget) continue;
-      double cost;
-      if (runs.footprint) {
+    if (runs.footprint) {
+      for (int sdec = 1; sdec >= 0; --sdec) {
+        const size_t smem = footprint_smem((int)S, sdec != 0, key_bytes, runs);
+        if (smem > kSmemBudget) continue;
         const double cpw = (tw + kSegs - 1) / kSegs;
         const double outputs = (double)tw * th;
-        cost = 2.0 * runs.nv + runs.nf / (cpw * th) + 2.0 * runs.nh / th + 8.0 * (double)S / outputs +
-               (sdec ? 0.0 : 12.0);
+        double cost = 2.0 * runs.nv + runs.nf / (cpw * th) + 2.0 * runs.nh / th + 8.0 * (double)S / outputs +
+                      (sdec ? 0.0 : 12.0);
         if (smem * 2 <= kSmemBudget) cost *= 0.9;  // two resident blocks per SM
-      } else {
-        cost = box_cost(g, tw, th, (double)S, sdec != 0);
-        if (smem * 2 <= kSmemBudget) cost *= 0.8;  // two resident blocks per SM
+        if (cost < best_cost) {
+          best_cost = cost;
+          best.TW = tw;
+          best.TH = th;
+          best.sdec = sdec != 0;
+          best.smem = smem;
+        }
+        return;
       }
+      return;
+    }
+    for (int in_smem = 1; in_smem >= 0; --in_smem) {
+      const size_t smem = box_smem(g, tw, th, tz, in_smem != 0);
+      if (smem > kSmemBudget) continue;
+      double cost = box_cost(g, tw, th, tz, (double)S, in_smem != 0);
+      if (smem <= kSmemPair) cost *= 0.75;  // two resident blocks per SM
       if (cost < best_cost) {
         best_cost = cost;
         best.TW = tw;
         best.TH = th;
-        best.sdec = sdec != 0;
+        best.TZ = tz;
+        best.in_smem = in_smem != 0;
         best.smem = smem;
       }
-      if (runs.footprint) return;
     }
   };
   if (force_tw > 0) {
@@ -1376,33 +1644,49 @@ HistChoice choose_tile(const Geom3& g, size_t key_bytes, const Runs& runs = Runs
       if (tw <= 32 || tw / 2 < g.W) consider(tw, 1);
     return best;
   }
-  for (int tw : {128, 64, 32}) {
+  for (int tw : {128, 64, 32, 16}) {
     if (tw > 32 && tw / 2 >= g.W) continue;
+    if (tw == 16 && (runs.footprint || g.kd == 1)) continue;
     for (int th : {256, 192, 128, 96, 64, 48, 32, 16, 8, 4, 2, 1}) {
       if (th > 1 && th / 2 >= g.H) continue;
       consider(tw, th);
     }
+    if (runs.footprint) continue;
+    // Boxes also take the heights between, where a support just fits, and deep
+    // ones several planes.
+    for (int th = 120; th > 8; th -= 4)
+      if (th / 2 < g.H) consider(tw, th);
+    if (g.kd > 1)
+      for (int tz : {2, 4, 8, 16})
+        for (int th = 64; th >= 4; th -= 4)
+          if (th / 2 < g.H && tz / 2 < g.D) consider(tw, th, tz);
   }
   return best;
 }
 
-HistArgs make_args_core(const Geom3& g, int TW, int TH, int dtype, bool sdec, const Runs& runs, const Reduce& r) {
+HistArgs make_args_core(const Geom3& g, const HistChoice& c, int dtype, const Runs& runs, const Reduce& r) {
   HistArgs a{};
   a.g = g;
-  a.TW = TW;
-  a.TH = TH;
+  a.TW = c.TW;
+  a.TH = c.TH;
   a.SW = a.TW + a.g.kw - 1;
   a.SH = a.TH + a.g.kh - 1;
+  a.TZ = c.TZ;
+  a.SZ = a.TZ + a.g.kd - 1;
   a.plane = a.SW * a.SH;
-  a.S = a.g.kd * a.plane;
+  a.S = a.SZ * a.plane;
   a.tiles_x = (a.g.W + a.TW - 1) / a.TW;
   a.tiles_yx = a.tiles_x * ((a.g.H + a.TH - 1) / a.TH);
-  a.tiles = a.tiles_yx * a.g.D;
+  a.tiles = a.tiles_yx * ((a.g.D + a.TZ - 1) / a.TZ);
   a.cols_per_warp = (a.TW + kSegs - 1) / kSegs;  // columns per half-warp segment
   a.words = (a.S + 31) / 32;
   a.slot_bytes = dtype == 0 ? slot_bytes_for<uint32_t>(a.S) : slot_bytes_for<unsigned long long>(a.S);
-  a.digit_bits = digit_bits_for(a.S, sdec, dtype == 0 ? 4 : 8, runs);
-  a.patch_w = patch_width(g, TH);
+  a.in_smem = c.in_smem;
+  a.digit_bits = c.in_smem ? kDigitBits
+                           : slot_digit_bits(runs.footprint ? work_bytes_for(a.S)
+                                                            : c.smem - (size_t)box_map_bytes(a.SH, a.SZ, a.SW));
+  a.patch_w = patch_width(g, c.TH);
+  a.plane_magic = (unsigned int)(((1ull << 32) + a.plane - 1) / (unsigned long long)a.plane);
   a.row_magic = (unsigned int)(((1ull << 32) + a.SW - 1) / (unsigned long long)a.SW);
   a.r = r;
   a.lists = nullptr;
@@ -1421,8 +1705,19 @@ Runs plan_runs(const Plan& p) {
   return runs;
 }
 
+HistChoice plan_choice(const Plan& p) {
+  HistChoice c;
+  c.TW = p.hist_block_w;
+  c.TH = p.hist_block_h;
+  c.TZ = p.hist_block_d;
+  c.sdec = p.hist_sdec;
+  c.in_smem = p.hist_in_smem;
+  c.smem = p.hist_smem;
+  return c;
+}
+
 HistArgs make_args(const Plan& p) {
-  HistArgs a = make_args_core(p.tile.g, p.hist_block_w, p.hist_block_h, p.dtype, p.hist_sdec, plan_runs(p), p.r);
+  HistArgs a = make_args_core(p.tile.g, plan_choice(p), p.dtype, plan_runs(p), p.r);
   if (p.hist_footprint) a.lists = p.d_hist_lists;
   return a;
 }
@@ -1430,14 +1725,15 @@ HistArgs make_args(const Plan& p) {
 template <typename T>
 void* kernel_for(bool sdec, bool fp = false) {
   if (fp) return sdec ? (void*)histogram_kernel<T, true, true> : (void*)histogram_kernel<T, false, true>;
-  return sdec ? (void*)histogram_kernel<T, true, false> : (void*)histogram_kernel<T, false, false>;
+  return (void*)histogram_kernel<T, false, false>;
 }
 
 template <typename T>
 cudaError_t launch_t(const Plan& p, const T* in, T* out, cudaStream_t s) {
   HistArgs a = make_args(p);
-  long long slots = (long long)(p.scratch_bytes / (size_t)a.slot_bytes);
-  long long grid = std::min<long long>(a.tiles, slots);
+  // Sorts in shared memory: a block per tile; through slots: a block per slot.
+  const long long grid = a.in_smem ? std::min<long long>(a.tiles, INT_MAX)
+                                   : std::min<long long>(a.tiles, (long long)(p.scratch_bytes / (size_t)a.slot_bytes));
   if (grid < 1) return cudaErrorInvalidValue;
   unsigned char* scratch = (unsigned char*)p.d_scratch;
   const unsigned blocks = (unsigned)grid;
@@ -1447,10 +1743,7 @@ cudaError_t launch_t(const Plan& p, const T* in, T* out, cudaStream_t s) {
     else
       histogram_kernel<T, false, true><<<blocks, kHThreads, p.smem_bytes, s>>>(in, out, a, scratch);
   } else {
-    if (p.hist_sdec)
-      histogram_kernel<T, true, false><<<blocks, kHThreads, p.smem_bytes, s>>>(in, out, a, scratch);
-    else
-      histogram_kernel<T, false, false><<<blocks, kHThreads, p.smem_bytes, s>>>(in, out, a, scratch);
+    histogram_kernel<T, false, false><<<blocks, kHThreads, p.smem_bytes, s>>>(in, out, a, scratch);
   }
   return cudaGetLastError();
 }
@@ -1496,7 +1789,10 @@ void histogram_configure(Plan& p, int tw, int th) {
   HistChoice c = choose_tile(p.tile.g, p.dtype == 0 ? 4 : 8, runs, tw, th);
   p.hist_block_w = c.TW;
   p.hist_block_h = c.TH;
+  p.hist_block_d = c.TZ;
   p.hist_sdec = c.sdec;
+  p.hist_in_smem = c.in_smem;
+  p.hist_smem = c.smem;
   p.hist_footprint = runs.footprint;
   p.hist_nf = runs.nf;
   p.hist_nv = runs.nv;
@@ -1537,13 +1833,10 @@ void histogram_configure(Plan& p, int tw, int th) {
   p.hist_blocks_y = a.tiles / a.tiles_x;
 }
 
-size_t histogram_smem(const Plan& p) {
-  HistArgs a = make_args(p);
-  return smem_bytes_for(a.S, p.hist_sdec, p.dtype == 0 ? 4 : 8, plan_runs(p));
-}
+size_t histogram_smem(const Plan& p) { return p.hist_smem; }
 
-// Scratch slots for the block sort: one per resident block (occupancy x
-// SMs), capped by the number of tiles.
+// Scratch slots for a block sort through them: one per resident block
+// (occupancy x SMs), capped by the number of tiles.
 cudaError_t histogram_allocate(Plan& p) {
   HistArgs a = make_args(p);
   void* kernel = p.dtype == 0 ? kernel_for<float>(p.hist_sdec, p.hist_footprint)
@@ -1557,6 +1850,8 @@ cudaError_t histogram_allocate(Plan& p) {
                    cudaMemcpyHostToDevice);
   }
   if (e != cudaSuccess) return e;
+  p.scratch_bytes = 0;
+  if (a.in_smem) return cudaSuccess;
   int per_sm = 1;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kHThreads, p.smem_bytes);
   if (e != cudaSuccess) return e;
@@ -1569,12 +1864,12 @@ namespace {
 
 int hist_family_variant(const Plan& p) {
   if (p.algo != Algo::kHistogram || p.dtype != 0) return -1;
-  return (p.hist_sdec ? 1 : 0) + (p.hist_footprint ? 2 : 0);
+  return p.hist_footprint ? (p.hist_sdec ? 3 : 2) : 0;
 }
 
 long long hist_family_tiles(const Plan& p) { return make_args(p).tiles; }
 
-long long hist_family_slot_bytes(const Plan& p) { return make_args(p).slot_bytes; }
+long long hist_family_slot_bytes(const Plan& p) { return p.hist_in_smem ? 0 : make_args(p).slot_bytes; }
 
 void hist_family_write_task(const Plan& p, const void* in, void* out, long long first_tile, void* task) {
   HistTask t{};
@@ -1588,7 +1883,6 @@ void hist_family_write_task(const Plan& p, const void* in, void* out, long long 
 const void* hist_family_kernel(int v) {
   switch (v) {
     case 0: return (const void*)histogram_family_kernel<false, false>;
-    case 1: return (const void*)histogram_family_kernel<true, false>;
     case 2: return (const void*)histogram_family_kernel<false, true>;
     default: return (const void*)histogram_family_kernel<true, true>;
   }
@@ -1761,7 +2055,7 @@ extern "C" int ndf_histogram_filter_noalloc(const void* d_in, void* d_out, int32
   r.cval = dtype == NDF_FLOAT32 ? (double)(float)cval : cval;
   HistChoice c = choose_tile(g, dtype == 0 ? 4 : 8);
   if (c.TW == 0) return noalloc_fail(NDF_ERR_UNSUPPORTED, "window too large for the histogram kernel");
-  HistArgs a = make_args_core(g, c.TW, c.TH, dtype, c.sdec, Runs{}, r);
+  HistArgs a = make_args_core(g, c, dtype, Runs{}, r);
   if ((size_t)a.slot_bytes > kNoAllocScratchBytes)
     return noalloc_fail(NDF_ERR_MEMORY,
                         "the window's sort slot exceeds the 16 MiB allocation-free scratch");
@@ -1773,7 +2067,7 @@ extern "C" int ndf_histogram_filter_noalloc(const void* d_in, void* d_out, int32
     cudaGetLastError();
     return noalloc_fail(NDF_ERR_NO_DEVICE, "no usable CUDA device");
   }
-  const size_t smem = smem_bytes_for(a.S, c.sdec, dtype == 0 ? 4 : 8, Runs{});
+  const size_t smem = c.smem;
   if (smem > (size_t)optin) return noalloc_fail(NDF_ERR_UNSUPPORTED, "window too large for shared memory");
   void* scratch = nullptr;
   e = noalloc_scratch(device, &scratch);
@@ -1787,21 +2081,12 @@ extern "C" int ndf_histogram_filter_noalloc(const void* d_in, void* d_out, int32
   long long grid = std::min<long long>(std::min<long long>(a.tiles, slots),
                                        (long long)std::max(per_sm, 1) * sm_count);
   cudaStream_t s = (cudaStream_t)stream;
-  if (dtype == 0) {
-    if (c.sdec)
-      histogram_kernel<float, true, false><<<(unsigned)grid, kHThreads, smem, s>>>(
-          (const float*)d_in, (float*)d_out, a, (unsigned char*)scratch);
-    else
-      histogram_kernel<float, false, false><<<(unsigned)grid, kHThreads, smem, s>>>(
-          (const float*)d_in, (float*)d_out, a, (unsigned char*)scratch);
-  } else {
-    if (c.sdec)
-      histogram_kernel<double, true, false><<<(unsigned)grid, kHThreads, smem, s>>>(
-          (const double*)d_in, (double*)d_out, a, (unsigned char*)scratch);
-    else
-      histogram_kernel<double, false, false><<<(unsigned)grid, kHThreads, smem, s>>>(
-          (const double*)d_in, (double*)d_out, a, (unsigned char*)scratch);
-  }
+  if (dtype == 0)
+    histogram_kernel<float, false, false><<<(unsigned)grid, kHThreads, smem, s>>>(
+        (const float*)d_in, (float*)d_out, a, (unsigned char*)scratch);
+  else
+    histogram_kernel<double, false, false><<<(unsigned)grid, kHThreads, smem, s>>>(
+        (const double*)d_in, (double*)d_out, a, (unsigned char*)scratch);
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "histogram (allocation-free)");
   return NDF_OK;

@@ -168,8 +168,10 @@ struct Plan {
   unsigned int* d_status = nullptr; // device error flags
 
   // Histogram kernel geometry (1-D/2-D windows).
-  int hist_block_w = 0, hist_block_h = 0;
-  bool hist_sdec = false;  // sorted keys staged in shared memory
+  int hist_block_w = 0, hist_block_h = 0, hist_block_d = 1;
+  bool hist_sdec = false;     // footprints: sorted keys staged in shared memory
+  bool hist_in_smem = false;  // boxes: the block sort stays in shared memory
+  size_t hist_smem = 0;       // shared-memory bytes of the tile
   long long hist_blocks_x = 0, hist_blocks_y = 0;
   // Footprint windows: tap and run-end offsets in the tile's support
   // (taps | top | bottom | left | right ends) and their counts.
@@ -274,7 +276,7 @@ struct FamilyOps {
   cudaError_t (*launch)(int variant, const void* d_tasks, int ntasks, long long tiles, unsigned char* scratch,
                         long long slot_bytes, size_t smem, int grid, cudaStream_t s);
 };
-const FamilyOps& histogram_family_ops();  // sliding histogram (histogram.cu), 4 variants
+const FamilyOps& histogram_family_ops();  // sliding histogram (histogram.cu), variants 0, 2 and 3
 const FamilyOps& box_family_ops();        // box pair 3x3 / 5x5 / 7x7 (box.cu), 6 variants
 const FamilyOps& slide_family_ops();      // sliding exact moments (moments_slide.cu), 1 variant
 const FamilyOps& rank_family_ops();       // ranked networks (rank_network.cu), 13 variants
