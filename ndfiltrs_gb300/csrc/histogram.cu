@@ -1495,6 +1495,7 @@ struct HistChoice {
 };
 
 constexpr size_t kSmemBudget = 225 * 1024;
+constexpr double kBoxSMs = 152;
 constexpr size_t kSmemPair = 113 * 1024 - 640;  // two blocks per SM (with 1 KB and the static variables each)
 
 // Run-list entries of a footprint window (0 for a rectangular one).
@@ -1556,7 +1557,7 @@ Runs count_runs(const std::vector<uint8_t>& mask, int kd, int kh, int kw) {
 // where a tile has single rows, else 8 columns.
 int patch_width(const Geom3& g, int th) { return th % 4 != 0 && g.kd == 1 ? 32 : 8; }
 
-// Work per output of a box window's tile in warp instructions (measured on
+// Work of a box window's tile in warp instructions (measured on
 // windows from 13 x 13 to 129 x 129 and 9 x 33 x 33): the block sort of the
 // support (13 per sample in shared memory, 29 through a slot, and a share of the
 // passes' scans and barriers per tile), pairs of rows
@@ -1582,7 +1583,7 @@ double box_cost(const Geom3& g, int tw, int th, int tz, double S, bool in_smem) 
   const double ranks = std::min(S, 1.6 * moves * S / volume + 0.01 * S);
   const double idle = std::max(1.0, kHWarps / (columns * runs));
   const double patches = outputs / 32.0 * (deep ? (double)pz * ((tz + pz - 1) / pz) / tz : 1.0);
-  return ((in_smem ? 13.0 : 29.0) * S + 12000.0 + idle * patches * (pairs * pair + 65.0 * (ranks / 32.0 + 2.0) + 250.0)) / outputs;
+  return (in_smem ? 13.0 : 29.0) * S + 12000.0 + idle * patches * (pairs * pair + 65.0 * (ranks / 32.0 + 2.0) + 250.0);
 }
 
 // Pick the output tile by a cost model: for boxes box_cost; for footprints in
@@ -1623,8 +1624,12 @@ HistChoice choose_tile(const Geom3& g, size_t key_bytes, const Runs& runs = Runs
     for (int in_smem = 1; in_smem >= 0; --in_smem) {
       const size_t smem = box_smem(g, tw, th, tz, in_smem != 0);
       if (smem > kSmemBudget) continue;
-      double cost = box_cost(g, tw, th, tz, (double)S, in_smem != 0);
-      if (smem <= kSmemPair) cost *= 0.75;  // two resident blocks per SM
+      // Tiles that an SM takes one after the other, whole ones: small arrays
+      // prefer tiles that leave no SM idle. Two resident blocks overlap.
+      const double tiles = std::ceil((double)g.W / tw) * std::ceil((double)g.H / th) * std::ceil((double)g.D / tz);
+      const double turns = std::ceil(tiles / kBoxSMs);
+      const double cost = turns * (smem <= kSmemPair && turns > 1 ? 0.75 : 1.0) *
+                          box_cost(g, tw, th, tz, (double)S, in_smem != 0);
       if (cost < best_cost) {
         best_cost = cost;
         best.TW = tw;
