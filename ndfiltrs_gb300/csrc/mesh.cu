@@ -10,11 +10,14 @@
 // reference writes mul_add), so results equal the reference bit for bit.
 //
 // GB300 design:
-//  * mesh_stats_kernel: one 128-thread block per mesh gathers the mesh's
-//    finite, unmasked samples as order-preserving 64-bit keys into shared
-//    memory (global scratch for meshes beyond 8192 samples), bitonic-sorts
-//    them and runs the SExtractor or sigma-clip sequence with the whole
-//    block. The reference accumulates Neumaier sums in sorted order; the
+//  * mesh_stats32_kernel (float32 meshes of up to 16,384 samples): one block per
+//    mesh gathers the finite, unmasked samples as order-preserving 32-bit keys,
+//    radix-sorts them in shared memory and runs the SExtractor or sigma-clip
+//    sequence; mesh_stats_kernel does the same for the rest with 64-bit keys
+//    and a bitonic network (global scratch for meshes beyond 8192 samples).
+//    Passes that only decide which samples stay run in float32 with an error
+//    bound (m_decide); what is returned, and what the bound does not decide,
+//    runs in the reference's float64. The reference accumulates Neumaier sums in sorted order; the
 //    block sums the terms exactly in fixed point, in parallel, and proves
 //    from the exact sum and a bound on the compensation's rounding that the
 //    sequential sum rounds to the same double (thread 0 runs the sequential
@@ -85,10 +88,29 @@ struct SV {
   __device__ __forceinline__ SV at(long long k) const { return {p + k}; }
 };
 
+// The same over float32 samples (exactly widened).
+struct SVF {
+  const float* p;
+  __device__ __forceinline__ double operator[](long long i) const {
+    const unsigned int b = __float_as_uint(p[i]);
+    const unsigned int e = (b >> 23) & 0xFFu;
+    return e != 0u || (b << 1) == 0u ? f32_to_f64_exact(b) : (double)p[i];
+  }
+  __device__ __forceinline__ SVF at(long long k) const { return {p + k}; }
+};
+
+// v[i] - v[j] rounded to float32 (monotone in i).
+__device__ __forceinline__ float m_diff(SV v, long long i, long long j) {
+  return __double2float_rn(__dsub_rn(v[i], v[j]));
+}
+__device__ __forceinline__ float m_diff(SVF v, long long i, long long j) { return __fsub_rn(v.p[i], v.p[j]); }
+
 // Block state of the statistics: per-warp partial sums and a broadcast slot.
+constexpr int kMWarps = 16;  // of the largest block
 struct MeshShared {
-  W3 part[kMThreads / 32];
-  int low[kMThreads / 32];
+  W3 part[kMWarps];
+  int low[kMWarps];
+  float sums[2][kMWarps];
   double value;
 };
 
@@ -102,7 +124,8 @@ __device__ double broadcast(double v, MeshShared& sh) {
 }
 
 // median_sorted, src/background.rs:950-963.
-__device__ double m_median(SV v, long long n) {
+template <typename V>
+__device__ double m_median(V v, long long n) {
   if (n % 2 == 1) return v[n / 2];
   const double a = v[n / 2 - 1], b = v[n / 2];
   const double mid = __ddiv_rn(__dadd_rn(a, b), 2.0);
@@ -136,8 +159,7 @@ __device__ double block_sum(Term&& term, long long n, int H, MeshShared& sh) {
   e.ok = !__syncthreads_or(!e.ok);
   e.s = sh.part[0];
   e.low = sh.low[0];
-#pragma unroll
-  for (int w = 1; w < kMThreads / 32; ++w) {
+  for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
     add3(e.s, sh.part[w].w0, sh.part[w].w1, sh.part[w].w2);
     e.low = min(e.low, sh.low[w]);
   }
@@ -154,7 +176,8 @@ __device__ double block_sum(Term&& term, long long n, int H, MeshShared& sh) {
 }
 
 // mean_of, src/background.rs:965-978 (mean_valid on overflow).
-__device__ double m_mean(SV v, long long n, MeshShared& sh) {
+template <typename V>
+__device__ double m_mean(V v, long long n, MeshShared& sh) {
   const int H = bound_exponent(fmax(abs64(v[0]), abs64(v[n - 1])));
   const double total = block_sum([&](long long i) { return v[i]; }, n, H, sh);
   if (finite64(total)) return __ddiv_rn(total, (double)n);
@@ -170,7 +193,8 @@ __device__ double m_mean(SV v, long long n, MeshShared& sh) {
 // std_about, src/background.rs:1000-1015. Every scaled deviation is at most
 // 1 in magnitude (the extremes of sorted samples set the scale and rounding
 // is monotone), so the squares lie below 2^1.
-__device__ double m_std(SV v, long long n, double mean, MeshShared& sh) {
+template <typename V>
+__device__ double m_std(V v, long long n, double mean, MeshShared& sh) {
   if (n == 0) return nan_of(0.0);
   const double scale = fmax(abs64(__dsub_rn(v[0], mean)), abs64(__dsub_rn(v[n - 1], mean)));
   if (scale == 0.0) return 0.0;
@@ -189,7 +213,8 @@ __device__ double m_std(SV v, long long n, double mean, MeshShared& sh) {
 // sorted v, divided by Phi^-1(0.75). The deviations ascend on both sides of
 // the first sample at or above the median, so the two middle ranks of their
 // union come from a binary search over the split between the two sides.
-__device__ double m_mad_std(SV v, long long n, double median) {
+template <typename V>
+__device__ double m_mad_std(V v, long long n, double median) {
   long long lo = 0, hi = n;
   while (lo < hi) {
     const long long mid = (lo + hi) / 2;
@@ -219,7 +244,8 @@ __device__ double m_mad_std(SV v, long long n, double median) {
 }
 
 // within, src/background.rs:1024-1032 (two binary searches).
-__device__ void m_within(SV v, long long r0, long long r1, double low, double high, long long& lo,
+template <typename V>
+__device__ void m_within(V v, long long r0, long long r1, double low, double high, long long& lo,
                          long long& hi) {
   long long a = r0, b = r1;
   while (a < b) {
@@ -236,22 +262,94 @@ __device__ void m_within(SV v, long long r0, long long r1, double low, double hi
   hi = a > lo ? a : lo;
 }
 
+// The run [lo, hi) of [s0, s1) within center - lower std .. center + upper std
+// of the samples [q0, q1) (center their mean or median), decided in float32.
+// A clipping pass only needs to know which samples stay: the float64 mean and
+// scatter that the reference computes for it cost some 20 operations per sample
+// on the FP64 pipe, exact sums among them, for bounds that almost never fall
+// within a float32 rounding of a sample. Deviations are taken from a median of
+// the samples, so that |mean| stays near the spread and nothing cancels. With
+// c terms per thread, then a tree, the sums are off by (c + 10) u of their
+// absolute sums, which bounds the error of the limits below; a limit closer to
+// its neighbouring samples than that (or sums out of float32's range) is not
+// decided, and the caller runs the float64 pass. The reference's own roundings
+// lie below 2^-50 of the center. Every thread of the block gets the same answer.
+template <typename V>
+__device__ bool m_decide(V v, long long q0, long long q1, long long s0, long long s1, int center, double lower,
+                         double upper, long long& lo, long long& hi, MeshShared& sh) {
+  const long long n = q1 - q0, pivot = q0 + (n - 1) / 2;
+  const float reach = fmaxf(-m_diff(v, q0, pivot), m_diff(v, q1 - 1, pivot));
+  if (!(reach >= 8.8817842e-16f && reach <= 1.1529215e18f)) return false;
+  float s1f = 0.0f, s2f = 0.0f;
+  for (long long i = q0 + threadIdx.x; i < q1; i += blockDim.x) {
+    const float d = m_diff(v, i, pivot);
+    s1f += d;
+    s2f = __fmaf_rn(d, d, s2f);
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    s1f += __shfl_xor_sync(0xffffffffu, s1f, off);
+    s2f += __shfl_xor_sync(0xffffffffu, s2f, off);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    sh.sums[0][threadIdx.x >> 5] = s1f;
+    sh.sums[1][threadIdx.x >> 5] = s2f;
+  }
+  __syncthreads();
+  s1f = s2f = 0.0f;
+  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
+    s1f += sh.sums[0][w];
+    s2f += sh.sums[1][w];
+  }
+  __syncthreads();
+  const float mean = s1f / (float)n, var = s2f / (float)n - mean * mean;
+  if (!(mean * mean <= 4.0f * var)) return false;
+  const float sd = sqrtf(var);
+  const float middle = center == 0 ? mean : 0.5f * m_diff(v, q0 + n / 2, pivot);
+  const float low = middle - (float)lower * sd, high = middle + (float)upper * sd;
+  const float c = (float)((n + blockDim.x - 1) / blockDim.x);
+  const float unit = (8.0f * c + 128.0f) * 5.9604645e-8f * sd, slack = (float)abs64(v[pivot]) * 8.8817842e-16f;
+  const float low_error = unit * (fabsf((float)lower) + 1.0f) + slack;
+  const float high_error = unit * (fabsf((float)upper) + 1.0f) + slack;
+  long long a = s0, b = s1;
+  while (a < b) {
+    const long long m = (a + b) / 2;
+    if (m_diff(v, m, pivot) < low) a = m + 1; else b = m;
+  }
+  lo = a;
+  if (!(lo == s0 || low - m_diff(v, lo - 1, pivot) > low_error)) return false;
+  if (!(lo == s1 || m_diff(v, lo, pivot) - low > low_error)) return false;
+  a = s0;
+  b = s1;
+  while (a < b) {
+    const long long m = (a + b) / 2;
+    if (m_diff(v, m, pivot) <= high) a = m + 1; else b = m;
+  }
+  if (!(a == s0 || high - m_diff(v, a - 1, pivot) > high_error)) return false;
+  if (!(a == s1 || m_diff(v, a, pivot) - high > high_error)) return false;
+  hi = a > lo ? a : lo;
+  return true;
+}
+
 // clip_sorted, src/background.rs:1034-1069.
-__device__ void m_clip(SV v, long long& r0, long long& r1, double lower, double upper, long long maxiters,
+template <typename V>
+__device__ void m_clip(V v, long long& r0, long long& r1, double lower, double upper, long long maxiters,
                        int center, int spread, MeshShared& sh) {
   long long iteration = 0;
   while (r1 - r0 >= 1 && (maxiters < 0 || iteration < maxiters)) {
-    const SV kept = v.at(r0);
+    const V kept = v.at(r0);
     const long long n = r1 - r0;
-    const double middle = center == 0 ? m_mean(kept, n, sh) : m_median(kept, n);
-    double width;
-    if (spread == 0)
-      width = m_std(kept, n, center == 0 ? middle : m_mean(kept, n, sh), sh);
-    else
-      width = m_mad_std(kept, n, center == 1 ? middle : m_median(kept, n));
     long long lo, hi;
-    m_within(v, r0, r1, __dsub_rn(middle, __dmul_rn(lower, width)), __dadd_rn(middle, __dmul_rn(upper, width)),
-             lo, hi);
+    if (spread != 0 || !m_decide(v, r0, r1, r0, r1, center, lower, upper, lo, hi, sh)) {
+      const double middle = center == 0 ? m_mean(kept, n, sh) : m_median(kept, n);
+      double width;
+      if (spread == 0)
+        width = m_std(kept, n, center == 0 ? middle : m_mean(kept, n, sh), sh);
+      else
+        width = m_mad_std(kept, n, center == 1 ? middle : m_median(kept, n));
+      m_within(v, r0, r1, __dsub_rn(middle, __dmul_rn(lower, width)), __dadd_rn(middle, __dmul_rn(upper, width)),
+               lo, hi);
+    }
     ++iteration;
     if (lo == r0 && hi == r1) break;
     r0 = lo;
@@ -272,24 +370,28 @@ __device__ double m_mode(double mean, double median, double sd, int estimator, d
 // finish_stats with sextractor_stats / clipped_stats, src/background.rs:652-705,
 // 1071-1152. Every thread of the block runs it with the same values; thread
 // 0 writes the mesh's results.
-__device__ void m_finish(SV v, long long n, long long volume, const MeshArgs& a, const MeshOut& o, long long mesh,
+template <typename V>
+__device__ void m_finish(V v, long long n, long long volume, const MeshArgs& a, const MeshOut& o, long long mesh,
                          MeshShared& sh) {
   double background = nan_of(0.0), rms = nan_of(0.0);
   long long retained = 0;
   if (n > 0) {
     if (a.estimator == 0) {
-      const double mean = m_mean(v, n, sh);
-      const double sd = m_std(v, n, mean, sh);
+      // The samples [s0, s1) within `width` std of the mean of [q0, q1).
+      auto around_mean = [&](long long q0, long long q1, double width, long long& s0, long long& s1) {
+        if (m_decide(v, q0, q1, 0, n, 0, width, width, s0, s1, sh)) return;
+        const double mean = m_mean(v.at(q0), q1 - q0, sh);
+        const double sd = m_std(v.at(q0), q1 - q0, mean, sh);
+        m_within(v, 0, n, __dsub_rn(mean, __dmul_rn(width, sd)), __dadd_rn(mean, __dmul_rn(width, sd)), s0, s1);
+      };
       long long f0, f1;
-      m_within(v, 0, n, __dsub_rn(mean, __dmul_rn(2.0, sd)), __dadd_rn(mean, __dmul_rn(2.0, sd)), f0, f1);
+      around_mean(0, n, 2.0, f0, f1);
       if (f0 != f1) {
-        const double mean2 = m_mean(v.at(f0), f1 - f0, sh);
-        const double sd2 = m_std(v.at(f0), f1 - f0, mean2, sh);
         long long s0, s1;
-        m_within(v, 0, n, __dsub_rn(mean2, __dmul_rn(5.0, sd2)), __dadd_rn(mean2, __dmul_rn(5.0, sd2)), s0, s1);
+        around_mean(f0, f1, 5.0, s0, s1);
         m_clip(v, s0, s1, 3.0, 3.0, 100, 1, 0, sh);
         if (s0 != s1) {
-          const SV k = v.at(s0);
+          const V k = v.at(s0);
           const long long c = s1 - s0;
           const double mean3 = m_mean(k, c, sh);
           const double sd3 = m_std(k, c, mean3, sh);
@@ -303,7 +405,7 @@ __device__ void m_finish(SV v, long long n, long long volume, const MeshArgs& a,
       m_clip(v, r0, r1, a.lower, a.upper, a.maxiters, a.center, a.spread, sh);
       retained = r1 - r0;
       if (retained > 0) {
-        const SV k = v.at(r0);
+        const V k = v.at(r0);
         const double mean = m_mean(k, retained, sh);
         const double median = m_median(k, retained);
         const bool need_std = a.statistic == 2 || a.rms == 0;
@@ -389,6 +491,163 @@ __global__ void __launch_bounds__(kMThreads)
       keys[i] = (unsigned long long)__double_as_longlong(mval(keys[i]));
     __syncthreads();
     m_finish(SV{keys}, n, volume, a, o, mesh, sh);
+    __syncthreads();
+  }
+}
+
+// Float32 meshes of up to 16,384 samples: 32-bit keys, sorted by four-bit digits
+// in shared memory. Each thread counts the digits of a run of consecutive keys
+// in sixteen counters of its own (digits d and d + 8 share a word in the
+// thread's bank; a run has twice an odd number of keys, so that the runs lie in
+// different banks), a scan over (digit, thread) makes them first places, and the
+// thread places its keys in order. The 64-bit bitonic network above took 78
+// rounds of 16-byte exchanges for 4,096 samples. Mesh statistics of 4096^2 in boxes of 64:
+// 4.0 ms with that network and the float64 clipping passes, 0.68 ms now.
+template <int NT>
+__device__ uint32_t* m_sort(uint32_t* keys, uint32_t* other, int n, unsigned int* table, uint32_t varying) {
+  __shared__ unsigned int warp_sum[NT / 32];
+  constexpr int kRake = 8;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (varying == 0) return keys;
+  const int first = __ffs((int)varying) - 1, bits = 32 - __clz((int)varying) - first;
+  const int run = 2 * (((n + 2 * NT - 1) / (2 * NT)) | 1);
+  const int begin = min(n, tid * run), end = min(n, begin + run);
+  uint16_t* counters = reinterpret_cast<uint16_t*>(table + tid);
+  uint32_t* src = keys;
+  uint32_t* dst = other;
+  for (int done = 0; done < bits; done += 4) {
+    const int shift = first + done;
+    auto counter = [&](uint32_t key) -> uint16_t& {
+      const unsigned int d = (key >> shift) & 15u;
+      return counters[(d & 7) * 2 * NT + (d >> 3)];
+    };
+#pragma unroll
+    for (int j = 0; j < kRake; ++j) table[j * NT + tid] = 0;
+    __syncthreads();
+    for (int i = begin; i + 1 < end; i += 2) {
+      const uint2 k = *reinterpret_cast<const uint2*>(src + i);
+      ++counter(k.x);
+      ++counter(k.y);
+    }
+    if ((end - begin) & 1) ++counter(src[end - 1]);
+    __syncthreads();
+    uint4* mine = reinterpret_cast<uint4*>(table + tid * kRake);
+    const uint4 u = mine[0], v = mine[1];
+    const unsigned int c[kRake] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+    unsigned int sum = 0;
+#pragma unroll
+    for (int j = 0; j < kRake; ++j) sum += c[j];
+    unsigned int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned int up = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += up;
+    }
+    if (lane == 31) warp_sum[warp] = incl;
+    __syncthreads();
+    unsigned int base = incl - sum, total = 0;
+#pragma unroll
+    for (int w = 0; w < NT / 32; ++w) {
+      const unsigned int t = warp_sum[w];
+      base += w < warp ? t : 0;
+      total += t;
+    }
+    base += total << 16;  // the digits 8 to 15 come after all lower ones
+    unsigned int p[kRake];
+#pragma unroll
+    for (int j = 0; j < kRake; ++j) {
+      p[j] = base;
+      base += c[j];
+    }
+    mine[0] = make_uint4(p[0], p[1], p[2], p[3]);
+    mine[1] = make_uint4(p[4], p[5], p[6], p[7]);
+    __syncthreads();
+    for (int i = begin; i + 1 < end; i += 2) {
+      const uint2 k = *reinterpret_cast<const uint2*>(src + i);
+      dst[counter(k.x)++] = k.x;
+      dst[counter(k.y)++] = k.y;
+    }
+    if ((end - begin) & 1) dst[counter(src[end - 1])] = src[end - 1];
+    __syncthreads();
+    uint32_t* t = src;
+    src = dst;
+    dst = t;
+  }
+  return src;
+}
+
+template <int NT>
+__global__ void __launch_bounds__(NT)
+    mesh_stats32_kernel(const float* __restrict__ in, const unsigned char* __restrict__ mask,
+                        const __grid_constant__ MeshArgs a, int capacity, MeshOut o) {
+  extern __shared__ __align__(16) unsigned long long skeys[];
+  __shared__ unsigned int count, all, any;
+  __shared__ MeshShared sh;
+  uint32_t* keys = reinterpret_cast<uint32_t*>(skeys);
+  uint32_t* other = keys + capacity;
+  unsigned int* table = other + capacity;
+  const int ndim = a.ndim, lane = threadIdx.x & 31;
+  for (long long mesh = blockIdx.x; mesh < a.mesh_len; mesh += gridDim.x) {
+    long long start[kMaxMeshRank], extent[kMaxMeshRank];
+    long long rest = mesh, volume = 1;
+    for (int d = ndim - 1; d >= 0; --d) {
+      const long long k = rest % a.mesh_shape[d];
+      rest /= a.mesh_shape[d];
+      start[d] = k * a.box[d];
+      extent[d] = min(start[d] + a.box[d], a.shape[d]) - start[d];
+      volume *= extent[d];
+    }
+    if (threadIdx.x == 0) {
+      count = 0;
+      all = ~0u;
+      any = 0;
+    }
+    __syncthreads();
+    // Pieces of 32 samples along the last axis go to warps (the mesh has at most
+    // 16,384 samples, so its indices are small).
+    const int width = (int)extent[ndim - 1], pieces = (width + 31) / 32;
+    const int items = (int)volume / width * pieces;
+    uint32_t k_and = ~0u, k_or = 0;
+    for (int item = threadIdx.x >> 5; item < items; item += NT / 32) {
+      int q = item / pieces;
+      const int x = (item - q * pieces) * 32 + lane;
+      long long offset = start[ndim - 1] + x, stride = a.shape[ndim - 1];
+      for (int d = ndim - 2; d >= 0; --d) {
+        const int e = (int)extent[d], c = d > 0 ? q % e : q;
+        offset += (start[d] + c) * stride;
+        q /= e;
+        stride *= a.shape[d];
+      }
+      bool take = x < width;
+      float v = 0.0f;
+      if (take) {
+        v = __ldg(in + offset);
+        take = isfinite(v) && !(mask && mask[offset]);
+      }
+      const unsigned int taken = __ballot_sync(0xffffffffu, take);
+      unsigned int at = 0;
+      if (lane == 0 && taken) at = atomicAdd(&count, (unsigned int)__popc(taken));
+      at = __shfl_sync(0xffffffffu, at, 0);
+      if (take) {
+        const uint32_t key = KeyOf<float>::key(v);
+        keys[at + __popc(taken & ((1u << lane) - 1u))] = key;
+        k_and &= key;
+        k_or |= key;
+      }
+    }
+    k_and = __reduce_and_sync(0xffffffffu, k_and);
+    k_or = __reduce_or_sync(0xffffffffu, k_or);
+    if (lane == 0) {
+      atomicAnd(&all, k_and);
+      atomicOr(&any, k_or);
+    }
+    __syncthreads();
+    const int n = (int)count;
+    uint32_t* sorted = m_sort<NT>(keys, other, n, table, n > 0 ? all ^ any : 0u);
+    float* values = reinterpret_cast<float*>(sorted);
+    for (int i = threadIdx.x; i < n; i += NT) values[i] = KeyOf<float>::value(sorted[i]);
+    __syncthreads();
+    m_finish(SVF{values}, n, volume, a, o, mesh, sh);
     __syncthreads();
   }
 }
@@ -1070,12 +1329,20 @@ int run_device(const T* d_in, const uint8_t* d_mask, const Rules& r, T* d_bg, T*
     for (int d = 0; d < a.ndim; ++d) largest *= std::min(r.box[d], r.shape[d]);
     long long padded = 1;
     while (padded < largest) padded <<= 1;
+    // Float32 meshes that fit sort 32-bit keys (two buffers and the counters);
+    // 512 threads where few such blocks share an SM.
+    const long long capacity32 = (largest + 3) / 4 * 4;
+    const bool keys32 = sizeof(T) == 4 && largest <= 16384;
+    const int threads32 = largest <= 4096 ? 128 : 512;
+    const size_t smem32 = (size_t)capacity32 * 8 + (size_t)threads32 * 32;
     // One block per mesh when the sort fits in shared memory; otherwise the
     // blocks share a bounded global workspace and stride over the meshes.
     long long blocks = std::min(m, (long long)INT_MAX);
     unsigned long long* scratch = nullptr;
     size_t smem = 0;
-    if (padded * 8 <= std::min((long long)smem_optin, kMeshSmemBytes)) {
+    if (keys32) {
+      a.capacity = 0;
+    } else if (padded * 8 <= std::min((long long)smem_optin, kMeshSmemBytes)) {
       smem = (size_t)padded * 8;
       a.capacity = 0;
     } else {
@@ -1091,9 +1358,15 @@ int run_device(const T* d_in, const uint8_t* d_mask, const Rules& r, T* d_bg, T*
     if (e == cudaSuccess) e = buf.alloc(&o.retained, (size_t)m * 8);
     if (e == cudaSuccess) e = buf.alloc(&o.valid, (size_t)m);
     if (e != cudaSuccess) return fail(NDF_ERR_MEMORY, "unable to allocate mesh workspace");
-    auto k = mesh_stats_kernel<T>;
-    if ((e = allow_max_smem((const void*)k)) != cudaSuccess) return cuda_fail(e, "mesh statistics");
-    k<<<(unsigned)blocks, kMThreads, smem, s>>>(d_in, d_mask, a, scratch, o);
+    if (keys32) {
+      auto k = threads32 == 128 ? mesh_stats32_kernel<128> : mesh_stats32_kernel<512>;
+      if ((e = allow_max_smem((const void*)k)) != cudaSuccess) return cuda_fail(e, "mesh statistics");
+      k<<<(unsigned)blocks, threads32, smem32, s>>>(reinterpret_cast<const float*>(d_in), d_mask, a, (int)capacity32, o);
+    } else {
+      auto k = mesh_stats_kernel<T>;
+      if ((e = allow_max_smem((const void*)k)) != cudaSuccess) return cuda_fail(e, "mesh statistics");
+      k<<<(unsigned)blocks, kMThreads, smem, s>>>(d_in, d_mask, a, scratch, o);
+    }
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(bg.data(), o.background, (size_t)m * 8, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(rms.data(), o.rms, (size_t)m * 8, cudaMemcpyDeviceToHost, s);
