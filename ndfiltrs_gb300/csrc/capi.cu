@@ -633,6 +633,7 @@ int apply_candidate_impl(Plan& p, const Candidate& c, int smem_limit) {
       return NDF_OK;
     case Algo::kExtremaPasses: {
       if (!extrema_passes_configure(p, smem_limit)) return fail(NDF_ERR_UNSUPPORTED, "window too large");
+      if (p.scratch_bytes == 0) return NDF_OK;
       cudaError_t e = cudaMalloc(&p.d_scratch, p.scratch_bytes);
       if (e != cudaSuccess) {
         cudaGetLastError();

@@ -5,8 +5,10 @@
 // policies, min_count), because a window's minimum is the minimum of its
 // column minima and every comparison runs on order-preserving keys.
 //
-// GB300 design, two kernels:
-//  * extrema_pass_kernel (the default): two launches of one column pass.
+// GB300 design, three kernels:
+//  * extrema_strip_kernel (the default up to 129 x 129 without counts): both
+//    axes in one pass over the array, a warp per strip of 64 columns.
+//  * extrema_pass_kernel: two launches of one column pass.
 //    Each block takes a strip of 32 columns and R rows, stages those rows
 //    plus the window halo (through the boundary mode) as keys, runs van Herk
 //    down every column in blocks of the window length (prefix and suffix
@@ -151,6 +153,229 @@ __global__ void __launch_bounds__(kEThreads)
     const bool missing = red.omit ? ((long long)n < red.min_count) : ((int)n != red.count);
     const T v = (missing || n == 0) ? nan_of(T()) : KO::value(MAXIMUM ? ~m : m);
     out[(z * g.H + gy) * g.W + gx] = canonical(v);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Both axes in one pass. A warp takes a strip of 64 output columns and walks
+// down a segment of rows. Lane l holds the columns l + 32 i of a support row in
+// registers; the minima along the row come from doubling (spans of 1, 2, 4 ...
+// columns, then two spans that cover the window), each step a shuffle per
+// register. Down the columns it is van Herk's scheme as a stream: within blocks
+// of kh rows, the running minimum of the block so far joins the suffix minimum
+// of the block before. The suffix minima live in shared memory, and the row
+// minima of the current block take their places as they are used up, so a warp
+// needs kh x 64 keys and no barrier.
+// The two column passes staged every sample in shared memory twice, wrote a
+// transposed key array in between and issued 230 warp instructions per 32 outputs:
+// 181 us for 31 x 31 on 4096^2 float32, 103 us here.
+constexpr int kStripWidth = 64;
+constexpr int kStripWarps = 4;     // most warps per block (tall windows take fewer: each holds kh x 64 keys)
+constexpr int kStripMax = 129;  // largest window side
+
+template <typename K>
+__device__ __forceinline__ K shift_left(K a, K b, int s) {
+  // Column l + s of the 64 columns (a, b), for lane l: lanes below s serve b's.
+  const int lane = threadIdx.x & 31;
+  return __shfl_sync(0xffffffffu, lane >= s ? a : b, (lane + s) & 31);
+}
+
+template <typename K>
+__device__ __forceinline__ K least(K a, K b) {
+  return a < b ? a : b;
+}
+
+// NR registers hold 32 NR columns; afterwards the first two hold the minima of
+// k columns from each of the first 64 columns on. Columns past 32 NR are never
+// part of those.
+template <typename K, int NR>
+__device__ __forceinline__ void row_minima(K (&v)[NR], int k) {
+  int span = 1;
+#pragma unroll
+  for (int s = 1; s < 32; s <<= 1) {
+    if (2 * s > k) break;
+#pragma unroll
+    for (int i = 0; i < NR; ++i) v[i] = least(v[i], shift_left(v[i], v[i + 1 < NR ? i + 1 : i], s));
+    span = 2 * s;
+  }
+  if (NR > 3 && k >= 64) {
+#pragma unroll
+    for (int i = 0; i + 1 < NR; ++i) v[i] = least(v[i], v[i + 1]);
+    span = 64;
+  }
+  if (NR > 5 && k >= 128) {
+#pragma unroll
+    for (int i = 0; i + 2 < NR; ++i) v[i] = least(v[i], v[i + 2]);
+    span = 128;
+  }
+  // The window's last span starts k - span columns on.
+  const int rest = k - span, words = rest >> 5, s = rest & 31;
+  if (rest == 0) return;
+  K a[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    a[i] = v[i < NR ? i : NR - 1];
+    if (NR > 3 && words == 1) a[i] = v[i + 1 < NR ? i + 1 : NR - 1];
+    if (NR > 4 && words >= 2) a[i] = v[i + 2 < NR ? i + 2 : NR - 1];
+  }
+  const K m0 = least(v[0], shift_left(a[0], a[1], s)), m1 = least(v[1], shift_left(a[1], a[2], s));
+  v[0] = m0;
+  v[1] = m1;
+}
+
+template <typename T, bool MAXIMUM, int NR>
+__global__ void __launch_bounds__(kStripWarps * 32)
+    extrema_strip_kernel(const T* __restrict__ in, T* __restrict__ out, const __grid_constant__ Geom3 g,
+                         const __grid_constant__ Reduce r, int rows_per, long long strips, long long items) {
+  using KO = KeyOf<T>;
+  using K = typename KO::K;
+  constexpr K kNone = KO::kSentinel;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long item = blockIdx.x * (long long)(blockDim.x >> 5) + warp;
+  if (item >= items) return;
+  const int kh = g.kh, kw = g.kw;
+  K* suffix = reinterpret_cast<K*>(smem_raw) + (size_t)warp * kh * kStripWidth + lane;
+  const long long x0 = (item % strips) * kStripWidth, y0 = (item / strips) * rows_per;
+  const int rows = (int)min((long long)rows_per, g.H - y0);
+  const bool omit = r.omit, drop_inf = r.drop_inf;
+  auto conv = [&](T v) -> K {
+    if (isnan(v)) return omit ? kNone : (K)0;
+    if (drop_inf && isinf(v)) return kNone;
+    const K key = KO::key(v);
+    return MAXIMUM ? (K)~key : key;
+  };
+  const T cval = (T)r.cval;
+  long long column[NR];
+#pragma unroll
+  for (int i = 0; i < NR; ++i) {
+    long long m;
+    column[i] = map_index(x0 + lane + 32 * i - g.ax, g.W, g.mx, &m) ? m : -1;
+  }
+  const bool store0 = x0 + lane < g.W, store1 = x0 + lane + 32 < g.W;
+  auto load = [&](long long row, T (&t)[NR]) {
+    long long m;
+    const bool inside = map_index(row, g.H, g.my, &m);
+    const T* src = in + (inside ? m * g.W : 0);
+#pragma unroll
+    for (int i = 0; i < NR; ++i) t[i] = inside && column[i] >= 0 ? __ldg(src + column[i]) : cval;
+  };
+  const int total = rows + kh - 1;
+  K p0 = kNone, p1 = kNone;
+  T* dst = out + (y0 - (kh - 1)) * g.W + x0 + lane;
+  int j = 0;  // place in the block of kh rows
+  auto step = [&](const T (&t)[NR], int i) {
+    K v[NR];
+#pragma unroll
+    for (int q = 0; q < NR; ++q) v[q] = conv(t[q]);
+    row_minima<K, NR>(v, kw);
+    p0 = j == 0 ? v[0] : least(p0, v[0]);
+    p1 = j == 0 ? v[1] : least(p1, v[1]);
+    K m0 = p0, m1 = p1;
+    if (j + 1 < kh && i >= kh) {
+      m0 = least(m0, suffix[(j + 1) * kStripWidth]);
+      m1 = least(m1, suffix[(j + 1) * kStripWidth + 32]);
+    }
+    suffix[j * kStripWidth] = v[0];
+    suffix[j * kStripWidth + 32] = v[1];
+    if (i >= kh - 1) {
+      auto value = [&](K m) -> T {
+        return m == kNone || m == (K)0 ? nan_of(T()) : canonical(KO::value(MAXIMUM ? (K)~m : m));
+      };
+      if (store0) dst[0] = value(m0);
+      if (store1) dst[32] = value(m1);
+    }
+    dst += g.W;
+    if (++j == kh) {
+      // The block is complete: its suffix minima.
+      K s0 = v[0], s1 = v[1];
+#pragma unroll 4
+      for (int q = kh - 2; q > 0; --q) {
+        s0 = least(s0, suffix[q * kStripWidth]);
+        s1 = least(s1, suffix[q * kStripWidth + 32]);
+        suffix[q * kStripWidth] = s0;
+        suffix[q * kStripWidth + 32] = s1;
+      }
+      j = 0;
+    }
+  };
+  // Rows are loaded kAhead steps early, which hides their latency from the
+  // warp's chain of steps.
+  constexpr int kAhead = sizeof(T) == 4 ? 4 : 2;
+  T rows_ahead[kAhead][NR];
+#pragma unroll
+  for (int q = 0; q < kAhead; ++q)
+    if (q < total) load(y0 + q - g.ay, rows_ahead[q]);
+  for (int i = 0; i < total; i += kAhead) {
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q) {
+      if (i + q >= total) break;
+      T now[NR];
+#pragma unroll
+      for (int c = 0; c < NR; ++c) now[c] = rows_ahead[q][c];
+      if (i + q + kAhead < total) load(y0 + i + q + kAhead - g.ay, rows_ahead[q]);
+      step(now, i + q);
+    }
+  }
+}
+
+// Warps per block: fewer for tall windows, whose keys fill shared memory.
+int strip_warps(size_t per_warp) {
+  int warps = kStripWarps;
+  while (warps > 1 && warps * per_warp > 48 * 1024) warps /= 2;
+  return warps;
+}
+
+// Rows per warp, or 0 when the two passes serve the window better. As many
+// warps as are resident at once (16 per SM, or the whole blocks that shared
+// memory lets in: one block more is a second turn, 0.31 against 0.18 ms at 65 x 65)
+// share the rows; each repeats kh - 1. Measured on 4096^2: 31 x 31 float32
+// 0.103 ms with 16 warps per SM against 0.181 for the passes, 97 x 97 0.279 with
+// 8 against 0.383, float64 31 x 31 0.249 against 0.322. A warp walks its rows one
+// after the other, about 0.6 us each at first, so arrays whose segments would be
+// shorter than twice the window (2.5 times for float64, whose shuffles are
+// double) are faster in passes (31 x 31 on 2000 x 1500: 0.041 against 0.033 ms), except
+// for the short walks of windows of up to 15 rows of float32.
+int strip_rows(const Plan& p) {
+  const Geom3& g = p.tile.g;
+  if (g.kh > kStripMax || g.kw > kStripMax || (p.r.omit && p.r.min_count > 1)) return 0;
+  const long long key = p.dtype == 0 ? 4 : 8;
+  const long long strips = (g.W + kStripWidth - 1) / kStripWidth;
+  const size_t per_warp = (size_t)(g.kh * kStripWidth * key);
+  const int warps = strip_warps(per_warp);
+  const long long resident = std::max(1ll, std::min(16ll, (long long)(227 * 1024 / (warps * per_warp + 1024)) * warps));
+  const long long segments = std::max(1ll, std::max(1, p.sm_count) * resident / strips);
+  long long rows = (g.H + segments - 1) / segments;
+  rows = std::max<long long>(rows, std::min<long long>(g.H, std::max(16, g.kh)));
+  const bool long_enough = p.dtype == 0 ? rows >= 2ll * g.kh || g.kh <= 15 : 2 * rows >= 5ll * g.kh;
+  return long_enough ? (int)std::min<long long>(rows, 1 << 20) : 0;
+}
+
+template <typename T, bool MAXIMUM, int NR>
+cudaError_t launch_strip_n(const Plan& p, const T* in, T* out, cudaStream_t s) {
+  using K = typename KeyOf<T>::K;
+  const Geom3& g = p.tile.g;
+  auto kernel = extrema_strip_kernel<T, MAXIMUM, NR>;
+  cudaError_t e = allow_max_smem((const void*)kernel);
+  if (e != cudaSuccess) return e;
+  const long long strips = (g.W + kStripWidth - 1) / kStripWidth;
+  const long long items = strips * ((g.H + p.ext_strip - 1) / p.ext_strip);
+  const size_t per_warp = (size_t)g.kh * kStripWidth * sizeof(K);
+  const int warps = strip_warps(per_warp);
+  kernel<<<(unsigned)((items + warps - 1) / warps), warps * 32, warps * per_warp, s>>>(in, out, g, p.r, p.ext_strip,
+                                                                                      strips, items);
+  return cudaGetLastError();
+}
+
+template <typename T, bool MAXIMUM>
+cudaError_t launch_strip(const Plan& p, const T* in, T* out, cudaStream_t s) {
+  // 64 columns and the kw - 1 that windows reach beyond them.
+  switch ((kStripWidth + p.tile.g.kw - 1 + 31) / 32) {
+    case 2: return launch_strip_n<T, MAXIMUM, 2>(p, in, out, s);
+    case 3: return launch_strip_n<T, MAXIMUM, 3>(p, in, out, s);
+    case 4: return launch_strip_n<T, MAXIMUM, 4>(p, in, out, s);
+    case 5: return launch_strip_n<T, MAXIMUM, 5>(p, in, out, s);
+    default: return launch_strip_n<T, MAXIMUM, 6>(p, in, out, s);
   }
 }
 
@@ -341,6 +566,8 @@ cudaError_t launch_passes_t(const Plan& p, const T* in, T* out, cudaStream_t s) 
 
 template <typename T>
 cudaError_t launch_passes(const Plan& p, const T* in, T* out, cudaStream_t s) {
+  if (p.ext_strip > 0)
+    return p.r.kind == kMax ? launch_strip<T, true>(p, in, out, s) : launch_strip<T, false>(p, in, out, s);
   const bool maximum = p.r.kind == kMax, count = p.r.omit && p.r.min_count > 1;
   if (maximum) return count ? launch_passes_t<T, true, true>(p, in, out, s) : launch_passes_t<T, true, false>(p, in, out, s);
   return count ? launch_passes_t<T, false, true>(p, in, out, s) : launch_passes_t<T, false, false>(p, in, out, s);
@@ -409,6 +636,9 @@ bool extrema_passes_configure(Plan& p, int smem_limit) {
   const Geom3& g = p.tile.g;
   if (p.ndim > 2 || g.D != 1 || !p.footprint.empty()) return false;
   if (p.r.kind != kMin && p.r.kind != kMax) return false;
+  p.ext_strip = strip_rows(p);
+  p.scratch_bytes = 0;
+  if (p.ext_strip > 0) return true;
   const bool count = p.r.omit && p.r.min_count > 1;
   if (count && (long long)g.kh * g.kw > 65535) return false;
   auto rows = [&](int k) {
