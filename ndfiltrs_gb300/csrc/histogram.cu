@@ -54,6 +54,7 @@ constexpr int kHWarps = kHThreads / 32;
 constexpr uint16_t kOmitted = 0xFFFF;
 constexpr uint16_t kPropagated = 0xFFFE;
 constexpr int kMaxSupport = 65534;
+constexpr unsigned int kFull = 0xffffffffu;
 
 struct HistArgs {
   Geom3 g;
@@ -77,13 +78,36 @@ struct HistArgs {
   int nf, nv, nh;
 };
 
-// A block's sort slot: ping-pong keys and 16-bit payloads (support indices).
+// A block's sort slot: two arrays of keys with their support indices. A key and
+// its index lie together, so that the scatter of a pass writes one 32-byte
+// sector per sample (apart they wrote two, and those stores bound the sort:
+// 6.9 of the 14.0 ms of a (9, 33, 33) median of a 64 x 512 x 512 cube; 13.1 ms now).
+template <typename K>
+struct Entry;
+template <>
+struct __align__(8) Entry<uint32_t> {
+  uint32_t key;
+  uint32_t at;
+};
+template <>
+struct __align__(16) Entry<unsigned long long> {
+  unsigned long long key;
+  unsigned long long at;
+};
+
+// The sorted keys of a footprint's support: the decode table, or every second
+// word of a slot's entries.
+template <typename K>
+struct SortedKeys {
+  const K* p;
+  int step;
+  __device__ __forceinline__ K operator[](int rank) const { return p[rank * step]; }
+};
+
 template <typename K>
 struct Slot {
-  K* keys_a;
-  K* keys_b;
-  uint16_t* pay_a;
-  uint16_t* pay_b;
+  Entry<K>* a;
+  Entry<K>* b;
 };
 
 __host__ __device__ inline long long align16(long long v) { return (v + 15) & ~15ll; }
@@ -96,55 +120,37 @@ __host__ __device__ inline long long box_map_bytes(int SH, int SZ, int SW) {
 
 template <typename K>
 __host__ __device__ inline long long slot_bytes_for(int S) {
-  return 2 * align16((long long)S * sizeof(K)) + 2 * align16((long long)S * 2);
+  return 2 * align16((long long)S * sizeof(Entry<K>));
 }
 
 template <typename K>
 __device__ inline Slot<K> slot_at(unsigned char* base, int S) {
-  Slot<K> s;
-  long long off = 0;
-  s.keys_a = reinterpret_cast<K*>(base + off);
-  off += align16((long long)S * sizeof(K));
-  s.keys_b = reinterpret_cast<K*>(base + off);
-  off += align16((long long)S * sizeof(K));
-  s.pay_a = reinterpret_cast<uint16_t*>(base + off);
-  off += align16((long long)S * 2);
-  s.pay_b = reinterpret_cast<uint16_t*>(base + off);
-  return s;
+  return {reinterpret_cast<Entry<K>*>(base), reinterpret_cast<Entry<K>*>(base + align16((long long)S * sizeof(Entry<K>)))};
 }
 
 // Accesses to the sort slots in global memory with an L2 evict-last policy.
-// A block rewrites its slot on every radix pass; together the slots hold
-// (grid) x S x 12 bytes (67 MB for 152 blocks of 36,864 samples), which fits
-// in the 126 MB L2, and the hint keeps them there against the input stream
-// (read with evict-first loads), so the ping-pong does not reach DRAM.
+// A block rewrites its slot on every radix pass; the hint keeps the slots in
+// L2 against the input stream (the support's samples), so that most of the
+// ping-pong does not reach DRAM.
 __device__ __forceinline__ unsigned long long keep_policy() {
   unsigned long long p;
   asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
   return p;
 }
-__device__ __forceinline__ void st_keep(uint32_t* a, uint32_t v, unsigned long long p) {
-  asm volatile("st.global.L2::cache_hint.b32 [%0], %1, %2;" ::"l"(a), "r"(v), "l"(p) : "memory");
+__device__ __forceinline__ void st_keep(Entry<uint32_t>* a, Entry<uint32_t> v, unsigned long long p) {
+  asm volatile("st.global.L2::cache_hint.v2.b32 [%0], {%1, %2}, %3;" ::"l"(a), "r"(v.key), "r"(v.at), "l"(p) : "memory");
 }
-__device__ __forceinline__ void st_keep(unsigned long long* a, unsigned long long v, unsigned long long p) {
-  asm volatile("st.global.L2::cache_hint.b64 [%0], %1, %2;" ::"l"(a), "l"(v), "l"(p) : "memory");
+__device__ __forceinline__ void st_keep(Entry<unsigned long long>* a, Entry<unsigned long long> v, unsigned long long p) {
+  asm volatile("st.global.L2::cache_hint.v2.b64 [%0], {%1, %2}, %3;" ::"l"(a), "l"(v.key), "l"(v.at), "l"(p) : "memory");
 }
-__device__ __forceinline__ void st_keep(uint16_t* a, uint16_t v, unsigned long long p) {
-  asm volatile("st.global.L2::cache_hint.b16 [%0], %1, %2;" ::"l"(a), "h"(v), "l"(p) : "memory");
-}
-__device__ __forceinline__ uint32_t ld_keep(const uint32_t* a, unsigned long long p) {
-  uint32_t v;
-  asm volatile("ld.global.L2::cache_hint.b32 %0, [%1], %2;" : "=r"(v) : "l"(a), "l"(p) : "memory");
+__device__ __forceinline__ Entry<uint32_t> ld_keep(const Entry<uint32_t>* a, unsigned long long p) {
+  Entry<uint32_t> v;
+  asm volatile("ld.global.L2::cache_hint.v2.b32 {%0, %1}, [%2], %3;" : "=r"(v.key), "=r"(v.at) : "l"(a), "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ unsigned long long ld_keep(const unsigned long long* a, unsigned long long p) {
-  unsigned long long v;
-  asm volatile("ld.global.L2::cache_hint.b64 %0, [%1], %2;" : "=l"(v) : "l"(a), "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ uint16_t ld_keep(const uint16_t* a, unsigned long long p) {
-  uint16_t v;
-  asm volatile("ld.global.L2::cache_hint.b16 %0, [%1], %2;" : "=h"(v) : "l"(a), "l"(p) : "memory");
+__device__ __forceinline__ Entry<unsigned long long> ld_keep(const Entry<unsigned long long>* a, unsigned long long p) {
+  Entry<unsigned long long> v;
+  asm volatile("ld.global.L2::cache_hint.v2.b64 {%0, %1}, [%2], %3;" : "=l"(v.key), "=l"(v.at) : "l"(a), "l"(p) : "memory");
   return v;
 }
 
@@ -154,15 +160,12 @@ __host__ __device__ inline long long sort_table_words(int nd) { return (long lon
 
 // One stable counting pass over `nd`-valued digits. `table` holds
 // kHWarps x nd counters, `totals` nd. Each warp owns a contiguous segment
-// and ranks its 32-key chunks in order with match_any, so equal digits keep
-// their order. Loads are batched (kBatch keys per lane in registers) so a
+// and ranks its 32-entry chunks in order, so equal digits keep their order. Loads are batched (kBatch entries per lane in registers) so a
 // pass costs one memory round trip per batch rather than one per chunk.
-constexpr int kBatch = 16;
-
 template <typename K, typename Digit>
-__device__ void radix_pass(const K* src_k, const uint16_t* src_p, K* dst_k, uint16_t* dst_p, int S,
-                           unsigned int* table, unsigned int* totals, int nd, Digit digit,
-                           unsigned long long keep) {
+__device__ void radix_pass(const Entry<K>* src, Entry<K>* dst, int S, unsigned int* table, unsigned int* totals,
+                           int nd, Digit digit, unsigned long long keep) {
+  constexpr int kBatch = sizeof(K) == 4 ? 8 : 4;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int i = threadIdx.x; i < kHWarps * nd; i += blockDim.x) table[i] = 0;
   __syncthreads();
@@ -171,15 +174,23 @@ __device__ void radix_pass(const K* src_k, const uint16_t* src_p, K* dst_k, uint
   const int end = min(S, begin + chunk);
   unsigned int* wt = table + warp * nd;
   for (int b = begin; b < end; b += 32 * kBatch) {
-    K keys[kBatch];
+    Entry<K> e[kBatch];
 #pragma unroll
     for (int j = 0; j < kBatch; ++j) {
       const int i = b + j * 32 + lane;
-      keys[j] = i < end ? ld_keep(src_k + i, keep) : K(0);
+      e[j] = i < end ? ld_keep(src + i, keep) : Entry<K>{0, 0};
     }
 #pragma unroll
-    for (int j = 0; j < kBatch; ++j)
-      if (b + j * 32 + lane < end) atomicAdd(&wt[digit(keys[j])], 1u);
+    for (int j = 0; j < kBatch; ++j) {
+      // A digit that many lanes share (the top ones are alike) is added once.
+      const bool valid = b + j * 32 + lane < end;
+      const int d = valid ? (int)digit(e[j].key) : -1;
+      const int first = __shfl_sync(kFull, d, 0);
+      const unsigned int same = __ballot_sync(kFull, d == first);
+      const bool shared = __popc(same) >= 8;
+      if (shared && lane == 0 && valid) atomicAdd(&wt[d], (unsigned int)__popc(same));
+      if (valid && (!shared || d != first)) atomicAdd(&wt[d], 1u);
+    }
   }
   __syncthreads();
   for (int d = threadIdx.x; d < nd; d += blockDim.x) {
@@ -216,29 +227,35 @@ __device__ void radix_pass(const K* src_k, const uint16_t* src_p, K* dst_k, uint
   }
   __syncthreads();
   for (int b = begin; b < end; b += 32 * kBatch) {
-    K keys[kBatch];
-    uint16_t pays[kBatch];
+    Entry<K> e[kBatch];
 #pragma unroll
     for (int j = 0; j < kBatch; ++j) {
       const int i = b + j * 32 + lane;
-      keys[j] = i < end ? ld_keep(src_k + i, keep) : K(0);
-      pays[j] = i < end ? ld_keep(src_p + i, keep) : uint16_t(0);
+      e[j] = i < end ? ld_keep(src + i, keep) : Entry<K>{0, 0};
+    }
+    // Lanes with equal digits by a ballot per digit bit (the match instruction
+    // takes its pipe some 46 clocks a warp).
+    unsigned int peers[kBatch];
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) peers[j] = __ballot_sync(kFull, b + j * 32 + lane < end);
+    for (int bit = 1; bit < nd; bit <<= 1) {
+#pragma unroll
+      for (int j = 0; j < kBatch; ++j) {
+        const bool set = (digit(e[j].key) & bit) != 0;
+        const unsigned int with = __ballot_sync(kFull, set);
+        peers[j] &= set ? with : ~with;
+      }
     }
 #pragma unroll
     for (int j = 0; j < kBatch; ++j) {
       const bool valid = b + j * 32 + lane < end;
-      const int d = valid ? (int)digit(keys[j]) : nd + lane;
-      const unsigned int peers = __match_any_sync(0xffffffffu, d);
-      const int before = __popc(peers & ((1u << lane) - 1u));
-      unsigned int pos = 0;
-      if (valid) pos = wt[d] + before;
+      const unsigned int d = digit(e[j].key);
+      unsigned int at = 0;
+      if (valid) at = wt[d];
       __syncwarp();
-      if (valid && lane == 31 - __clz(peers)) wt[d] += __popc(peers);
+      if (valid && lane == 31 - __clz(peers[j])) wt[d] = at + __popc(peers[j]);
       __syncwarp();
-      if (valid) {
-        st_keep(dst_k + pos, keys[j], keep);
-        st_keep(dst_p + pos, pays[j], keep);
-      }
+      if (valid) st_keep(dst + at + __popc(peers[j] & ((1u << lane) - 1u)), e[j], keep);
     }
   }
   __syncthreads();
@@ -273,7 +290,6 @@ __device__ __forceinline__ int select_in_word32(unsigned int word, int k) {
 // warp are done, so the two halves stay converged.
 constexpr int kSeg = 16;
 constexpr int kSegs = kHThreads / kSeg;
-constexpr unsigned int kFull = 0xffffffffu;
 constexpr int kSeqWords = 16;
 
 struct SegHist {
@@ -594,7 +610,7 @@ struct OutPipe {
     held_at = -1;
   }
   // Complete the held batch, then load the parked one's keys and hold it.
-  __device__ __forceinline__ void rotate(const HistArgs& a, const K* sorted, T* __restrict__ out) {
+  __device__ __forceinline__ void rotate(const HistArgs& a, SortedKeys<K> sorted, T* __restrict__ out) {
     complete(a, out);
     if (next_at >= 0) {
       kl = next.valid ? sorted[next.lo] : K(0);
@@ -616,7 +632,7 @@ template <typename T, bool PROPAGATE>
 __device__ __forceinline__ void walk(const uint16_t* codes, const uint16_t* lists, int c_begin,
                                      int ncols, int tw_eff, int th_eff, int SW,
                                      long long y0, long long x0, const Geom3& g, const HistArgs& a,
-                                     const typename KeyOf<T>::K* sorted, T* __restrict__ out,
+                                     SortedKeys<typename KeyOf<T>::K> sorted, T* __restrict__ out,
                                      SegHist& h) {
   const uint16_t* top = lists + a.nf;
   const uint16_t* bottom = top + a.nv;
@@ -1307,7 +1323,7 @@ __device__ __forceinline__ void histogram_tile(const T* __restrict__ in, T* __re
       ++sent;
     }
   };
-  const K* sorted = nullptr;
+  SortedKeys<K> sorted{nullptr, 0};
   if (!FP && a.in_smem) {
     sup.each([&](int, K key) { note(key); });
     const KeyBits<K> bits = block_bits<K>(k_and, k_or, sent, S);
@@ -1331,8 +1347,7 @@ __device__ __forceinline__ void histogram_tile(const T* __restrict__ in, T* __re
     Slot<K> slot = slot_at<K>(scratch_slot, S);
     const unsigned long long keep = keep_policy();
     sup.each([&](int e, K key) {
-      st_keep(slot.keys_a + e, key, keep);
-      st_keep(slot.pay_a + e, (uint16_t)e, keep);
+      st_keep(slot.a + e, Entry<K>{key, (K)e}, keep);
       note(key);
     });
     const KeyBits<K> bits = block_bits<K>(k_and, k_or, sent, S);
@@ -1341,10 +1356,8 @@ __device__ __forceinline__ void histogram_tile(const T* __restrict__ in, T* __re
     // dropped samples' all-ones keys take part like any other key: an LSD
     // sort orders the retained keys among themselves whatever lies between
     // them, and a dropped sample's position is never set in a histogram.
-    K* src_k = slot.keys_a;
-    K* dst_k = slot.keys_b;
-    uint16_t* src_p = slot.pay_a;
-    uint16_t* dst_p = slot.pay_b;
+    Entry<K>* src = slot.a;
+    Entry<K>* dst = slot.b;
     if (bits.varying != 0) {
       const int lo = lowest_set(bits.varying), hi = highest_set(bits.varying);
       // The fewest passes, with the smallest digits that still cover the bits.
@@ -1353,24 +1366,22 @@ __device__ __forceinline__ void histogram_tile(const T* __restrict__ in, T* __re
       const int nd = 1 << digits;
       const K mask = (K)(nd - 1);
       for (int shift = lo; shift <= hi; shift += digits) {
-        radix_pass(src_k, src_p, dst_k, dst_p, S, work, work + kHWarps * nd, nd,
-                   [shift, mask](K key) { return (unsigned int)((key >> shift) & mask); }, keep);
-        K* tk = src_k;
-        src_k = dst_k;
-        dst_k = tk;
-        uint16_t* tp = src_p;
-        src_p = dst_p;
-        dst_p = tp;
+        radix_pass<K>(src, dst, S, work, work + kHWarps * nd, nd,
+                      [shift, mask](K key) { return (unsigned int)((key >> shift) & mask); }, keep);
+        Entry<K>* t = src;
+        src = dst;
+        dst = t;
       }
     }
     for (int pos = threadIdx.x; pos < S; pos += blockDim.x) {
-      const K key = ld_keep(src_k + pos, keep);
-      const uint16_t at = ld_keep(src_p + pos, keep);
+      const Entry<K> e = ld_keep(src + pos, keep);
+      const K key = e.key;
+      const uint16_t at = (uint16_t)e.at;
       codes_s[at] = key == kSent ? dropped : (uint16_t)pos;
       if (!FP) place_s[pos] = key == kSent ? (uint16_t)0xFFFF : at;
       if (SDEC) decode_s[pos] = key;
     }
-    sorted = SDEC ? decode_s : src_k;
+    sorted = {SDEC ? decode_s : &src->key, SDEC ? 1 : 2};
   }
   if (!FP && threadIdx.x < 64) lists_s[threadIdx.x < 32 ? (int)threadIdx.x : S + (int)threadIdx.x] = 0xFFFF;
   __syncthreads();
@@ -1928,10 +1939,11 @@ cudaError_t launch_histogram(const Plan& p, const void* in, void* out, cudaStrea
 // Limits and sharing:
 //  * the array holds kNoAllocScratchBytes (16 MiB) on every GPU that loads
 //    the library, until the process exits;
-//  * the number of concurrently working thread blocks is the number of sort
-//    slots that fit in it (a slot is 2 x S keys + 2 x S u32 payloads for a
-//    support of S samples), capped by the device's resident capacity; a
-//    support whose slot does not fit is rejected with NDF_ERR_MEMORY;
+//  * supports sorted in shared memory do not use it; for the others the number
+//    of concurrently working thread blocks is the number of sort slots that
+//    fit in it (a slot is 2 x S entries of a key and its index for a support
+//    of S samples), capped by the device's resident capacity; a support whose
+//    slot does not fit is rejected with NDF_ERR_MEMORY;
 //  * every call shares the array and it keeps the last call's contents; the
 //    kernel writes every slot word before reading it, so nothing needs
 //    clearing; calls that overlap on the GPU (other streams, other host
@@ -2083,8 +2095,9 @@ extern "C" int ndf_histogram_filter_noalloc(const void* d_in, void* d_out, int32
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kHThreads, smem);
   if (e != cudaSuccess) return cuda_fail(e, "histogram (allocation-free) set-up");
   long long slots = (long long)(kNoAllocScratchBytes / (size_t)a.slot_bytes);
-  long long grid = std::min<long long>(std::min<long long>(a.tiles, slots),
-                                       (long long)std::max(per_sm, 1) * sm_count);
+  const long long grid = a.in_smem ? std::min<long long>(a.tiles, INT_MAX)
+                                   : std::min<long long>(std::min<long long>(a.tiles, slots),
+                                                         (long long)std::max(per_sm, 1) * sm_count);
   cudaStream_t s = (cudaStream_t)stream;
   if (dtype == 0)
     histogram_kernel<float, false, false><<<(unsigned)grid, kHThreads, smem, s>>>(
