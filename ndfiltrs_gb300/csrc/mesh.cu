@@ -702,34 +702,111 @@ __global__ void spline_expand_kernel(const double* __restrict__ cur, const doubl
   next[idx] = tap_eval(taps[p], cur + base + j, second + base + j, inner);
 }
 
-// The last axis: one block per line; the line's second derivatives in
-// shared memory, then every output of the line in the output dtype.
+// The last axis, in the output dtype: a thread per output column takes its tap
+// once for `per` lines (eight, fewer for lines of many nodes). (One block per line had thread 0 solve the line's
+// second derivatives while the others waited, and read 160 KB of taps per line
+// of 4,096 outputs: 0.38 ms per 4096^2 float32 map, half of it the FP64 pipe's;
+// 0.06 now.)
+constexpr int kSplineLines = 8;
+constexpr size_t kSplineSmem = 200 * 1024;
+
+// A float64 as the sum of two floats (to 2^-49 of it).
+__host__ __device__ __forceinline__ float2 two_floats(double v) {
+#ifndef __CUDA_ARCH__
+  const float top = (float)v;
+  return make_float2(top, (float)(v - (double)top));
+#else
+  const float hi = __double2float_rn(v);
+  return make_float2(hi, __double2float_rn(__dsub_rn(v, (double)hi)));
+#endif
+}
+
+// A tap's weights and a node's value and second derivative as pairs of floats,
+// split once (the conversions run on the FP64 pipe too).
+struct FloatTap {
+  float4 ab, cd;
+};
+
+__global__ void spline_nodes_kernel(const double* __restrict__ cur, const double* __restrict__ second,
+                                    float4* __restrict__ node, long long n) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const float2 y = two_floats(cur[i]), m = two_floats(second[i]);
+    node[i] = make_float4(y.x, y.y, m.x, m.y);
+  }
+}
+
+// a b as p + e: the rounded product and the rest to 2^-47 of it.
+__device__ __forceinline__ float product(float2 a, float2 b, float& e) {
+  const float p = __fmul_rn(a.x, b.x);
+  e += __fmaf_rn(a.x, b.y, __fmaf_rn(a.y, b.x, __fmaf_rn(a.x, b.x, -p)));
+  return p;
+}
+
+// s + p exactly: the rounded sum, and its error added to e.
+__device__ __forceinline__ float sum_of(float s, float p, float& e) {
+  const float t = __fadd_rn(s, p), pp = __fsub_rn(t, s);
+  e += __fadd_rn(__fsub_rn(s, __fsub_rn(t, pp)), __fsub_rn(p, pp));
+  return t;
+}
+
+// Float32 outputs are the float32 rounding of the float64 sum of four products.
+// Pairs of floats give that sum to 2^-44 of the products' magnitudes; when the
+// rounding is the same 2^-40 above and below (all but one output in some 2^15)
+// it is the float64 sum's rounding too, else the output runs in float64.
 template <typename T>
-__global__ void spline_last_kernel(const double* __restrict__ cur, const double* __restrict__ pivots,
-                                   const SplineTap* __restrict__ taps, T* __restrict__ out, long long lines,
-                                   long long nodes, long long length) {
-  extern __shared__ double m[];
-  for (long long line = blockIdx.x; line < lines; line += gridDim.x) {
-    const double* y = cur + line * nodes;
-    if (threadIdx.x == 0) {
-      for (long long i = 0; i < nodes; ++i) m[i] = 0.0;
-      if (nodes >= 3) {
-        for (long long i = 1; i + 1 < nodes; ++i) {
-          const double rhs = __dmul_rn(6.0, __dadd_rn(__dsub_rn(y[i - 1], __dmul_rn(2.0, y[i])), y[i + 1]));
-          m[i] = __dmul_rn(__dsub_rn(rhs, m[i - 1]), pivots[i]);
-        }
-        for (long long i = nodes - 3; i >= 1; --i) m[i] = __dsub_rn(m[i], __dmul_rn(pivots[i], m[i + 1]));
-      }
-    }
+__global__ void __launch_bounds__(256)
+    spline_last_kernel(const double* __restrict__ cur, const double* __restrict__ second,
+                       const SplineTap* __restrict__ taps, const FloatTap* __restrict__ float_taps,
+                       const float4* __restrict__ float_nodes, T* __restrict__ out, long long lines, long long nodes,
+                       long long length, long long column_blocks, int per) {
+  extern __shared__ float4 node[];
+  const bool staged = float_nodes != nullptr;
+  const long long first = blockIdx.x / column_blocks * per;
+  const long long p = blockIdx.x % column_blocks * blockDim.x + threadIdx.x;
+  const int count = (int)min((long long)per, lines - first);
+  if (sizeof(T) == 4 && staged) {
+    for (long long i = threadIdx.x; i < count * nodes; i += blockDim.x) node[i] = float_nodes[first * nodes + i];
     __syncthreads();
-    for (long long p = threadIdx.x; p < length; p += blockDim.x) {
-      const double v = nodes < 2 ? y[0] : tap_eval(taps[p], y, m, 1);
-      if constexpr (sizeof(T) == 4)
-        out[line * length + p] = __double2float_rn(v);
-      else
-        out[line * length + p] = v;
+  }
+  if (p >= length) return;
+  const long long seg = taps[p].seg;
+  T* dst = out + first * length + p;
+  const double* y = cur + first * nodes;
+  const double* m = second + first * nodes;
+  if (sizeof(T) == 4 && staged) {
+    const FloatTap w = float_taps[p];
+    const float2 a = make_float2(w.ab.x, w.ab.y), b = make_float2(w.ab.z, w.ab.w);
+    const float2 c = make_float2(w.cd.x, w.cd.y), d = make_float2(w.cd.z, w.cd.w);
+    for (int line = 0; line < count; ++line) {
+      const float4 u = node[line * nodes + seg], v = node[line * nodes + seg + 1];
+      float e = 0.0f;
+      const float t0 = product(a, make_float2(u.x, u.y), e), t1 = product(b, make_float2(v.x, v.y), e);
+      const float t2 = product(c, make_float2(u.z, u.w), e), t3 = product(d, make_float2(v.z, v.w), e);
+      const float size = (fabsf(t0) + fabsf(t1)) + (fabsf(t2) + fabsf(t3));
+      const float s = sum_of(sum_of(sum_of(t0, t1, e), t2, e), t3, e);
+      const float h = __fadd_rn(s, e), l = __fadd_rn(__fsub_rn(s, h), e);
+      const float off = size * 9.094947e-13f;
+      float value = __fadd_rn(h, __fadd_rn(l, off));
+      if (!(value == __fadd_rn(h, __fsub_rn(l, off)) && size >= 1e-25f && size <= 1e37f))
+        value = __double2float_rn(tap_eval(taps[p], y + line * nodes, m + line * nodes, 1));
+      dst[line * length] = value;
     }
-    __syncthreads();
+  } else {
+    for (int line = 0; line < count; ++line) {
+      const double v = tap_eval(taps[p], y + line * nodes, m + line * nodes, 1);
+      dst[line * length] = sizeof(T) == 4 ? (T)__double2float_rn(v) : (T)v;
+    }
+  }
+}
+
+// A single node: its value along the whole line.
+template <typename T>
+__global__ void spline_flat_kernel(const double* __restrict__ cur, T* __restrict__ out, long long lines,
+                                   long long length) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < lines * length;
+       i += (long long)gridDim.x * blockDim.x) {
+    const double v = cur[i / length];
+    out[i] = sizeof(T) == 4 ? (T)__double2float_rn(v) : (T)v;
   }
 }
 
@@ -1131,21 +1208,49 @@ int interpolate_spline(const std::vector<double>& mesh, const Rules& r, T* d_out
     if (e == cudaSuccess && !pivots.empty())
       e = cudaMemcpyAsync(d_pivots, pivots.data(), pivots.size() * sizeof(double), cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return cuda_fail(e, "mesh spline tables");
+    double* second = nullptr;
+    double* next = nullptr;
+    e = buf.alloc(&second, (size_t)(outer * nodes * inner) * sizeof(double));
     if (axis + 1 == ndim) {
-      const long long blocks = std::min(outer, (long long)std::max(1, sm_count) * 16);
-      const size_t smem = (size_t)std::max(nodes, 1ll) * sizeof(double);
-      auto k = spline_last_kernel<T>;
-      if ((e = allow_max_smem((const void*)k)) != cudaSuccess) return cuda_fail(e, "mesh spline");
-      k<<<(unsigned)std::max(blocks, 1ll), 256, smem, s>>>(cur, d_pivots, d_taps, d_out, outer, nodes, length);
+      if (e != cudaSuccess) return cuda_fail(e, "mesh spline buffers");
+      if (nodes < 2) {
+        spline_flat_kernel<T><<<(unsigned)std::max(1, sm_count) * 8, 256, 0, s>>>(cur, d_out, outer, length);
+      } else {
+        spline_second_kernel<<<(unsigned)((outer + 63) / 64), 64, 0, s>>>(cur, d_pivots, second, outer, nodes, 1);
+        const size_t line_bytes = (size_t)nodes * sizeof(float4);
+        const bool staged = sizeof(T) == 4 && line_bytes <= kSplineSmem;
+        const int per = staged ? (int)std::max<size_t>(1, std::min<size_t>(kSplineLines, 48 * 1024 / line_bytes))
+                               : kSplineLines;
+        const long long across = (length + 255) / 256, down = (outer + per - 1) / per;
+        const size_t smem = staged ? per * line_bytes : 0;
+        FloatTap* float_taps = nullptr;
+        float4* float_nodes = nullptr;
+        if (staged) {
+          std::vector<FloatTap> split((size_t)length);
+          for (long long p = 0; p < length; ++p) {
+            const float2 a = two_floats(taps[p].a), b = two_floats(taps[p].b), c = two_floats(taps[p].c),
+                         d = two_floats(taps[p].d);
+            split[p] = {make_float4(a.x, a.y, b.x, b.y), make_float4(c.x, c.y, d.x, d.y)};
+          }
+          e = buf.alloc(&float_taps, split.size() * sizeof(FloatTap));
+          if (e == cudaSuccess) e = buf.alloc(&float_nodes, (size_t)(outer * nodes) * sizeof(float4));
+          if (e == cudaSuccess)
+            e = cudaMemcpyAsync(float_taps, split.data(), split.size() * sizeof(FloatTap), cudaMemcpyHostToDevice, s);
+          if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // `split` goes out of scope
+          if (e != cudaSuccess) return cuda_fail(e, "mesh spline tables");
+          spline_nodes_kernel<<<(unsigned)std::max(1, sm_count) * 4, 256, 0, s>>>(cur, second, float_nodes, outer * nodes);
+        }
+        auto k = spline_last_kernel<T>;
+        if ((e = allow_max_smem((const void*)k)) != cudaSuccess) return cuda_fail(e, "mesh spline");
+        k<<<(unsigned)(across * down), 256, smem, s>>>(cur, second, d_taps, float_taps, float_nodes, d_out, outer,
+                                                nodes, length, across, per);
+      }
       e = cudaGetLastError();
       if (e != cudaSuccess) return cuda_fail(e, "mesh spline");
       // The temporaries are freed at scope exit: wait for the kernels first.
       e = cudaStreamSynchronize(s);
       return e == cudaSuccess ? NDF_OK : cuda_fail(e, "mesh spline");
     }
-    double* second = nullptr;
-    double* next = nullptr;
-    e = buf.alloc(&second, (size_t)(outer * nodes * inner) * sizeof(double));
     if (e == cudaSuccess) e = buf.alloc(&next, (size_t)(outer * length * inner) * sizeof(double));
     if (e != cudaSuccess) return cuda_fail(e, "mesh spline buffers");
     const long long cols = outer * inner;

@@ -43,3 +43,16 @@ def test_float32_meshes(gpu, oracle, style) -> None:
             actual = gpu.mesh_background(data, box, mask=mask, **options)
             expected = oracle.mesh_background(data, box, filter_size, mask=mask, **oracle_options)
             _compare(actual, expected, (shape, box, options))
+
+
+@pytest.mark.parametrize("shape,box", [((40, 700), (8, 5)), ((3, 5000), (3, 1)), ((19, 15000), (19, 1)), ((33, 64), (33, 64)),
+                                       ((20, 257), (4, 300)), ((15, 14, 300), (5, 7, 16))])
+def test_float32_maps(gpu, oracle, shape, box) -> None:
+    """The spline's last axis: few and many nodes (staged or not), one node, remainders of its blocks,
+    values large and small enough for float64."""
+    rng = np.random.default_rng(len(shape))
+    for scale in (1.0, 1e-30, 1e36):
+        data = ((500 + 22 * rng.normal(size=shape)) * scale).astype(np.float32)
+        actual = gpu.mesh_background(data, box, min_valid_fraction=0.0)
+        expected = oracle.mesh_background(data, box, 3, min_valid_fraction=0.0, pearson=2.5)
+        _compare(actual, expected, (shape, box, scale))
