@@ -71,41 +71,101 @@ struct Wide {
   unsigned long long w[W];
 };
 
+// Additions with the carry flag: two instructions a word, where comparing for
+// the carry took about ten.
 template <int W>
 __device__ __forceinline__ void wide_add(Wide<W>& a, const Wide<W>& b) {
-  unsigned long long carry = 0;
-#pragma unroll
-  for (int i = 0; i < W; ++i) {
-    const unsigned long long s = a.w[i] + b.w[i];
-    const unsigned long long t = s + carry;
-    carry = (s < a.w[i]) | (t < s);
-    a.w[i] = t;
+  static_assert(W <= 3 || W == 5 || W == 6, "words of the kernels' sums");
+  if constexpr (W == 1) {
+    a.w[0] += b.w[0];
+  } else if constexpr (W == 2) {
+    asm("add.cc.u64 %0, %0, %2;\n\taddc.u64 %1, %1, %3;" : "+l"(a.w[0]), "+l"(a.w[1]) : "l"(b.w[0]), "l"(b.w[1]));
+  } else if constexpr (W == 3) {
+    asm("add.cc.u64 %0, %0, %3;\n\taddc.cc.u64 %1, %1, %4;\n\taddc.u64 %2, %2, %5;"
+        : "+l"(a.w[0]), "+l"(a.w[1]), "+l"(a.w[2])
+        : "l"(b.w[0]), "l"(b.w[1]), "l"(b.w[2]));
+  } else if constexpr (W == 5) {
+    asm("add.cc.u64 %0, %0, %5;\n\taddc.cc.u64 %1, %1, %6;\n\taddc.cc.u64 %2, %2, %7;\n\t"
+        "addc.cc.u64 %3, %3, %8;\n\taddc.u64 %4, %4, %9;"
+        : "+l"(a.w[0]), "+l"(a.w[1]), "+l"(a.w[2]), "+l"(a.w[3]), "+l"(a.w[4])
+        : "l"(b.w[0]), "l"(b.w[1]), "l"(b.w[2]), "l"(b.w[3]), "l"(b.w[4]));
+  } else {
+    asm("add.cc.u64 %0, %0, %6;\n\taddc.cc.u64 %1, %1, %7;\n\taddc.cc.u64 %2, %2, %8;\n\t"
+        "addc.cc.u64 %3, %3, %9;\n\taddc.cc.u64 %4, %4, %10;\n\taddc.u64 %5, %5, %11;"
+        : "+l"(a.w[0]), "+l"(a.w[1]), "+l"(a.w[2]), "+l"(a.w[3]), "+l"(a.w[4]), "+l"(a.w[5])
+        : "l"(b.w[0]), "l"(b.w[1]), "l"(b.w[2]), "l"(b.w[3]), "l"(b.w[4]), "l"(b.w[5]));
   }
 }
 
 template <int W>
 __device__ __forceinline__ void wide_sub(Wide<W>& a, const Wide<W>& b) {
-  unsigned long long borrow = 0;
-#pragma unroll
-  for (int i = 0; i < W; ++i) {
-    const unsigned long long d = a.w[i] - b.w[i];
-    const unsigned long long t = d - borrow;
-    borrow = (a.w[i] < b.w[i]) | (d < borrow);
-    a.w[i] = t;
+  static_assert(W <= 3 || W == 5 || W == 6, "words of the kernels' sums");
+  if constexpr (W == 1) {
+    a.w[0] -= b.w[0];
+  } else if constexpr (W == 2) {
+    asm("sub.cc.u64 %0, %0, %2;\n\tsubc.u64 %1, %1, %3;" : "+l"(a.w[0]), "+l"(a.w[1]) : "l"(b.w[0]), "l"(b.w[1]));
+  } else if constexpr (W == 3) {
+    asm("sub.cc.u64 %0, %0, %3;\n\tsubc.cc.u64 %1, %1, %4;\n\tsubc.u64 %2, %2, %5;"
+        : "+l"(a.w[0]), "+l"(a.w[1]), "+l"(a.w[2])
+        : "l"(b.w[0]), "l"(b.w[1]), "l"(b.w[2]));
+  } else if constexpr (W == 5) {
+    asm("sub.cc.u64 %0, %0, %5;\n\tsubc.cc.u64 %1, %1, %6;\n\tsubc.cc.u64 %2, %2, %7;\n\t"
+        "subc.cc.u64 %3, %3, %8;\n\tsubc.u64 %4, %4, %9;"
+        : "+l"(a.w[0]), "+l"(a.w[1]), "+l"(a.w[2]), "+l"(a.w[3]), "+l"(a.w[4])
+        : "l"(b.w[0]), "l"(b.w[1]), "l"(b.w[2]), "l"(b.w[3]), "l"(b.w[4]));
+  } else {
+    asm("sub.cc.u64 %0, %0, %6;\n\tsubc.cc.u64 %1, %1, %7;\n\tsubc.cc.u64 %2, %2, %8;\n\t"
+        "subc.cc.u64 %3, %3, %9;\n\tsubc.cc.u64 %4, %4, %10;\n\tsubc.u64 %5, %5, %11;"
+        : "+l"(a.w[0]), "+l"(a.w[1]), "+l"(a.w[2]), "+l"(a.w[3]), "+l"(a.w[4]), "+l"(a.w[5])
+        : "l"(b.w[0]), "l"(b.w[1]), "l"(b.w[2]), "l"(b.w[3]), "l"(b.w[4]), "l"(b.w[5]));
   }
 }
 
+// high / n and high % n for n below 2^16 and high below 2^80 (2^64 for WIDE
+// false): digits of 16 bits from the top, each quotient digit the upper half of
+// the product with a reciprocal from below, at most two short, and corrected. (The
+// compiler's 128-bit division took most of the time of a float64 mean.)
+template <bool WIDE>
+__device__ __forceinline__ void divide_count(unsigned __int128 high, unsigned int n, unsigned __int128& q,
+                                             unsigned int& r) {
+  // 2^32 / n less at most 2^-21 of it: the constant lies 4 units in the last
+  // place below 2^32 and the reciprocal is rounded down.
+  const unsigned int inverse = (unsigned int)(4294966272.0f * __frcp_rz((float)n));
+  unsigned long long quotient = 0;
+  unsigned int top = 0;
+  r = 0;
+#pragma unroll
+  for (int i = WIDE ? 4 : 3; i >= 0; --i) {
+    const unsigned int x = (r << 16) | (unsigned int)((high >> (16 * i)) & 0xFFFFu);
+    unsigned int d = __umulhi(x, inverse);
+    r = x - d * n;
+    if (r >= n) {
+      r -= n;
+      ++d;
+    }
+    if (r >= n) {
+      r -= n;
+      ++d;
+    }
+    if (WIDE && i == 4)
+      top = d;
+    else
+      quotient |= (unsigned long long)d << (16 * i);
+  }
+  q = WIDE ? ((unsigned __int128)top << 64) | quotient : (unsigned __int128)quotient;
+}
+
 // The sample as a W-word two's-complement integer in units of
-// 2^(E0 + 64 * low_word); zero for zero and non-finite samples. The tile's
-// span guarantees pos >= 64 * low_word and that the value fits.
+// 2^(E0 + low); zero for zero and non-finite samples. The tile's span
+// guarantees pos >= low and that the value fits.
 template <typename T, int W>
-__device__ __forceinline__ Wide<W> encode(T v, int low_word) {
+__device__ __forceinline__ Wide<W> encode(T v, int low) {
   Wide<W> r;
   unsigned long long m;
   int pos;
   bool neg;
   const bool finite = decompose(v, m, pos, neg);
-  const int local = finite ? pos - 64 * low_word : 0;
+  const int local = finite ? pos - low : 0;
   const int wi = local >> 6, off = local & 63;
   const unsigned long long lo = finite ? m << off : 0ull;
   const unsigned long long hi = (finite && off) ? m >> (64 - off) : 0ull;
@@ -125,13 +185,13 @@ __device__ __forceinline__ Wide<W> encode(T v, int low_word) {
 __device__ __forceinline__ int bitlen64(unsigned long long x) { return x ? 64 - __clzll((long long)x) : 0; }
 
 // RN_T(S / n) for the NW-word two's-complement sum S in units of
-// 2^(E0 + 64 * low_word) and a count n >= 1, rounded once: with B the bit
+// 2^(E0 + low) and a count n >= 1, rounded once: with B the bit
 // length of |S| and t that of n, q = floor(|S| / (n 2^s)) for
 // s = max(B - t - p - 1, 0) has p + 1 or p + 2 bits (p, the precision), so
 // its low bits and the remainder decide the rounding exactly; s = 0 is the
 // subnormal grid, where no sample has bits below.
 template <typename T, int NW>
-__device__ __forceinline__ T exact_mean(const unsigned long long (&sum)[NW], int low_word, unsigned int n) {
+__device__ __forceinline__ T exact_mean(const unsigned long long (&sum)[NW], int low, unsigned int n) {
   using B = Bits<T>;
   constexpr int p = B::kP;
   const bool negative = (sum[NW - 1] >> 63) != 0;
@@ -148,10 +208,10 @@ __device__ __forceinline__ T exact_mean(const unsigned long long (&sum)[NW], int
     if (m[i]) blocal = 64 * i + bitlen64(m[i]);
   const typename B::U sign = negative ? (typename B::U)1 << (sizeof(T) * 8 - 1) : 0;
   if (blocal == 0) return from_bits<T>(0);  // exact cancellation gives +0
-  const int bits = blocal + 64 * low_word;
+  const int bits = blocal + low;
   const int t = 32 - __clz((int)n);
   const int s = max(bits - t - p - 1, 0);
-  const int sl = s - 64 * low_word;  // shift of the local words
+  const int sl = s - low;  // shift of the local words
   unsigned __int128 high = 0;
   bool sticky = false;
 #pragma unroll
@@ -168,8 +228,13 @@ __device__ __forceinline__ T exact_mean(const unsigned long long (&sum)[NW], int
       sticky = sticky || (m[i] & ((1ull << (-sh)) - 1)) != 0;
     }
   }
+  // At most t + p + 1 bits: 71 (float64) or 42 (float32) for counts below 2^16.
   unsigned __int128 q, r;
-  if constexpr (sizeof(T) == 4) {
+  if (n < 65536u) {
+    unsigned int rest;
+    divide_count<sizeof(T) == 8>(high, n, q, rest);
+    r = rest;
+  } else if constexpr (sizeof(T) == 4) {
     const unsigned long long h = (unsigned long long)high;  // at most 58 bits
     q = h / n;
     r = h % n;
