@@ -9,7 +9,8 @@
 // that arithmetic reaches the result:
 //  * the MAD is |2 v - (a + b)| / 2 for one sample v (two for even counts):
 //    which sample follows from float32 differences, because rounding is
-//    monotone, with the few rounding ties settled by exact differences;
+//    monotone; where the differences are exact they are the answer, else the
+//    few rounding ties are settled by exact differences;
 //  * a clipping pass only decides which sorted samples stay. The spread is
 //    evaluated in float32 with a bound on its error; a sample so close to the
 //    limit that the bound does not decide it sends the pass to float64 with a
@@ -33,8 +34,9 @@
 //
 // Bound now by the min / max pipe of the sort and by the shared-memory loads
 // of the passes over the column. Measured with the filling-in pass (frames of
-// noise with outliers, NaN and infinities): MAD 5 x 5 on 4096^2 7.63 -> 0.91 ms,
-// clipped mode 7 x 7 on 2048^2 30.7 -> 0.88 ms.
+// noise with outliers, NaN and infinities): MAD 5 x 5 on 4096^2 7.63 -> 0.74 ms
+// (0.91 with a few float64 operations per output, which cost a third of a 3 x 3
+// MAD), clipped mode 7 x 7 on 2048^2 30.7 -> 0.80 ms.
 #pragma once
 
 #include "network.cuh"
@@ -121,23 +123,63 @@ __device__ __forceinline__ int deviation_at(const Column& s, int n, int rank, fl
   return at;
 }
 
-// The MAD of the n sorted samples times `scale`; false when not decided.
-__device__ __forceinline__ bool mad_value(const Column& s, int n, double scale, double* out) {
+// The MAD of the n sorted samples times `scale`, rounded to float32; kUndecided
+// when not decided. (Samples of any set bits; out of line, as mad_value takes
+// nearly every window.)
+static __device__ __noinline__ float mad_general(const float* c, int n, double scale) {
+  const Column s{c};
+  const float undecided = __uint_as_float(kUndecided);
   const float a = s[(n - 1) / 2], b = s[n / 2];
-  if (!sum_exact(a, b)) return false;
+  if (!sum_exact(a, b)) return undecided;
   float value;
   const int at = deviation_at(s, n, n / 2, a, b, &value);
-  if (at < 0) return false;
+  if (at < 0) return undecided;
   const double center = __dadd_rn(widen(a), widen(b));
   Scaled d{abs64(__dsub_rn(twice(widen(s[at])), center)), -1};
   if ((n & 1) == 0) {
     const int before = deviation_at(s, n, n / 2 - 1, a, b, &value);
-    if (before < 0) return false;
+    if (before < 0) return undecided;
     // scaled_midpoint of two deviations of exponent -1: their float64 sum.
     d = {__dadd_rn(abs64(__dsub_rn(twice(widen(s[before])), center)), d.value), -2};
   }
-  *out = multiply_scaled(d, scale);
-  return true;
+  const double product = multiply_scaled(d, scale);
+  return nan64(product) ? nan_of(0.0f) : __double2float_rn(product);
+}
+
+// The same for samples that are multiples of 2^low. Differences below 2^24 of
+// those units are exact in float32, so the least maxima are the deviations
+// themselves and ties are equal deviations; their product with the scale (a pair
+// of floats, to 2^-49) is the float32 rounding of the float64 one when it rounds
+// the same 2^-40 above and below.
+__device__ __forceinline__ float mad_value(const Column& s, int n, int low, float2 scale, double scale64) {
+  const int h = n / 2;
+  const bool even = (n & 1) == 0;
+  const float a = s[(n - 1) / 2], b = s[h];
+  float mid = __int_as_float(0x7f800000), before = mid, r0 = __fsub_rn(s[max(h - 1, 0)], b);
+#pragma unroll 4
+  for (int i = 0; i < n - h; ++i) {
+    const float l = __fsub_rn(a, s[i]), r = __fsub_rn(s[i + h], b);
+    mid = fminf(mid, fmaxf(l, r));
+    before = fminf(before, fmaxf(l, r0));
+    r0 = r;
+  }
+  float d = mid;
+  if (even) {
+    before = fminf(before, fmaxf(__fsub_rn(a, s[h]), r0));
+    // Both deviations lack half the gap b - a; their mean is half of all three.
+    d = __fadd_rn(__fadd_rn(mid, before), __fsub_rn(b, a));
+  }
+  // 2^(low + 23) as a float; nothing is below it when that is out of range.
+  const float limit = low >= -140 && low <= 100 ? __uint_as_float((unsigned int)(low + 150) << 23) : 0.0f;
+  if (d < limit) {
+    if (even) d = __fmul_rn(d, 0.5f);
+    const float p = __fmul_rn(d, scale.x);
+    const float e = __fmaf_rn(d, scale.y, __fmaf_rn(d, scale.x, -p)), off = p * 9.094947e-13f;
+    const float value = __fadd_rn(p, __fadd_rn(e, off));
+    if (d == 0.0f) return 0.0f;
+    if (value == __fadd_rn(p, __fsub_rn(e, off)) && p >= 1e-25f && p <= 1e37f) return value;
+  }
+  return mad_general(s.c, n, scale64);
 }
 
 __device__ __forceinline__ float difference(float x, float y, float) { return __fsub_rn(x, y); }
@@ -203,7 +245,7 @@ __device__ __forceinline__ F mad_spread(const Column& s, int lo, int hi, float a
 // sample lies too close to its limit to be decided in F.
 template <typename F>
 __device__ __forceinline__ int clip_pass(const Column& s, int lo, int hi, const RobustArgs& ra, int* new_lo,
-                                         int* new_hi) {
+                                         int* new_hi, float* std) {
   const int n = hi - lo;
   const float a = s[lo + (n - 1) / 2], b = s[lo + n / 2];
   F center = (F)0.5 * difference(b, a, F()), spread = 0;  // center minus a
@@ -213,6 +255,7 @@ __device__ __forceinline__ int clip_pass(const Column& s, int lo, int hi, const 
   if (ra.spread == 0 || ra.center == 0) {
     const Moments<F> m = moments_of<F>(s, lo, hi, a);
     spread = m.std;
+    *std = (float)m.std;
     if (ra.center == 0) {
       center = m.mean;
       slack += (F)(4 * n) * unit_roundoff(F()) * m.std;
@@ -256,8 +299,8 @@ __device__ __forceinline__ int clip_pass(const Column& s, int lo, int hi, const 
 
 // Rare: kept out of line.
 static __device__ __noinline__ int clip_pass_f64(const float* c, int lo, int hi, const RobustArgs& ra, int* new_lo,
-                                          int* new_hi) {
-  return clip_pass<double>(Column{c}, lo, hi, ra, new_lo, new_hi);
+                                                 int* new_hi, float* std) {
+  return clip_pass<double>(Column{c}, lo, hi, ra, new_lo, new_hi, std);
 }
 
 // Whether the differences of the finite run s[lo, hi) stay clear of float32
@@ -305,23 +348,24 @@ __device__ __forceinline__ bool exact_mean_of(const Column& s, int lo, int hi, i
   return true;
 }
 
-// |difference| / std >= 0.3 for the standard deviation of s[lo, hi): 1 or 0,
+// |difference| / std >= 0.3 for the standard deviation of n samples: 1 or 0,
 // -1 when F does not decide.
 template <typename F>
-__device__ __forceinline__ int far_from_mean(const Column& s, int lo, int hi, double difference) {
-  const Moments<F> m = moments_of<F>(s, lo, hi, s[lo + (hi - lo - 1) / 2]);
-  const F d = (F)abs64(difference), limit = (F)0.3 * m.std, e = limit_error(hi - lo, F());
+__device__ __forceinline__ int far_from_mean(int n, F std, double difference) {
+  const F d = (F)abs64(difference), limit = (F)0.3 * std, e = limit_error(n, F());
   if (d >= limit * ((F)1 + e)) return 1;
   if (d <= limit * ((F)1 - e)) return 0;
   return -1;
 }
 
 static __device__ __noinline__ int far_from_mean_f64(const float* c, int lo, int hi, double difference) {
-  return far_from_mean<double>(Column{c}, lo, hi, difference);
+  const Column s{c};
+  return far_from_mean<double>(hi - lo, moments_of<double>(s, lo, hi, s[lo + (hi - lo - 1) / 2]).std, difference);
 }
 
-// mode_estimate (src/location.rs:36-54) of the sorted run.
-__device__ __forceinline__ bool mode_value(const Column& s, int lo, int hi, int low, const RobustArgs& ra,
+// mode_estimate (src/location.rs:36-54) of the sorted run; `std` is its standard
+// deviation in float32 where the last clipping pass has it already, else negative.
+__device__ __forceinline__ bool mode_value(const Column& s, int lo, int hi, int low, const RobustArgs& ra, float std,
                                            double* out) {
   const int n = hi - lo;
   double mean;
@@ -340,7 +384,8 @@ __device__ __forceinline__ bool mode_value(const Column& s, int lo, int hi, int 
   }
   if (!in_range(s, lo, hi)) return false;
   const double off = __dsub_rn(median, mean);
-  int far = far_from_mean<float>(s, lo, hi, off);
+  if (std < 0.0f) std = moments_of<float>(s, lo, hi, a).std;
+  int far = far_from_mean<float>(n, std, off);
   if (far < 0) far = far_from_mean_f64(s.c, lo, hi, off);
   if (far < 0) return false;
   *out = far ? median : __dadd_rn(median, __dmul_rn(__dsub_rn(ra.pearson, 1.0), off));
@@ -351,22 +396,24 @@ __device__ __forceinline__ bool mode_value(const Column& s, int lo, int hi, int 
 __device__ __forceinline__ bool clipped_value(const Column& s, int n, int low, const RobustArgs& ra, double* out) {
   int lo = 0, hi = n;
   long long iteration = 0;
+  float std = -1.0f;
   while (hi - lo >= ra.clip_min_count && (ra.maxiters < 0 || iteration < ra.maxiters)) {
     if (s[lo] == s[hi - 1]) break;  // no spread: every sample equals the center
     if (!in_range(s, lo, hi)) return false;
     int x, y;
-    if (!clip_pass<float>(s, lo, hi, ra, &x, &y) && !clip_pass_f64(s.c, lo, hi, ra, &x, &y)) return false;
+    if (!clip_pass<float>(s, lo, hi, ra, &x, &y, &std) && !clip_pass_f64(s.c, lo, hi, ra, &x, &y, &std)) return false;
     ++iteration;
     if (x == lo && y == hi) break;
     lo = x;
     hi = y;
+    std = -1.0f;
   }
   if (hi - lo < ra.clip_min_count) {
     *out = nan_of(0.0);
     return true;
   }
   if (ra.kind == kRobustSigmaMean) return exact_mean_of(s, lo, hi, low, out);
-  if (ra.kind == kRobustSigmaMode) return mode_value(s, lo, hi, low, ra, out);
+  if (ra.kind == kRobustSigmaMode) return mode_value(s, lo, hi, low, ra, std, out);
   const float a = s[lo + (hi - lo - 1) / 2], b = s[lo + (hi - lo) / 2];
   if (!sum_exact(a, b)) return false;
   *out = __float_as_uint(a) == __float_as_uint(b) ? widen(a) : __dmul_rn(__dadd_rn(widen(a), widen(b)), 0.5);
@@ -376,7 +423,7 @@ __device__ __forceinline__ bool clipped_value(const Column& s, int n, int low, c
 // Blocks per SM the registers must allow: the network's wires and a few more.
 template <int N>
 constexpr int min_blocks() {
-  return N <= 16 ? 12 : N <= 32 ? 8 : N <= 49 ? 6 : N <= 64 ? 5 : N <= 81 ? 4 : 2;
+  return N <= 32 ? 8 : N <= 49 ? 6 : N <= 64 ? 5 : N <= 81 ? 4 : 2;
 }
 
 // MAD: the MAD kind; otherwise sigma clipping and the mode kind.
@@ -384,7 +431,7 @@ template <int N, bool MAD>
 __global__ void __launch_bounds__(kT, min_blocks<N>())
     robust_tile_kernel(const float* __restrict__ in, float* __restrict__ out, const __grid_constant__ TileArgs a,
                        const __grid_constant__ net::TapTable<N> taps, const __grid_constant__ CUtensorMap tmap,
-                       const __grid_constant__ RobustArgs ra, int column_offset) {
+                       const __grid_constant__ RobustArgs ra, float2 scale, int column_offset) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int lowest;
   const Geom3& g = a.g;
@@ -403,7 +450,7 @@ __global__ void __launch_bounds__(kT, min_blocks<N>())
     return;
   __syncthreads();
   int low = 0;
-  if (!MAD && ra.kind != kRobustSigmaMedian) {
+  if (MAD || ra.kind != kRobustSigmaMedian) {
     const int staged = g.kd * t.SH * t.SW;
     int mine = INT_MAX;
     for (int i = threadIdx.x; i < staged; i += kT) mine = min(mine, lowest_bit(keys[i]));
@@ -429,24 +476,15 @@ __global__ void __launch_bounds__(kT, min_blocks<N>())
 #pragma unroll
     for (int i = 0; i < N; ++i) column[i * kT] = KeyOf<float>::value(k[i]);
     const Column s{column};
-    double value = 0.0;
-    bool ok;
     const bool none = clip ? n < ra.clip_min_count : (n == 0 || (a.r.omit ? n < a.r.min_count : n != V));
-    if (none) {
-      value = nan_of(0.0);
-      ok = true;
-    } else if constexpr (MAD) {
-      ok = mad_value(s, n, ra.parameter, &value);
-    } else if (clip) {
-      ok = clipped_value(s, n, low, ra, &value);
-    } else if (isinf(s[0]) || isinf(s[n - 1])) {
-      value = nan_of(0.0);
-      ok = true;
-    } else {
-      ok = mode_value(s, 0, n, low, ra, &value);
+    float result = nan_of(0.0f);
+    if constexpr (MAD) {
+      if (!none) result = mad_value(s, n, low, scale, ra.parameter);
+    } else if (!none && (clip || !(isinf(s[0]) || isinf(s[n - 1])))) {
+      double value = 0.0;
+      const bool ok = clip ? clipped_value(s, n, low, ra, &value) : mode_value(s, 0, n, low, ra, -1.0f, &value);
+      result = !ok ? __uint_as_float(kUndecided) : nan64(value) ? nan_of(0.0f) : __double2float_rn(value);
     }
-    float result = nan64(value) ? nan_of(0.0f) : __double2float_rn(value);
-    if (!ok) result = __uint_as_float(kUndecided);
     out[(z * g.H + y) * g.W + x] = result;
   }
 }
@@ -472,7 +510,9 @@ cudaError_t launch_width(const Plan& p, const float* in, float* out, cudaStream_
     smem = p.smem_bytes;
   }
   const size_t columns = (smem + 15) & ~(size_t)15;
-  kernel<<<(unsigned)args.t.tiles, kT, columns + kColumns, s>>>(in, out, args, taps, map, p.robust, (int)columns);
+  const float scale = (float)p.robust.parameter;
+  kernel<<<(unsigned)args.t.tiles, kT, columns + kColumns, s>>>(
+      in, out, args, taps, map, p.robust, make_float2(scale, (float)(p.robust.parameter - (double)scale)), (int)columns);
   return cudaGetLastError();
 }
 
