@@ -137,6 +137,15 @@ __device__ __forceinline__ void top48(unsigned long long w2, unsigned long long 
   e = len == 0 ? 0 : shift;
 }
 
+// top48 of one word.
+__device__ __forceinline__ void top48_word(unsigned long long d, float& hi, float& lo, int& e) {
+  const int c = d ? __clzll((long long)d) : 0;
+  const unsigned long long t = d << c;
+  hi = (float)(unsigned int)(t >> 40) * 16777216.0f;
+  lo = (float)((unsigned int)(t >> 16) & 0xFFFFFFu);
+  e = d ? 16 - c : 0;
+}
+
 // (hi + lo) / (dh + dl) as float-float (qh + ql).
 __device__ __forceinline__ void ff_div(float hi, float lo, float dh, float dl, float& qh, float& ql) {
   const float q1 = __fdiv_rn(hi, dh);
@@ -146,6 +155,35 @@ __device__ __forceinline__ void ff_div(float hi, float lo, float dh, float dl, f
   const float q2 = __fdiv_rn(r, dh);
   qh = __fadd_rn(q1, q2);  // renormalize (|q2| is far below |q1|)
   ql = __fsub_rn(q2, __fsub_rn(qh, q1));
+}
+
+// scalbnf(x, k): one multiplication where 2^k and the result are normal.
+__device__ __forceinline__ float scale_f32(float x, int k) {
+  const unsigned int b = __float_as_uint(x) & 0x7fffffffu;
+  if ((unsigned int)(k + 60) <= 120u && b - 0x20000000u < 0x40000000u)  // 2^-63 <= |x| < 2^65
+    return __fmul_rn(x, __uint_as_float((unsigned int)(k + 127) << 23));
+  return scalbnf(x, k);
+}
+
+// The variance (hi + lo) 2^e / (dh + dl), in units of 2^(2 quantum), or its root.
+template <int KIND>
+__device__ __forceinline__ float root_f32(float hi, float lo, int e, float dh, float dl, int quantum) {
+  float qh, ql;
+  ff_div(hi, lo, dh, dl, qh, ql);
+  if (KIND == kVar) return scale_f32(__fadd_rn(qh, ql), e + 2 * quantum);
+  // sqrt((qh + ql) 2^e) 2^quantum with an even power of two under the root.
+  if (e & 1) {
+    qh = __fmul_rn(qh, 2.0f);
+    ql = __fmul_rn(ql, 2.0f);
+    e -= 1;
+  }
+  const float r0 = __fsqrt_rn(qh);
+  float root = r0;
+  if (r0 > 0.0f) {
+    const float resid = __fadd_rn(fmaf(-r0, r0, qh), ql);
+    root = __fadd_rn(r0, __fdiv_rn(resid, __fmul_rn(2.0f, r0)));
+  }
+  return scale_f32(root, e / 2 + quantum);
 }
 
 // Variance / standard deviation of float32 output from the exact numerator
@@ -159,22 +197,20 @@ __device__ __forceinline__ float spread_f32(unsigned long long d2, unsigned long
   const unsigned long long den = (unsigned long long)finite * (unsigned long long)(finite - ddof);
   const float dh = (float)den;
   const float dl = (float)((long long)den - (long long)dh);
-  float qh, ql;
-  ff_div(hi, lo, dh, dl, qh, ql);
-  if (KIND == kVar) return scalbnf(__fadd_rn(qh, ql), e + 2 * quantum);
-  // sqrt((qh + ql) 2^e) 2^quantum with an even power of two under the root.
-  if (e & 1) {
-    qh = __fmul_rn(qh, 2.0f);
-    ql = __fmul_rn(ql, 2.0f);
-    e -= 1;
-  }
-  const float r0 = __fsqrt_rn(qh);
-  float root = r0;
-  if (r0 > 0.0f) {
-    const float resid = __fadd_rn(fmaf(-r0, r0, qh), ql);
-    root = __fadd_rn(r0, __fdiv_rn(resid, __fmul_rn(2.0f, r0)));
-  }
-  return scalbnf(root, e / 2 + quantum);
+  return root_f32<KIND>(hi, lo, e, dh, dl, quantum);
+}
+
+// The numerator in one word, and 0 <= ddof < finite < 2^16.
+template <int KIND>
+__device__ __forceinline__ float spread_word(unsigned long long d, unsigned int finite, unsigned int ddof,
+                                             int quantum) {
+  float hi, lo;
+  int e;
+  top48_word(d, hi, lo, e);
+  const unsigned int den = finite * (finite - ddof);
+  const float dh = (float)den;
+  const float dl = (float)(int)(den - (unsigned int)dh);
+  return root_f32<KIND>(hi, lo, e, dh, dl, quantum);
 }
 
 template <int KIND>
@@ -255,33 +291,45 @@ __device__ Span<T> tile_span(const T* s, int support) {
   Span<T> sp;
   sp.pivot = pivot_s;
   int lo = INT_MAX, top = -1, dev = -1075, nonfinite = 0;
-  {
-    unsigned long long m;
-    int pos;
-    bool neg;
-    if (threadIdx.x == 0 && decompose(sp.pivot, m, pos, neg)) {
-      lo = pos;
-      top = pos + bitlen64(m) - 1;
+  // The rounded difference's exponent plus one bounds the exact one.
+  if constexpr (sizeof(T) == 4) {
+    // The top bit and the exponent grow with the magnitude's bits, so only the
+    // lowest set bit is found per sample, in 32-bit integers.
+    unsigned int big = 0, far = 0;
+    bool any = false;
+    for (int e = threadIdx.x; e < support; e += blockDim.x) {
+      const float v = s[e];
+      const unsigned int b = __float_as_uint(v) & 0x7fffffffu;
+      if (b < 0x7f800000u) {
+        any = true;
+        big = max(big, b);
+        far = max(far, __float_as_uint(__fsub_rn(v, sp.pivot)) & 0x7fffffffu);
+        // Bit 23 is the hidden bit of a normal sample and above any other's lowest.
+        const int pos = max((int)(b >> 23), 1) - 2 + __ffs((int)(b | 0x800000u));
+        lo = b ? min(lo, pos) : lo;
+      } else {
+        nonfinite |= b > 0x7f800000u ? 1 : (v > 0.0f ? 2 : 4);
+      }
     }
-  }
-  for (int e = threadIdx.x; e < support; e += blockDim.x) {
-    const T v = s[e];
-    unsigned long long m;
-    int pos;
-    bool neg;
-    if (decompose(v, m, pos, neg)) {
-      lo = min(lo, pos);
-      top = max(top, pos + bitlen64(m) - 1);
+    if (any) {
+      top = exponent_of(__uint_as_float(big));
+      top = big ? top + 149 : -1;
+      dev = exponent_of(__uint_as_float(far));
     }
-    if (isfinite(v)) {
-      // The rounded difference's exponent plus one bounds the exact one; the
-      // float32 difference keeps float32 input off the FP64 pipe.
-      if constexpr (sizeof(T) == 4)
-        dev = max(dev, exponent_of(__fsub_rn((float)v, (float)sp.pivot)));
-      else
+  } else {
+    for (int e = threadIdx.x; e < support; e += blockDim.x) {
+      const T v = s[e];
+      unsigned long long m;
+      int pos;
+      bool neg;
+      if (decompose(v, m, pos, neg)) {
+        lo = min(lo, pos);
+        top = max(top, pos + bitlen64(m) - 1);
+      }
+      if (isfinite(v))
         dev = max(dev, exponent_of(__dsub_rn((double)v, (double)sp.pivot)));
-    } else {
-      nonfinite |= isnan(v) ? 1 : (v > (T)0 ? 2 : 4);
+      else
+        nonfinite |= isnan(v) ? 1 : (v > (T)0 ? 2 : 4);
     }
   }
   for (int o = 16; o >= 1; o >>= 1) {
@@ -377,6 +425,25 @@ __device__ __forceinline__ T fixed_combine_narrow(int kind, long long ddof, long
     const double unscaled = __ddiv_rn(num, __dmul_rn(n, (double)((long long)finite - ddof)));
     return kind == kStd ? __dmul_rn(__dsqrt_rn(unscaled), scale) : __dmul_rn(__dmul_rn(unscaled, scale), scale);
   }
+}
+
+// fixed_combine for float32 sums whose terms n S2, S1^2 and n P + S1 are below
+// 2^62 in magnitude, |S1| < 2^32, and ddof >= 0. Results equal fixed_combine's.
+__device__ __forceinline__ float fixed_combine_word(int kind, long long ddof, long long s1, unsigned long long s2,
+                                                    unsigned int finite, long long P, int quantum) {
+  if (kind == kMean) {
+    const long long sum = (long long)finite * P + s1;
+    float hi, lo, qh, ql;
+    int e;
+    top48_word((unsigned long long)(sum < 0 ? -sum : sum), hi, lo, e);
+    ff_div(hi, lo, (float)finite, 0.0f, qh, ql);
+    const float q = scale_f32(__fadd_rn(qh, ql), e + quantum);
+    return sum < 0 ? -q : q;
+  }
+  const unsigned int a = (unsigned int)(s1 < 0 ? -s1 : s1);
+  const unsigned long long d = s2 * finite - (unsigned long long)a * a;  // >= 0 (Cauchy-Schwarz)
+  return kind == kVar ? spread_word<kVar>(d, finite, (unsigned int)ddof, quantum)
+                      : spread_word<kStd>(d, finite, (unsigned int)ddof, quantum);
 }
 
 }  // namespace fixm

@@ -25,6 +25,10 @@
 //    FP32 pipe, float64 outputs convert it to float64 once and run FP64 only
 //    for the division by n (n - ddof), the power-of-two scaling and the
 //    square root;
+//  * float32 tiles run on instructions (66% of the issue slots), so the span and
+//    the deviations of float32 samples are found in 32-bit integers and the combine
+//    of tiles whose terms stay below 2^62 in one 64-bit word: 31 x 31 std of 4096^2
+//    with 1% NaN 0.515 -> 0.429 ms, 65 x 65 0.995 -> 0.763, 3 x 3 0.333 -> 0.288;
 //  * the classification of NaN / infinities / counts is the reference's
 //    (decide_special); tiles whose value range does not fit the integer
 //    widths compute their outputs with the reference's float64 arithmetic.
@@ -105,8 +109,8 @@ __device__ __forceinline__ int skew(int c) { return c + (c >> 3); }
 //      class (Counts::sample) as a third sum.
 template <typename T, int XK, bool NARROW, int CM>
 __device__ __forceinline__ void column_walk(unsigned char* base, const SlideLayout& L, const T* s, const TileArgs& a,
-                                            const SlideArgs& sa, const Span<T>& sp, i128 P, int bits, long long z,
-                                            long long y0, long long x0, T* __restrict__ out) {
+                                            const SlideArgs& sa, const Span<T>& sp, i128 P, int bits, bool word,
+                                            long long z, long long y0, long long x0, T* __restrict__ out) {
   using S1 = typename std::conditional<NARROW, long long, i128>::type;
   using S2 = typename std::conditional<NARROW, unsigned long long, u128>::type;
   using XW = typename std::conditional<XK == 0, int, long long>::type;
@@ -197,6 +201,9 @@ __device__ __forceinline__ void column_walk(unsigned char* base, const SlideLayo
     double result;
     if (mom::decide_special(r, (long long)finite + pos + neg, nanc != 0, pos != 0, neg != 0, &result))
       return canonical(from_f64<T>(result));
+    if constexpr (NARROW && sizeof(T) == 4)
+      if (word)
+        return canonical(fixed_combine_word(r.kind, r.param, a1, a2, finite, (long long)P, quantum));
     if constexpr (NARROW)
       return canonical(fixed_combine_narrow<T>(r.kind, r.param, a1, a2, finite, P, quantum));
     else
@@ -298,6 +305,20 @@ __device__ __forceinline__ void deviations_in_place(T* s, int support, int lo, i
   for (int e = threadIdx.x; e < support; e += blockDim.x) {
     const T v = s[e];
     XW x;
+    if constexpr (sizeof(XW) == 4) {
+      // X fits 31 bits, so the difference is formed modulo 2^32 (a left shift by
+      // 32 or more leaves none of the sample's bits there; a right shift drops zeros).
+      const unsigned int b = __float_as_uint(v), be = (b >> 23) & 255u;
+      if (be == 255u) {
+        xw[e] = kMark + (b << 9 ? 0 : (b >> 31 ? 2 : 1));
+        continue;
+      }
+      const unsigned int m = (b & 0x7fffffu) | (be ? 0x800000u : 0u);
+      const int sh = max((int)be, 1) - 1 - lo;
+      const unsigned int f = sh >= 0 ? __funnelshift_lc(0u, m, sh) : __funnelshift_rc(m, 0u, -sh);
+      xw[e] = (int)(((int)b < 0 ? 0u - f : f) - (unsigned int)P64);
+      continue;
+    }
     if (!isfinite(v)) {
       x = kMark + (XW)(isnan(v) ? 0 : (v > (T)0 ? 1 : 2));
     } else if (small) {
@@ -361,35 +382,41 @@ __device__ __forceinline__ void moments_slide_body(const T* __restrict__ in, T* 
   const int cm = sp.classes == 0 ? 0
                  : (__popc(sp.classes) == 1 && narrow && bits + 2 * sa.count_bits <= 62) ? 1
                                                                                       : 2;
+  // The combine in 64-bit words: n S2, S1^2 and n P + S1 below 2^62 and |S1|
+  // below 2^32 (float32 noise around a level: 2 * (15 + 10) at 31 x 31). A mean's
+  // two parts are added before they are scaled, which is exact where neither part
+  // can become subnormal.
+  const bool word = 2 * (bits + sa.count_bits) <= 62 && sp.top - lo + 1 + sa.count_bits <= 62 && r.param >= 0 &&
+                    (r.kind != kMean || sp.lo > 100);
   if constexpr (sizeof(T) == 4) {
     if (bits <= 30 && small) {
       deviations_in_place<T, int>(s, support, lo, P, true);
       __syncthreads();
       if (narrow) {
         if (cm == 0)
-          column_walk<T, 0, true, 0>(smem_raw, L, s, a, sa, sp, P, bits, z, y0, x0, out);
+          column_walk<T, 0, true, 0>(smem_raw, L, s, a, sa, sp, P, bits, word, z, y0, x0, out);
         else if (cm == 1)
-          column_walk<T, 0, true, 1>(smem_raw, L, s, a, sa, sp, P, bits, z, y0, x0, out);
+          column_walk<T, 0, true, 1>(smem_raw, L, s, a, sa, sp, P, bits, word, z, y0, x0, out);
         else
-          column_walk<T, 0, true, 2>(smem_raw, L, s, a, sa, sp, P, bits, z, y0, x0, out);
+          column_walk<T, 0, true, 2>(smem_raw, L, s, a, sa, sp, P, bits, word, z, y0, x0, out);
       } else {
-        column_walk<T, 0, false, 2>(smem_raw, L, s, a, sa, sp, P, bits, z, y0, x0, out);
+        column_walk<T, 0, false, 2>(smem_raw, L, s, a, sa, sp, P, bits, word, z, y0, x0, out);
       }
     } else {
-      column_walk<T, 2, false, 2>(smem_raw, L, s, a, sa, sp, P, bits, z, y0, x0, out);
+      column_walk<T, 2, false, 2>(smem_raw, L, s, a, sa, sp, P, bits, word, z, y0, x0, out);
     }
   } else {
     deviations_in_place<T, long long>(s, support, lo, P, small);
     __syncthreads();
     if (narrow) {
       if (cm == 0)
-        column_walk<T, 1, true, 0>(smem_raw, L, s, a, sa, sp, P, bits, z, y0, x0, out);
+        column_walk<T, 1, true, 0>(smem_raw, L, s, a, sa, sp, P, bits, word, z, y0, x0, out);
       else if (cm == 1)
-        column_walk<T, 1, true, 1>(smem_raw, L, s, a, sa, sp, P, bits, z, y0, x0, out);
+        column_walk<T, 1, true, 1>(smem_raw, L, s, a, sa, sp, P, bits, word, z, y0, x0, out);
       else
-        column_walk<T, 1, true, 2>(smem_raw, L, s, a, sa, sp, P, bits, z, y0, x0, out);
+        column_walk<T, 1, true, 2>(smem_raw, L, s, a, sa, sp, P, bits, word, z, y0, x0, out);
     } else {
-      column_walk<T, 1, false, 2>(smem_raw, L, s, a, sa, sp, P, bits, z, y0, x0, out);
+      column_walk<T, 1, false, 2>(smem_raw, L, s, a, sa, sp, P, bits, word, z, y0, x0, out);
     }
   }
 }
@@ -472,11 +499,11 @@ cudaError_t launch_t(const Plan& p, const T* in, T* out, cudaStream_t s) {
 
 // Tile shape and chunk rows of the sliding moments kernel, in the order
 // measured fastest on the GB300 (4096^2 float32 / float64): 64 x 32 outputs
-// in chunks of 16 rows for most windows (31 x 31: 0.53 ms; 9 x 9: 0.36 ms;
+// in chunks of 16 rows for most windows (31 x 31: 0.43 ms; 9 x 9: 0.29 ms;
 // 31 x 31 float64: 1.87 ms); 128 x 16 in chunks of 8 for flat windows whose
-// width is at least four times their height (7 x 51: 0.48 ms; 1 x 31:
-// 0.35 ms); 128 x 64 / 64 x 64 in chunks of 16 for windows of 48 rows and
-// columns or more (65 x 65: 1.02 ms; 101 x 101: 1.88 ms); then smaller
+// width is at least four times their height (7 x 51: 0.48 ms; 1 x 31: 0.35 ms,
+// with the wider combine); 128 x 64 / 64 x 64 in chunks of 16 for windows of 48
+// rows and columns or more (65 x 65: 0.76 ms); then smaller
 // tiles down to 32 x 8 when shared memory is short. Single-row arrays take
 // 1024 x 1 tiles. False when the window or the array does not suit the
 // kernel (footprints, rank 3, counts beyond 16 bits, supports beyond shared
