@@ -235,10 +235,11 @@ def issue_roofline(workload: str, ms_per_step: float, sm_count: int, sm_mhz: flo
             "frac": round(achieved / peak, 4), "instructions_per_call": int(known[0]), "source": known[1]}
 
 
-# Kernels of this library one filter call launches, per algorithm (the band
-# and tiled exact means add a wider pass and the direct pass for bands or
-# tiles their words cannot hold; the separable extrema run two passes).
-LAUNCHES_PER_CALL = {"boxcar_band": 3, "boxcar_tile": 2, "extrema_passes": 2}
+# Kernels of this library one filter call launches, where it is more than one: the
+# band and tiled exact means add a wider pass and the direct pass for bands or
+# tiles their words cannot hold, the MAD and sigma clipping the pass that
+# finishes the windows their tile kernel marks.
+LAUNCHES_PER_CALL = {"boxcar_band": 3, "boxcar_tile": 2, "robust mad": 2, "robust sigma_mode": 2}
 
 
 def oracle_kind(kind: str) -> str:
@@ -1140,7 +1141,8 @@ def main() -> None:
                 device).multi_processor_count), clocks.summary().get("sm_mhz")),
             "cpu_baseline": base,
             "clocks": clocks.summary(),
-            "gpu_launches": args.steps * LAUNCHES_PER_CALL.get(plan.algorithm, 1),
+            "gpu_launches": args.steps * LAUNCHES_PER_CALL.get(
+                f"{plan.algorithm} {spec.kind}", LAUNCHES_PER_CALL.get(plan.algorithm, 1)),
             "nanstd_precision": precision,
             "batched": batched,
             "parity_check_rows64": check,
