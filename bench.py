@@ -200,11 +200,11 @@ DEFAULT_WORKLOAD = "nanmedian_sortnet_5x5_4096_f32"
 # when the kernel ends are not counted there.
 MEASURED_TRAFFIC = {
     "nanmedian_sortnet_5x5_4096_f32": (67.182592e6 + 29.531392e6, "profiles/tile_box_kernel_nanmedian_sortnet_5x5_4096_f32.md"),
-    "nanmedian_hist_65x65_4096_f32": (114.892544e6 + 111.829248e6, "profiles/histogram_kernel_nanmedian_hist_65x65_4096_f32.md"),
+    "nanmedian_hist_65x65_4096_f32": (67.946240e6 + 39.831552e6, "profiles/histogram_kernel_nanmedian_hist_65x65_4096_f32.md"),
     "nanmedian_ring_4_6_4096_f32": (67.191808e6 + 28.039424e6, "profiles/rank_network_kernel_nanmedian_ring_4_6_4096_f32.md"),
-    "nanstd_31x31_4096_f32": (67.200512e6 + 30.526208e6, "profiles/moments_slide_kernel_nanstd_31x31_4096_f32.md"),
-    "nanmin_31x31_4096_f32": (67.144192e6 + 21.329152e6, "profiles/extrema_pass_kernel_nanmin_31x31_4096_f32.md"),
-    "nanmad_5x5_4096_f32": (73.826048e6 + 668.445440e6, "profiles/robust_kernel_nanmad_5x5_4096_f32.md"),
+    "nanstd_31x31_4096_f32": (67.203072e6 + 30.213632e6, "profiles/moments_slide_kernel_nanstd_31x31_4096_f32.md"),
+    "nanmin_31x31_4096_f32": (84.810240e6 + 23.049728e6, "profiles/extrema_strip_kernel_nanmin_31x31_4096_f32.md"),
+    "nanmad_5x5_4096_f32": (67.206400e6 + 31.348736e6, "profiles/robust_tile_kernel_nanmad_5x5_4096_f32.md"),
 }
 
 
@@ -213,12 +213,12 @@ MEASURED_TRAFFIC = {
 # integer kernels, whose bound is the instruction issue rather than HBM.
 MEASURED_INSTRUCTIONS = {
     "nanmedian_sortnet_5x5_4096_f32": (211559951, "profiles/tile_box_kernel_nanmedian_sortnet_5x5_4096_f32.md"),
-    "nanmedian_hist_65x65_4096_f32": (3994439428, "profiles/histogram_kernel_nanmedian_hist_65x65_4096_f32.md"),
+    "nanmedian_hist_65x65_4096_f32": (2193752494, "profiles/histogram_kernel_nanmedian_hist_65x65_4096_f32.md"),
     "nanmedian_ring_4_6_4096_f32": (875186480, "profiles/rank_network_kernel_nanmedian_ring_4_6_4096_f32.md"),
-    "nanstd_31x31_4096_f32": (418849122, "profiles/moments_slide_kernel_nanstd_31x31_4096_f32.md"),
-    "nanmin_31x31_4096_f32": (60.5e6 + 57.8e6, "profiles/extrema_pass_kernel_nanmin_31x31_4096_f32.md"),
-    "nanmean_boxcar_31x31_4096_f32": (501907311, "profiles/boxcar_band_kernel_nanmean_boxcar_31x31_4096_f32.md"),
-    "nanmad_5x5_4096_f32": (3313524878, "profiles/robust_kernel_nanmad_5x5_4096_f32.md"),
+    "nanstd_31x31_4096_f32": (344461279, "profiles/moments_slide_kernel_nanstd_31x31_4096_f32.md"),
+    "nanmin_31x31_4096_f32": (80728736, "profiles/extrema_strip_kernel_nanmin_31x31_4096_f32.md"),
+    "nanmean_boxcar_31x31_4096_f32": (389130095, "profiles/boxcar_band_kernel_nanmean_boxcar_31x31_4096_f32.md"),
+    "nanmad_5x5_4096_f32": (593685816, "profiles/robust_tile_kernel_nanmad_5x5_4096_f32.md"),
 }
 
 
