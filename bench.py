@@ -899,10 +899,10 @@ def run_mesh(args) -> None:
                              "statistics sort each mesh and sum in exact fixed point per block"},
         "cpu_baseline": base,
         "clocks": clocks.summary(),
-        # Per call: the statistics kernel, then per map (background, rms) the
-        # spline's second-derivative and expansion passes along axis 0 and the
-        # last-axis pass.
-        "gpu_launches": args.steps * 7,
+        # Per call: the statistics and filter kernels, then per map (background,
+        # rms) the spline's second-derivative and expansion passes along axis 0 and
+        # the last axis's second derivatives, nodes and outputs.
+        "gpu_launches": args.steps * 12,
         "parity_check_full": bool(check),
     }
     print(json.dumps(line))
