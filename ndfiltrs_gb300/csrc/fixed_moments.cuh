@@ -366,6 +366,17 @@ __device__ Span<T> tile_span(const T* s, int support) {
   return sp;
 }
 
+// X of the finite float32 sample with bits b where it fits 31 bits, P being the pivot
+// modulo 2^32: the difference is formed modulo 2^32 (a left shift by 32 or more leaves none of
+// the sample's bits there; a right shift drops zeros).
+__device__ __forceinline__ int deviation32(unsigned int b, int lo, unsigned int P) {
+  const unsigned int be = (b >> 23) & 255u;
+  const unsigned int m = (b & 0x7fffffu) | (be ? 0x800000u : 0u);
+  const int sh = max((int)be, 1) - 1 - lo;
+  const unsigned int f = sh >= 0 ? __funnelshift_lc(0u, m, sh) : __funnelshift_rc(m, 0u, -sh);
+  return (int)(((int)b < 0 ? 0u - f : f) - P);
+}
+
 // Bits of |X| = |x - P| / 2^(E0 + lo): the rounded difference's exponent
 // plus one bounds the exact one.
 template <typename T>

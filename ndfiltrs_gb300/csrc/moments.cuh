@@ -226,6 +226,75 @@ __device__ __forceinline__ void tile_moments_body(const T* __restrict__ in, T* _
       const int lo = sp.lo;
       const fixm::i128 P = fixm::fixed(sp.pivot, lo);
       const bool count = !sp.all_finite;
+      const int plane = t.SH * t.SW;
+      const int bits = fixm::deviation_bits(sp);
+      const bool narrow = bits <= 31 && 2 * bits + count_bits <= 63;
+      const long long index = (z * g.H + y) * g.W + x;
+      if constexpr (sizeof(T) == 4) {
+        // Float32 tiles whose deviations fit 31 bits (noise around a level): a tap is
+        // one word, or one word and the sample's class in 10-bit fields, where 64-bit
+        // deviations and 16-bit count fields took two loads of two words. The taps'
+        // loads and adds are the time: std over a disk of 113 taps of 4096^2 with 1% NaN
+        // 1.48 -> 1.19 ms, all finite 1.27 -> 1.16.
+        if (narrow && bits <= 30 && sp.top - lo <= 62 && (!count || r.count < 1024)) {
+          int* x1 = reinterpret_cast<int*>(xs);
+          int2* x2 = reinterpret_cast<int2*>(xs);
+          for (int e = threadIdx.x; e < support; e += blockDim.x) {
+            const unsigned int b = __float_as_uint((float)s[e]);
+            if (!count)
+              x1[e] = fixm::deviation32(b, lo, (unsigned int)P);
+            else if (((b >> 23) & 255u) == 255u)
+              x2[e] = make_int2(0, b << 9 ? 1 : (b >> 31 ? 1 << 20 : 1 << 10));
+            else
+              x2[e] = make_int2(fixm::deviation32(b, lo, (unsigned int)P), 0);
+          }
+          __syncthreads();
+          if (!active) return;
+          long long s1 = 0;
+          unsigned long long s2 = 0;
+          unsigned int classes = 0;
+          auto add = [&](int o) {
+            int xi;
+            if (count) {
+              const int2 v = x2[o];
+              xi = v.x;
+              classes += (unsigned int)v.y;
+            } else {
+              xi = x1[o];
+            }
+            s1 += xi;
+            s2 += (unsigned long long)((long long)xi * xi);
+          };
+          auto each = [&](auto&& f) {
+            if (box) {
+              for (int kz = 0; kz < g.kd; ++kz)
+                for (int ky = 0; ky < g.kh; ++ky) {
+                  const int row = base + kz * plane + ky * t.SW;
+#pragma unroll 4
+                  for (int kx = 0; kx < g.kw; ++kx) f(row + kx);
+                }
+            } else {
+#pragma unroll 4
+              for (int i = 0; i < r.count; ++i) f(base + taps[i]);
+            }
+          };
+          each(add);
+          const unsigned int n0 = classes & 1023u, n1 = (classes >> 10) & 1023u, n2 = classes >> 20;
+          const unsigned int finite = (unsigned int)r.count - n0 - n1 - n2;
+          const unsigned int nanc = r.omit ? 0u : n0, pos = r.drop_inf ? 0u : n1, neg = r.drop_inf ? 0u : n2;
+          double special;
+          if (decide_special(r, (long long)finite + pos + neg, nanc != 0, pos != 0, neg != 0, &special))
+            out[index] = canonical(from_f64<T>(special));
+          else if (2 * (bits + count_bits) <= 62 && sp.top - lo + 1 + count_bits <= 62 && r.param >= 0 &&
+                   (r.kind != kMean || lo > 100))
+            out[index] = canonical(
+                fixm::fixed_combine_word(r.kind, r.param, s1, s2, finite, (long long)P, sp.e0() + lo));
+          else
+            out[index] =
+                canonical(fixm::fixed_combine_narrow<T>(r.kind, r.param, s1, s2, finite, P, sp.e0() + lo));
+          return;
+        }
+      }
       for (int e = threadIdx.x; e < support; e += blockDim.x) {
         const T v = s[e];
         xs[e] = isfinite(v) ? (long long)(fixm::fixed(v, lo) - P) : 0ll;
@@ -233,7 +302,6 @@ __device__ __forceinline__ void tile_moments_body(const T* __restrict__ in, T* _
       }
       __syncthreads();
       if (!active) return;
-      const int plane = t.SH * t.SW;
       auto visit = [&](auto&& f) {
         if (box) {
           for (int kz = 0; kz < g.kd; ++kz)
@@ -250,8 +318,6 @@ __device__ __forceinline__ void tile_moments_body(const T* __restrict__ in, T* _
           }
         }
       };
-      const int bits = fixm::deviation_bits(sp);
-      const bool narrow = bits <= 31 && 2 * bits + count_bits <= 63;
       fixm::i128 s1;
       fixm::u128 s2;
       unsigned long long cnt = 0;
@@ -270,7 +336,6 @@ __device__ __forceinline__ void tile_moments_body(const T* __restrict__ in, T* _
       const unsigned int finite = (unsigned int)(cnt & 0xFFFF), nanc = (unsigned int)((cnt >> 16) & 0xFFFF);
       const unsigned int pos = (unsigned int)((cnt >> 32) & 0xFFFF), neg = (unsigned int)(cnt >> 48);
       double special;
-      const long long index = (z * g.H + y) * g.W + x;
       if (decide_special(r, (long long)finite + pos + neg, nanc != 0, pos != 0, neg != 0, &special))
         out[index] = canonical(from_f64<T>(special));
       else

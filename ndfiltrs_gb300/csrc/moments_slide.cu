@@ -306,17 +306,11 @@ __device__ __forceinline__ void deviations_in_place(T* s, int support, int lo, i
     const T v = s[e];
     XW x;
     if constexpr (sizeof(XW) == 4) {
-      // X fits 31 bits, so the difference is formed modulo 2^32 (a left shift by
-      // 32 or more leaves none of the sample's bits there; a right shift drops zeros).
-      const unsigned int b = __float_as_uint(v), be = (b >> 23) & 255u;
-      if (be == 255u) {
+      const unsigned int b = __float_as_uint(v);
+      if (((b >> 23) & 255u) == 255u)
         xw[e] = kMark + (b << 9 ? 0 : (b >> 31 ? 2 : 1));
-        continue;
-      }
-      const unsigned int m = (b & 0x7fffffu) | (be ? 0x800000u : 0u);
-      const int sh = max((int)be, 1) - 1 - lo;
-      const unsigned int f = sh >= 0 ? __funnelshift_lc(0u, m, sh) : __funnelshift_rc(m, 0u, -sh);
-      xw[e] = (int)(((int)b < 0 ? 0u - f : f) - (unsigned int)P64);
+      else
+        xw[e] = deviation32(b, lo, (unsigned int)P64);
       continue;
     }
     if (!isfinite(v)) {
