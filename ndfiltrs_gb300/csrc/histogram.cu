@@ -112,9 +112,9 @@ struct Slot {
 
 __host__ __device__ inline long long align16(long long v) { return (v + 15) & ~15ll; }
 
-// Bytes of a box tile's axis maps: 64-bit offsets of its rows, planes and
+// Bytes of a tile's axis maps: 64-bit offsets of its rows, planes and
 // columns (not for a single row).
-__host__ __device__ inline long long box_map_bytes(int SH, int SZ, int SW) {
+__host__ __device__ inline long long axis_map_bytes(int SH, int SZ, int SW) {
   return align16(8ll * (SH + SZ + (SH * SZ > 1 ? SW : 0)));
 }
 
@@ -1294,7 +1294,7 @@ __device__ __forceinline__ void histogram_tile(const T* __restrict__ in, T* __re
   // the outer ones) | key bits [S] u16 and counters of the sort in shared
   // memory. A sort through a slot has its counters where the codes come.
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long map_bytes = FP ? 0 : box_map_bytes(a.SH, a.SZ, a.SW);
+  const long long map_bytes = FP ? 0 : axis_map_bytes(a.SH, a.SZ, a.SW);
   uint16_t* codes_s = reinterpret_cast<uint16_t*>(smem + map_bytes);
   const long long code_bytes = align16((long long)(FP ? a.S : a.S + 64) * 2);
   const long long list_bytes = FP ? align16((long long)(a.nf + 2 * a.nv + 2 * a.nh) * 2) : code_bytes;
@@ -1516,25 +1516,30 @@ struct Runs {
   int entries() const { return footprint ? nf + 2 * nv + 2 * nh : 0; }
 };
 
-// Footprints: bytes of the work region (the sort's 8-bit-digit tables, or the
-// segments' bit histograms while sliding, whichever is larger).
-size_t work_bytes_for(int S) {
+// Footprints: bytes of the work region, the largest of its three uses in turn:
+// the axis maps while gathering, the sort's 8-bit-digit tables, and the
+// segments' bit histograms while sliding. (Supports of two wide rows need 8 bytes
+// a column for the maps and for the histograms alike, and the maps the offsets of
+// the rows besides.)
+size_t work_bytes_for(int SH, int SZ, int SW) {
+  const size_t maps = (size_t)axis_map_bytes(SH, SZ, SW);
   const size_t sort = (size_t)sort_table_words(256) * 4;
-  const size_t hist = (size_t)kSegs * ((S + 31) / 32) * 4;
-  return std::max(sort, hist);
+  const size_t hist = (size_t)kSegs * (((long long)SZ * SH * SW + 31) / 32) * 4;
+  return std::max(maps, std::max(sort, hist));
 }
 
-size_t footprint_smem(int S, bool sdec, size_t key_bytes, const Runs& runs) {
-  const size_t codes = (size_t)align16((long long)S * 2);
+size_t footprint_smem(int SH, int SZ, int SW, bool sdec, size_t key_bytes, const Runs& runs) {
+  const long long S = (long long)SZ * SH * SW;
+  const size_t codes = (size_t)align16(S * 2);
   const size_t lists = (size_t)align16((long long)runs.entries() * 2);
-  const size_t decode = sdec ? (size_t)align16((long long)S * (long long)key_bytes) : 0;
-  return codes + lists + decode + work_bytes_for(S);
+  const size_t decode = sdec ? (size_t)align16(S * (long long)key_bytes) : 0;
+  return codes + lists + decode + work_bytes_for(SH, SZ, SW);
 }
 
 size_t box_smem(const Geom3& g, int tw, int th, int tz, bool in_smem) {
   const int SH = th + g.kh - 1, SW = tw + g.kw - 1, SZ = tz + g.kd - 1;
   const long long S = (long long)SZ * SH * SW;
-  const size_t maps = (size_t)box_map_bytes(SH, SZ, SW), codes = 2 * (size_t)align16((S + 64) * 2);
+  const size_t maps = (size_t)axis_map_bytes(SH, SZ, SW), codes = 2 * (size_t)align16((S + 64) * 2);
   if (in_smem) return maps + codes + (size_t)align16(S * 2) + (size_t)kCounterWords * 4;
   return maps + std::max(codes, (size_t)sort_table_words(256) * 4);
 }
@@ -1614,7 +1619,7 @@ HistChoice choose_tile(const Geom3& g, size_t key_bytes, const Runs& runs = Runs
     if (S > kMaxSupport) return;
     if (runs.footprint) {
       for (int sdec = 1; sdec >= 0; --sdec) {
-        const size_t smem = footprint_smem((int)S, sdec != 0, key_bytes, runs);
+        const size_t smem = footprint_smem(th + g.kh - 1, g.kd, tw + g.kw - 1, sdec != 0, key_bytes, runs);
         if (smem > kSmemBudget) continue;
         const double cpw = (tw + kSegs - 1) / kSegs;
         const double outputs = (double)tw * th;
@@ -1699,8 +1704,8 @@ HistArgs make_args_core(const Geom3& g, const HistChoice& c, int dtype, const Ru
   a.slot_bytes = dtype == 0 ? slot_bytes_for<uint32_t>(a.S) : slot_bytes_for<unsigned long long>(a.S);
   a.in_smem = c.in_smem;
   a.digit_bits = c.in_smem ? kDigitBits
-                           : slot_digit_bits(runs.footprint ? work_bytes_for(a.S)
-                                                            : c.smem - (size_t)box_map_bytes(a.SH, a.SZ, a.SW));
+                           : slot_digit_bits(runs.footprint ? work_bytes_for(a.SH, a.SZ, a.SW)
+                                                            : c.smem - (size_t)axis_map_bytes(a.SH, a.SZ, a.SW));
   a.patch_w = patch_width(g, c.TH);
   a.plane_magic = (unsigned int)(((1ull << 32) + a.plane - 1) / (unsigned long long)a.plane);
   a.row_magic = (unsigned int)(((1ull << 32) + a.SW - 1) / (unsigned long long)a.SW);

@@ -1,0 +1,61 @@
+"""Shared memory of the histogram kernel's tiles, as the library's host code
+chooses them (a small program linked against it; no device is needed)."""
+
+from __future__ import annotations
+
+import subprocess
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parent.parent
+
+
+@pytest.fixture(scope="module")
+def tiles(tmp_path_factory):
+    """tiles(windows): the chosen tile of each (D, H, W, kd, kh, kw, hole, double)."""
+    from ndfiltrs_gb300 import _build
+
+    library = _build.build()
+    program = tmp_path_factory.mktemp("tiles") / "histogram_tiles"
+    cuda = Path(_build.nvcc()).resolve().parent.parent / "include"
+    subprocess.run(["g++", "-std=c++17", "-O1", f"-I{cuda}", str(ROOT / "tests" / "histogram_tiles.cpp"), "-o",
+                    str(program), str(library), f"-Wl,-rpath,{library.parent}"], check=True)
+
+    def run(windows):
+        text = "\n".join(" ".join(str(int(v)) for v in w) for w in windows)
+        lines = subprocess.run([str(program)], input=text, capture_output=True, text=True, check=True).stdout.split("\n")
+        return [tuple(int(v) for v in line.split()) for line in lines if line]
+
+    return run
+
+
+def _align16(n: int) -> int:
+    return (n + 15) & ~15
+
+
+def test_footprint_tiles_hold_their_axis_maps(tiles) -> None:
+    """A footprint tile gathers its support through 64-bit offsets of the support's
+    rows, planes and columns, which lie in the last region of shared memory, after
+    the rank codes, the run lists and the decode table. The region must hold them;
+    supports of two wide rows have little else there."""
+    windows = [(d, h, w, kd, kh, kw, kw // 2, double)
+               for d, h, w in ((1, 1, 5000), (1, 512, 16384), (3, 1, 5000))
+               for kd, kh in ((1, 2), (2, 1), (1, 1), (1, 3))
+               for kw in (*range(1990, 2010), *range(2100, 2150), *range(4960, 4980), *range(9990, 10010))
+               for double in (0, 1)]
+    seen = set()
+    for (d, h, w, kd, kh, kw, hole, double), (tw, th, tz, sdec, in_smem, smem, entries) in zip(windows, tiles(windows)):
+        if tw == 0:  # run lists too long for shared memory
+            assert kw > 9000
+            continue
+        assert tz == 1 and not in_smem
+        rows, columns = (th + kh - 1) * kd, tw + kw - 1
+        support = rows * columns
+        before = _align16(2 * support) + _align16(2 * entries) + (_align16(support * (8 if double else 4)) if sdec else 0)
+        bitsets = 32 * 4 * ((support + 31) // 32)
+        maps = 8 * (th + kh - 1 + kd + (columns if rows > 1 else 0))
+        assert smem >= before + max(bitsets, maps, 17 * 256 * 4), (d, h, w, kd, kh, kw)
+        if rows == 2:
+            seen.add(columns % 16)
+    assert seen >= {13, 14, 15, 0, 1}
