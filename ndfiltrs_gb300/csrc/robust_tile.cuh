@@ -149,8 +149,8 @@ static __device__ __noinline__ float mad_general(const float* c, int n, double s
 // The same for samples that are multiples of 2^low. Differences below 2^24 of
 // those units are exact in float32, so the least maxima are the deviations
 // themselves and ties are equal deviations; their product with the scale (a pair
-// of floats, to 2^-49) is the float32 rounding of the float64 one when it rounds
-// the same 2^-40 above and below.
+// of floats, to 2^-49; zero where a pair does not hold the scale so well) is the
+// float32 rounding of the float64 one when it rounds the same 2^-40 above and below.
 __device__ __forceinline__ float mad_value(const Column& s, int n, int low, float2 scale, double scale64) {
   const int h = n / 2;
   const bool even = (n & 1) == 0;
@@ -510,9 +510,12 @@ cudaError_t launch_width(const Plan& p, const float* in, float* out, cudaStream_
     smem = p.smem_bytes;
   }
   const size_t columns = (smem + 15) & ~(size_t)15;
-  const float scale = (float)p.robust.parameter;
-  kernel<<<(unsigned)args.t.tiles, kT, columns + kColumns, s>>>(
-      in, out, args, taps, map, p.robust, make_float2(scale, (float)(p.robust.parameter - (double)scale)), (int)columns);
+  // The second float of a scale below 2^-100 lies among the subnormals and lacks
+  // bits that the product's bound counts on: no pair, every window in float64.
+  const float scale = p.robust.parameter >= 7.888609052210118e-31 ? (float)p.robust.parameter : 0.0f;
+  const float rest = scale > 0.0f ? (float)(p.robust.parameter - (double)scale) : 0.0f;
+  kernel<<<(unsigned)args.t.tiles, kT, columns + kColumns, s>>>(in, out, args, taps, map, p.robust,
+                                                                make_float2(scale, rest), (int)columns);
   return cudaGetLastError();
 }
 
