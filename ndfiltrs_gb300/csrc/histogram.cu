@@ -67,6 +67,7 @@ struct HistArgs {
   int digit_bits;           // largest radix digit width of the block sort (8 to 11)
   int patch_w;              // boxes: columns of a warp's patch of outputs (8 or 32)
   int in_smem;              // boxes: the support is sorted in shared memory (else through a slot)
+  int column_map;           // the columns' offsets lie in a table (else mapped as they go)
   unsigned int row_magic;   // ceil(2^32 / SW): row of an in-plane support index
   unsigned int plane_magic; // ceil(2^32 / plane): plane of a support index
   Reduce r;
@@ -112,10 +113,10 @@ struct Slot {
 
 __host__ __device__ inline long long align16(long long v) { return (v + 15) & ~15ll; }
 
-// Bytes of a tile's axis maps: 64-bit offsets of its rows, planes and
-// columns (not for a single row).
-__host__ __device__ inline long long axis_map_bytes(int SH, int SZ, int SW) {
-  return align16(8ll * (SH + SZ + (SH * SZ > 1 ? SW : 0)));
+// Bytes of a tile's axis maps: 64-bit offsets of its rows and planes, and of
+// its columns where those have a table.
+__host__ __device__ inline long long axis_map_bytes(int SH, int SZ, int SW, bool column_map) {
+  return align16(8ll * (SH + SZ + (column_map ? SW : 0)));
 }
 
 template <typename K>
@@ -675,8 +676,8 @@ __device__ __forceinline__ void walk(const uint16_t* codes, const uint16_t* list
 
 // ---------------------------------------------------------------------------
 // A tile's support: its samples in the array, each axis mapped through its
-// boundary mode once per tile. (A single row maps its columns as it goes: a
-// table for it would not fit.)
+// boundary mode once per tile. (A single row maps its columns as it goes, as do
+// supports so wide that a table would leave no room for their codes.)
 template <typename T>
 struct Support {
   using K = typename KeyOf<T>::K;
@@ -691,13 +692,12 @@ struct Support {
     long long m;
     return map_index(x0 + sx - a.g.ax, a.g.W, a.g.mx, &m) ? m : -1;
   }
-  __device__ __forceinline__ bool line() const { return a.SZ * a.SH == 1; }
 
   // Fill the tables (the caller synchronizes).
   __device__ __forceinline__ void build(long long z0, long long y0) {
     const Geom3& g = a.g;
     const int lines = a.SH + a.SZ;
-    for (int i = threadIdx.x; i < lines + (line() ? 0 : a.SW); i += blockDim.x) {
+    for (int i = threadIdx.x; i < lines + (a.column_map ? a.SW : 0); i += blockDim.x) {
       long long m;
       if (i < a.SH)
         row_map[i] = map_index(y0 + i - g.ay, g.H, g.my, &m) ? m * g.W : -1;
@@ -708,17 +708,22 @@ struct Support {
     }
   }
 
-  // f(support index, key) for every sample, rows to warps.
+  // f(support index, key) for every sample, rows to warps (rows without a table to
+  // the whole block).
   template <typename F>
   __device__ __forceinline__ void each(F&& f) const {
     const bool drop_inf = a.r.drop_inf;
     const K out_key = sample_key<T>(outside, drop_inf);
-    if (line()) {
-      const bool inside = row_map[0] >= 0 && row_map[1] >= 0;
-      const T* src = in + (inside ? row_map[0] + row_map[1] : 0);
-      for (int sx = threadIdx.x; sx < a.SW; sx += blockDim.x) {
-        const long long ox = column(sx);
-        f(sx, inside && ox >= 0 ? sample_key<T>(__ldg(src + ox), drop_inf) : out_key);
+    if (!a.column_map) {
+      for (int row = 0; row < a.SZ * a.SH; ++row) {
+        const int sz = row / a.SH;
+        const long long oy = row_map[row - sz * a.SH], oz = row_map[a.SH + sz];
+        const bool inside = oy >= 0 && oz >= 0;
+        const T* src = in + (inside ? oy + oz : 0);
+        for (int sx = threadIdx.x; sx < a.SW; sx += blockDim.x) {
+          const long long ox = column(sx);
+          f(row * a.SW + sx, inside && ox >= 0 ? sample_key<T>(__ldg(src + ox), drop_inf) : out_key);
+        }
       }
       return;
     }
@@ -746,7 +751,7 @@ struct Support {
     const unsigned int sy = __umulhi(e, a.row_magic);
     const int sx = (int)(e - sy * a.SW);
     const long long oy = row_map[sy], oz = row_map[a.SH + sz];
-    const long long ox = line() ? column(sx) : column_map[sx];
+    const long long ox = a.column_map ? column_map[sx] : column(sx);
     return oy >= 0 && oz >= 0 && ox >= 0 ? __ldg(in + oy + oz + ox) : outside;
   }
 };
@@ -1294,7 +1299,7 @@ __device__ __forceinline__ void histogram_tile(const T* __restrict__ in, T* __re
   // the outer ones) | key bits [S] u16 and counters of the sort in shared
   // memory. A sort through a slot has its counters where the codes come.
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long map_bytes = FP ? 0 : axis_map_bytes(a.SH, a.SZ, a.SW);
+  const long long map_bytes = FP ? 0 : axis_map_bytes(a.SH, a.SZ, a.SW, a.column_map);
   uint16_t* codes_s = reinterpret_cast<uint16_t*>(smem + map_bytes);
   const long long code_bytes = align16((long long)(FP ? a.S : a.S + 64) * 2);
   const long long list_bytes = FP ? align16((long long)(a.nf + 2 * a.nv + 2 * a.nh) * 2) : code_bytes;
@@ -1502,6 +1507,7 @@ struct HistChoice {
   int TW = 0, TH = 0, TZ = 1;
   bool sdec = false;     // footprints: sorted keys in shared memory
   bool in_smem = false;  // boxes: sorted in shared memory
+  bool column_map = false;
   size_t smem = 0;
 };
 
@@ -1521,25 +1527,25 @@ struct Runs {
 // segments' bit histograms while sliding. (Supports of two wide rows need 8 bytes
 // a column for the maps and for the histograms alike, and the maps the offsets of
 // the rows besides.)
-size_t work_bytes_for(int SH, int SZ, int SW) {
-  const size_t maps = (size_t)axis_map_bytes(SH, SZ, SW);
+size_t work_bytes_for(int SH, int SZ, int SW, bool column_map) {
+  const size_t maps = (size_t)axis_map_bytes(SH, SZ, SW, column_map);
   const size_t sort = (size_t)sort_table_words(256) * 4;
   const size_t hist = (size_t)kSegs * (((long long)SZ * SH * SW + 31) / 32) * 4;
   return std::max(maps, std::max(sort, hist));
 }
 
-size_t footprint_smem(int SH, int SZ, int SW, bool sdec, size_t key_bytes, const Runs& runs) {
+size_t footprint_smem(int SH, int SZ, int SW, bool column_map, bool sdec, size_t key_bytes, const Runs& runs) {
   const long long S = (long long)SZ * SH * SW;
   const size_t codes = (size_t)align16(S * 2);
   const size_t lists = (size_t)align16((long long)runs.entries() * 2);
   const size_t decode = sdec ? (size_t)align16(S * (long long)key_bytes) : 0;
-  return codes + lists + decode + work_bytes_for(SH, SZ, SW);
+  return codes + lists + decode + work_bytes_for(SH, SZ, SW, column_map);
 }
 
-size_t box_smem(const Geom3& g, int tw, int th, int tz, bool in_smem) {
+size_t box_smem(const Geom3& g, int tw, int th, int tz, bool column_map, bool in_smem) {
   const int SH = th + g.kh - 1, SW = tw + g.kw - 1, SZ = tz + g.kd - 1;
   const long long S = (long long)SZ * SH * SW;
-  const size_t maps = (size_t)axis_map_bytes(SH, SZ, SW), codes = 2 * (size_t)align16((S + 64) * 2);
+  const size_t maps = (size_t)axis_map_bytes(SH, SZ, SW, column_map), codes = 2 * (size_t)align16((S + 64) * 2);
   if (in_smem) return maps + codes + (size_t)align16(S * 2) + (size_t)kCounterWords * 4;
   return maps + std::max(codes, (size_t)sort_table_words(256) * 4);
 }
@@ -1614,12 +1620,19 @@ HistChoice choose_tile(const Geom3& g, size_t key_bytes, const Runs& runs = Runs
   if ((long long)g.kw > kMaxSupport || (long long)g.kh > kMaxSupport || (long long)g.kd > kMaxSupport)
     return best;
   double best_cost = 1e300;
+  // Columns go through a table, but for single rows and where no tile has room for
+  // one: 8 bytes a column beside the 4 of each sample's code and place would shut
+  // out boxes of two rows beyond 14,350 columns and of three beyond 11,473, which fit
+  // without it (up to some 28,000 and 19,000).
+  bool tables = true;
   auto consider = [&](int tw, int th, int tz = 1) {
-    long long S = (long long)(g.kd + tz - 1) * (tw + g.kw - 1) * (th + g.kh - 1);
+    const int SH = th + g.kh - 1, SZ = tz + g.kd - 1, SW = tw + g.kw - 1;
+    const long long S = (long long)SZ * SW * SH;
     if (S > kMaxSupport) return;
+    const bool column_map = tables && SH * SZ > 1;
     if (runs.footprint) {
       for (int sdec = 1; sdec >= 0; --sdec) {
-        const size_t smem = footprint_smem(th + g.kh - 1, g.kd, tw + g.kw - 1, sdec != 0, key_bytes, runs);
+        const size_t smem = footprint_smem(SH, SZ, SW, column_map, sdec != 0, key_bytes, runs);
         if (smem > kSmemBudget) continue;
         const double cpw = (tw + kSegs - 1) / kSegs;
         const double outputs = (double)tw * th;
@@ -1631,6 +1644,7 @@ HistChoice choose_tile(const Geom3& g, size_t key_bytes, const Runs& runs = Runs
           best.TW = tw;
           best.TH = th;
           best.sdec = sdec != 0;
+          best.column_map = column_map;
           best.smem = smem;
         }
         return;
@@ -1638,7 +1652,7 @@ HistChoice choose_tile(const Geom3& g, size_t key_bytes, const Runs& runs = Runs
       return;
     }
     for (int in_smem = 1; in_smem >= 0; --in_smem) {
-      const size_t smem = box_smem(g, tw, th, tz, in_smem != 0);
+      const size_t smem = box_smem(g, tw, th, tz, column_map, in_smem != 0);
       if (smem > kSmemBudget) continue;
       // Tiles that an SM takes one after the other, whole ones: small arrays
       // prefer tiles that leave no SM idle. Two resident blocks overlap.
@@ -1652,6 +1666,7 @@ HistChoice choose_tile(const Geom3& g, size_t key_bytes, const Runs& runs = Runs
         best.TH = th;
         best.TZ = tz;
         best.in_smem = in_smem != 0;
+        best.column_map = column_map;
         best.smem = smem;
       }
     }
@@ -1665,22 +1680,29 @@ HistChoice choose_tile(const Geom3& g, size_t key_bytes, const Runs& runs = Runs
       if (tw <= 32 || tw / 2 < g.W) consider(tw, 1);
     return best;
   }
-  for (int tw : {128, 64, 32, 16}) {
-    if (tw > 32 && tw / 2 >= g.W) continue;
-    if (tw == 16 && (runs.footprint || g.kd == 1)) continue;
-    for (int th : {256, 192, 128, 96, 64, 48, 32, 16, 8, 4, 2, 1}) {
-      if (th > 1 && th / 2 >= g.H) continue;
-      consider(tw, th);
+  auto consider_all = [&] {
+    for (int tw : {128, 64, 32, 16}) {
+      if (tw > 32 && tw / 2 >= g.W) continue;
+      if (tw == 16 && (runs.footprint || g.kd == 1)) continue;
+      for (int th : {256, 192, 128, 96, 64, 48, 32, 16, 8, 4, 2, 1}) {
+        if (th > 1 && th / 2 >= g.H) continue;
+        consider(tw, th);
+      }
+      if (runs.footprint) continue;
+      // Boxes also take the heights between, where a support just fits, and deep
+      // ones several planes.
+      for (int th = 120; th > 8; th -= 4)
+        if (th / 2 < g.H) consider(tw, th);
+      if (g.kd > 1)
+        for (int tz : {2, 4, 8, 16})
+          for (int th = 64; th >= 4; th -= 4)
+            if (th / 2 < g.H && tz / 2 < g.D) consider(tw, th, tz);
     }
-    if (runs.footprint) continue;
-    // Boxes also take the heights between, where a support just fits, and deep
-    // ones several planes.
-    for (int th = 120; th > 8; th -= 4)
-      if (th / 2 < g.H) consider(tw, th);
-    if (g.kd > 1)
-      for (int tz : {2, 4, 8, 16})
-        for (int th = 64; th >= 4; th -= 4)
-          if (th / 2 < g.H && tz / 2 < g.D) consider(tw, th, tz);
+  };
+  consider_all();
+  if (best.TW == 0) {
+    tables = false;
+    consider_all();
   }
   return best;
 }
@@ -1703,9 +1725,11 @@ HistArgs make_args_core(const Geom3& g, const HistChoice& c, int dtype, const Ru
   a.words = (a.S + 31) / 32;
   a.slot_bytes = dtype == 0 ? slot_bytes_for<uint32_t>(a.S) : slot_bytes_for<unsigned long long>(a.S);
   a.in_smem = c.in_smem;
+  a.column_map = c.column_map;
   a.digit_bits = c.in_smem ? kDigitBits
-                           : slot_digit_bits(runs.footprint ? work_bytes_for(a.SH, a.SZ, a.SW)
-                                                            : c.smem - (size_t)axis_map_bytes(a.SH, a.SZ, a.SW));
+                           : slot_digit_bits(runs.footprint
+                                                 ? work_bytes_for(a.SH, a.SZ, a.SW, c.column_map)
+                                                 : c.smem - (size_t)axis_map_bytes(a.SH, a.SZ, a.SW, c.column_map));
   a.patch_w = patch_width(g, c.TH);
   a.plane_magic = (unsigned int)(((1ull << 32) + a.plane - 1) / (unsigned long long)a.plane);
   a.row_magic = (unsigned int)(((1ull << 32) + a.SW - 1) / (unsigned long long)a.SW);
@@ -1733,6 +1757,7 @@ HistChoice plan_choice(const Plan& p) {
   c.TZ = p.hist_block_d;
   c.sdec = p.hist_sdec;
   c.in_smem = p.hist_in_smem;
+  c.column_map = p.hist_column_map;
   c.smem = p.hist_smem;
   return c;
 }
@@ -1813,6 +1838,7 @@ void histogram_configure(Plan& p, int tw, int th) {
   p.hist_block_d = c.TZ;
   p.hist_sdec = c.sdec;
   p.hist_in_smem = c.in_smem;
+  p.hist_column_map = c.column_map;
   p.hist_smem = c.smem;
   p.hist_footprint = runs.footprint;
   p.hist_nf = runs.nf;

@@ -171,6 +171,7 @@ struct Plan {
   int hist_block_w = 0, hist_block_h = 0, hist_block_d = 1;
   bool hist_sdec = false;     // footprints: sorted keys staged in shared memory
   bool hist_in_smem = false;  // boxes: the block sort stays in shared memory
+  bool hist_column_map = false;  // the tile's columns have a table of offsets
   size_t hist_smem = 0;       // shared-memory bytes of the tile
   long long hist_blocks_x = 0, hist_blocks_y = 0;
   // Footprint windows: tap and run-end offsets in the tile's support

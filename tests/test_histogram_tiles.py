@@ -59,3 +59,30 @@ def test_footprint_tiles_hold_their_axis_maps(tiles) -> None:
         if rows == 2:
             seen.add(columns % 16)
     assert seen >= {13, 14, 15, 0, 1}
+
+
+def test_wide_boxes_find_a_tile(tiles) -> None:
+    """Boxes of a few very wide rows: every box whose smallest tile fits the
+    225 KB at six bytes a sample (rank codes and 32 segments' bit histograms; the
+    run lists too of boxes deeper than a plane) has a tile, and the tile holds
+    its codes, its places and the offsets of its rows."""
+    budget = 225 * 1024
+    windows, fits = [], 0
+    for d, h, w in ((1, 1, 4000), (1, 3, 3000), (1, 600, 20000), (4, 5, 3000)):
+        for kd, kh in ((1, 1), (1, 2), (1, 3), (1, 4), (1, 5), (1, 9), (2, 1), (3, 1), (2, 2)):
+            if kd > 1 and d == 1:
+                continue
+            limit = 40000 // (kd * kh)
+            windows += [(d, h, w, kd, kh, kw, -1, 0) for kw in range(limit // 4, limit, 97)]
+    for (d, h, w, kd, kh, kw, _, _), (tw, th, tz, _, in_smem, smem, _) in zip(windows, tiles(windows)):
+        smallest = kd * kh * (kw + 31)
+        lists = 2 * (kd * kh * kw + 2 * kd * kw + 2 * kd * kh) if kd > 1 else 0
+        if 2 * smallest + 16 + lists + 16 + max(17 * 256 * 4, 128 * ((smallest + 31) // 32)) > budget:
+            continue
+        fits += 1
+        assert tw > 0, (d, h, w, kd, kh, kw)
+        rows = (th + kh - 1) * (tz + kd - 1)
+        support = rows * (tw + kw - 1)
+        need = 8 * (th + kh - 1 + tz + kd - 1) + 2 * _align16(2 * (support + 64))
+        assert need + (2 * support + 16 * 1024 if in_smem else 0) <= smem <= budget
+    assert fits > 500
