@@ -66,6 +66,7 @@ struct HistArgs {
   long long slot_bytes;     // scratch bytes per block slot (sorts through a slot)
   int digit_bits;           // largest radix digit width of the block sort (8 to 11)
   int patch_w;              // boxes: columns of a warp's patch of outputs (8 or 32)
+  int sideways;             // patches of one row are walked along it (else down)
   int in_smem;              // boxes: the support is sorted in shared memory (else through a slot)
   int column_map;           // the columns' offsets lie in a table (else mapped as they go)
   unsigned int row_magic;   // ceil(2^32 / SW): row of an in-plane support index
@@ -708,22 +709,22 @@ struct Support {
     }
   }
 
-  // f(support index, key) for every sample, rows to warps (rows without a table to
-  // the whole block).
+  // f(support index, key) for every sample, rows to warps (without a table of columns:
+  // samples to threads).
   template <typename F>
   __device__ __forceinline__ void each(F&& f) const {
     const bool drop_inf = a.r.drop_inf;
     const K out_key = sample_key<T>(outside, drop_inf);
     if (!a.column_map) {
-      for (int row = 0; row < a.SZ * a.SH; ++row) {
-        const int sz = row / a.SH;
-        const long long oy = row_map[row - sz * a.SH], oz = row_map[a.SH + sz];
-        const bool inside = oy >= 0 && oz >= 0;
-        const T* src = in + (inside ? oy + oz : 0);
-        for (int sx = threadIdx.x; sx < a.SW; sx += blockDim.x) {
-          const long long ox = column(sx);
-          f(row * a.SW + sx, inside && ox >= 0 ? sample_key<T>(__ldg(src + ox), drop_inf) : out_key);
-        }
+      if (a.SZ * a.SH > 1) {
+        for (int e = threadIdx.x; e < a.S; e += blockDim.x) f(e, sample_key<T>(value(e), drop_inf));
+        return;
+      }
+      const bool inside = row_map[0] >= 0 && row_map[1] >= 0;
+      const T* src = in + (inside ? row_map[0] + row_map[1] : 0);
+      for (int sx = threadIdx.x; sx < a.SW; sx += blockDim.x) {
+        const long long ox = column(sx);
+        f(sx, inside && ox >= 0 ? sample_key<T>(__ldg(src + ox), drop_inf) : out_key);
       }
       return;
     }
@@ -1006,12 +1007,12 @@ struct PatchWalk {
   int below, dropped;     // the lane's window: samples of rank below t, dropped samples
   Transpose transpose;
 
-  // Add to the lane's counts those of two support rows (its kw columns from
+  // Add to the lane's counts those of two support rows (`width` columns from
   // px + lx), negated for the first if FLIP; `first` and `second` say whether
   // the rows lie in (or leave and enter) the lane's window. `row` is the first
   // one's start, the second lies `apart` codes further.
   template <bool FLIP>
-  __device__ __forceinline__ void add_rows(const uint16_t* row, int apart, bool first, bool second) {
+  __device__ __forceinline__ void add_rows(const uint16_t* row, int width, int apart, bool first, bool second) {
     const uint16_t* at = row + px + (threadIdx.x & 31);
     int u = at[0], v = at[apart];
     unsigned int a0 = __ballot_sync(kFull, u < t), b0 = __ballot_sync(kFull, v < t), c0 = 0, d0 = 0;
@@ -1020,7 +1021,7 @@ struct PatchWalk {
       d0 = __ballot_sync(kFull, v >= (int)kPropagated);
     }
     int na = 0, nb = 0, nc = 0, nd = 0;
-    int left = a.g.kw;
+    int left = width;
 #pragma unroll 1
     for (; left >= 32; left -= 32) {
       at += 32;
@@ -1079,20 +1080,32 @@ struct PatchWalk {
       const uint16_t* row = codes + (pz + dz) * a.plane + py * a.SW;
       const bool deep = in_depth(dz);
       for (int q = 0; q < a.g.kh + PH - 1; q += 2, row += 2 * a.SW)
-        add_rows<false>(row, a.SW, deep && (unsigned)(q - ly) < (unsigned)a.g.kh,
+        add_rows<false>(row, a.g.kw, a.SW, deep && (unsigned)(q - ly) < (unsigned)a.g.kh,
                         deep && (unsigned)(q + 1 - ly) < (unsigned)a.g.kh);
     }
   }
 
-  // Move the windows down by the patch height.
-  __device__ __forceinline__ void move_down() {
+  // Move the windows down by the patch height or, those of a patch of one row, along
+  // it by the patch width: of each support row 32 columns leave and 32 enter.
+  __device__ __forceinline__ void move(bool sideways) {
+    if (PW == 32) {
+      const uint16_t* row = codes + py * a.SW;
+      const int rows = sideways ? a.g.kh : 1, width = sideways ? PW : a.g.kw, apart = sideways ? a.g.kw : a.g.kh * a.SW;
+#pragma unroll 1
+      for (int q = 0; q < rows; ++q, row += a.SW) add_rows<true>(row, width, apart, true, true);
+      if (sideways)
+        px += PW;
+      else
+        py += PH;
+      return;
+    }
     for (int dz = 0; dz < depth(); ++dz) {
       const uint16_t* row = codes + (pz + dz) * a.plane + py * a.SW;
       const bool deep = in_depth(dz);
 #pragma unroll 1
       for (int q = 0; q < 2 * PH - 1; ++q, row += a.SW) {
         const bool mine = deep && (PH == 1 || (unsigned)(q - ly) < (unsigned)PH);
-        add_rows<true>(row, a.g.kh * a.SW, mine, mine);
+        add_rows<true>(row, a.g.kw, a.g.kh * a.SW, mine, mine);
       }
     }
     py += PH;
@@ -1215,18 +1228,17 @@ struct PatchWalk {
     return o;
   }
 
-  // Walk patches down the tile's rows [row0, row1) of the columns from px.
-  __device__ __forceinline__ void walk(int row0, int row1, int tw_eff, int th_eff, int tz_eff,
-                                       T* __restrict__ out) {
-    // Counting whole windows costs kh + PH - 1 rows a plane, moving them
+  // Walk `patches` patches from (px, py, pz) on, down the tile's rows or along one.
+  __device__ __forceinline__ void walk(int patches, int tw_eff, int th_eff, int tz_eff, T* __restrict__ out) {
+    const bool sideways = PW == 32 && a.sideways;
+    // Counting whole windows costs kh + PH - 1 rows a plane, moving them down
     // 2 (2 PH - 1).
-    const bool recount = a.g.kh + PH - 1 <= 2 * (2 * PH - 1);
-    py = row0;
+    const bool recount = !sideways && a.g.kh + PH - 1 <= 2 * (2 * PH - 1);
     Ranks held;
     T vl = 0, vh = 0;
     long long held_at = -1;
-    for (;;) {
-      if (py == row0 || recount) count_all();
+    for (int i = 1;; ++i) {
+      if (i == 1 || recount) count_all();
       const bool live = px + lx < tw_eff && py + ly < th_eff && pz + lz < tz_eff;
       const Ranks o = select(live);
       // The previous patch's samples have arrived by now.
@@ -1237,27 +1249,27 @@ struct PatchWalk {
         vl = sup.value(place[o.lo]);
         vh = o.two ? sup.value(place[o.hi]) : vl;
       }
-      const int next = py + PH;
       const int least = __reduce_min_sync(kFull, o.valid ? o.lo : INT_MAX);
       const int most = __reduce_max_sync(kFull, o.valid ? o.hi : -1);
-      if (next >= row1) {
+      if (i == patches) {
         if (most >= 0) t = (least + most) >> 1;
         break;
       }
       if (recount) {
         if (most >= 0) t = (least + most) >> 1;
-        py = next;
+        py += PH;
       } else {
         if (most >= 0 && (t < least || t > most)) move_threshold((least + most) >> 1);
-        move_down();
+        move(sideways);
       }
     }
     if (held_at >= 0) out[held_at] = canonical(hist_value<T>(held, a, vl, vh));
   }
 };
 
-// Every patch column of a tile: columns of patches split into runs of rows so
-// that the block's warps all have work. `out` is the tile's first output.
+// Every patch of a tile: columns of patches split into runs of rows, or rows into
+// runs of columns, so that the block's warps all have work. `out` is the tile's
+// first output.
 template <typename T, int PW, bool DEEP, bool DROPS>
 __device__ __forceinline__ void walk_patches(const HistArgs& a, const uint16_t* codes, const uint16_t* place,
                                              const Support<T>& sup, int nret, int tw_eff, int th_eff, int tz_eff,
@@ -1266,17 +1278,27 @@ __device__ __forceinline__ void walk_patches(const HistArgs& a, const uint16_t* 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int across = (tw_eff + PW - 1) / PW, columns = across * ((tz_eff + Walk::PZ - 1) / Walk::PZ);
   const int rows = (th_eff + Walk::PH - 1) / Walk::PH;
-  const int runs = min(rows, max(1, kHWarps / columns));
+  const bool sideways = PW == 32 && a.sideways;
+  const int lines = sideways ? rows : columns, length = sideways ? across : rows;
+  const int runs = min(length, max(1, kHWarps / lines));
   Walk p{a, codes, place, sup, lane % PW, DEEP ? 0 : lane / PW, DEEP ? lane / PW : 0, 0, 0, 0, 0, 0, 0};
   const Reduce& r = a.r;
   p.t = r.kind == kMin ? 0 : r.kind == kMax ? nret : r.kind == kPercentile ? (int)(nret * r.q_fraction) : nret / 2;
   if (r.kind == kRank || r.kind == kRankHistogram)
     p.t = (int)min((long long)nret, r.param * nret / max(1, a.g.kd * a.g.kh * a.g.kw));
-  for (int item = warp; item < columns * runs; item += kHWarps) {
-    const int run = item / columns, column = item - run * columns, deep = column / across;
-    p.px = (column - deep * across) * PW;
-    p.pz = deep * Walk::PZ;
-    p.walk(rows * run / runs * Walk::PH, rows * (run + 1) / runs * Walk::PH, tw_eff, th_eff, tz_eff, out);
+  for (int item = warp; item < lines * runs; item += kHWarps) {
+    const int run = item / lines, line = item - run * lines;
+    const int begin = length * run / runs, end = length * (run + 1) / runs;
+    if (sideways) {
+      p.px = begin * PW;
+      p.py = line;
+    } else {
+      const int deep = line / across;
+      p.px = (line - deep * across) * PW;
+      p.pz = deep * Walk::PZ;
+      p.py = begin * Walk::PH;
+    }
+    p.walk(end - begin, tw_eff, th_eff, tz_eff, out);
   }
 }
 
@@ -1587,16 +1609,20 @@ int patch_width(const Geom3& g, int th) { return th % 4 != 0 && g.kd == 1 ? 32 :
 // over the window and with the spread of the patch's order statistics (that of
 // windows shifted across the patch, for independent samples, and 1% of the
 // support for a slope).
-double box_cost(const Geom3& g, int tw, int th, int tz, double S, bool in_smem) {
+double box_cost(const Geom3& g, int tw, int th, int tz, double S, bool in_smem, bool sideways) {
   const int pw = patch_width(g, th), lines = 32 / pw;
   const bool deep = g.kd > 1;
+  if (sideways && pw != 32) return 1e300;
   const int ph = deep ? 1 : lines, pz = deep ? lines : 1;
   const double outputs = (double)tw * th * tz, volume = (double)g.kd * g.kh * g.kw;
   const double words = (g.kw + pw - 1 + 31) / 32;
   const double pair = 20.0 * words + 25.0;
   const double planes = g.kd + pz - 1;
-  const double all = planes * (g.kh + ph - 1) / 2, moved = planes * (2 * ph - 1);
-  const double columns = (double)(tw / pw) * ((tz + pz - 1) / pz), steps_all = std::max(1, th / ph);
+  const double all = sideways ? (g.kh + 1) / 2 : planes * (g.kh + ph - 1) / 2;
+  // Moving a patch along its row counts two words of each support row.
+  const double moved = sideways ? g.kh * 65.0 / pair : planes * (2 * ph - 1);
+  double columns = (double)(tw / pw) * ((tz + pz - 1) / pz), steps_all = std::max(1, th / ph);
+  if (sideways) std::swap(columns, steps_all);
   const double runs = std::min(steps_all, std::max(1.0, kHWarps / columns));
   const double steps = std::max(1.0, steps_all / runs);
   const double pairs = std::min(all, moved + all / steps);
@@ -1606,6 +1632,15 @@ double box_cost(const Geom3& g, int tw, int th, int tz, double S, bool in_smem) 
   const double idle = std::max(1.0, kHWarps / (columns * runs));
   const double patches = outputs / 32.0 * (deep ? (double)pz * ((tz + pz - 1) / pz) / tz : 1.0);
   return (in_smem ? 13.0 : 29.0) * S + 12000.0 + idle * patches * (pairs * pair + 65.0 * (ranks / 32.0 + 2.0) + 250.0);
+}
+
+// Whether a tile's patches are walked along its rows: those of one row, where the
+// windows are so wide that moving them beats counting them again. (Counted anew for
+// every patch, a median over 20,001 samples of a line of 2^20 took 1.01 ms and one of
+// 2 x 10001 over 512 x 2048 11.5 ms, the latter in tiles of at most 128 columns too;
+// walked along rows of up to 1,024 columns 0.24 and 1.03.)
+bool walks_sideways(const Geom3& g, int tw, int th, int tz, double S, bool in_smem) {
+  return box_cost(g, tw, th, tz, S, in_smem, true) < box_cost(g, tw, th, tz, S, in_smem, false);
 }
 
 // Pick the output tile by a cost model: for boxes box_cost; for footprints in
@@ -1659,7 +1694,8 @@ HistChoice choose_tile(const Geom3& g, size_t key_bytes, const Runs& runs = Runs
       const double tiles = std::ceil((double)g.W / tw) * std::ceil((double)g.H / th) * std::ceil((double)g.D / tz);
       const double turns = std::ceil(tiles / kBoxSMs);
       const double cost = turns * (smem <= kSmemPair && turns > 1 ? 0.75 : 1.0) *
-                          box_cost(g, tw, th, tz, (double)S, in_smem != 0);
+                          std::min(box_cost(g, tw, th, tz, (double)S, in_smem != 0, false),
+                                   box_cost(g, tw, th, tz, (double)S, in_smem != 0, true));
       if (cost < best_cost) {
         best_cost = cost;
         best.TW = tw;
@@ -1681,6 +1717,12 @@ HistChoice choose_tile(const Geom3& g, size_t key_bytes, const Runs& runs = Runs
     return best;
   }
   auto consider_all = [&] {
+    // Flat windows thousands of columns wide: longer rows share their support among
+    // more outputs.
+    if (!runs.footprint && g.kd == 1 && g.kw >= 1024)
+      for (int tw : {1024, 512, 256})
+        for (int th : {1, 2})
+          if (tw / 2 < g.W && th <= g.H) consider(tw, th);
     for (int tw : {128, 64, 32, 16}) {
       if (tw > 32 && tw / 2 >= g.W) continue;
       if (tw == 16 && (runs.footprint || g.kd == 1)) continue;
@@ -1731,6 +1773,7 @@ HistArgs make_args_core(const Geom3& g, const HistChoice& c, int dtype, const Ru
                                                  ? work_bytes_for(a.SH, a.SZ, a.SW, c.column_map)
                                                  : c.smem - (size_t)axis_map_bytes(a.SH, a.SZ, a.SW, c.column_map));
   a.patch_w = patch_width(g, c.TH);
+  a.sideways = !runs.footprint && walks_sideways(g, c.TW, c.TH, c.TZ, a.S, c.in_smem);
   a.plane_magic = (unsigned int)(((1ull << 32) + a.plane - 1) / (unsigned long long)a.plane);
   a.row_magic = (unsigned int)(((1ull << 32) + a.SW - 1) / (unsigned long long)a.SW);
   a.r = r;

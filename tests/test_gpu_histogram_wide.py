@@ -74,3 +74,46 @@ def test_wide_box_without_allocation(gpu, oracle) -> None:
     torch.cuda.synchronize()
     expected = oracle.window_filter(values, "median", size, mode=["reflect", "wrap"], omit_nan=True)
     np.testing.assert_array_equal(bits(target.cpu().numpy()), bits(expected))
+
+
+# Windows whose patches of outputs are walked along the rows, several to a warp:
+# (shape, size, output tile).
+SIDEWAYS = [((160000,), (2001,), (2048, 1)), ((160000,), (700,), (1024, 1)), ((100, 3000), (2, 1100), (1024, 1)),
+            ((200, 1500), (3, 1500), (512, 2)), ((300, 1100), (1, 1500), (1024, 2)), ((400, 1030), (4, 1200), (512, 2))]
+
+
+@pytest.mark.parametrize("style", ("noise", "slope", "steps", "sparse"))
+@pytest.mark.parametrize("dtype", (np.float32, np.float64))
+def test_flat_windows_match_oracle(gpu, oracle, dtype, style) -> None:
+    from ndfiltrs_gb300 import _core
+
+    for i, (shape, size, _) in enumerate(SIDEWAYS):
+        rng = np.random.default_rng(i)
+        x = np.arange(shape[-1])
+        values = rng.normal(size=shape)
+        if style == "slope":
+            values = 0.01 * values + x
+        elif style == "steps":
+            values = np.where(x // 150 % 2 == 0, -1e3, 1e3) + np.round(values)
+        elif style == "sparse":
+            values[rng.random(shape) < 0.995] = np.nan
+        values[rng.random(shape) < 0.0003] = np.inf
+        values = values.astype(dtype)
+        if style == "noise":
+            values[..., 700:] = np.where(rng.random(values[..., 700:].shape) < 0.002, np.nan, values[..., 700:])
+        rows = slice(0, 6) if len(shape) == 2 else slice(None)
+        strip = values[:10] if len(shape) == 2 else values
+        mode = ["reflect"] * (len(shape) - 1) + [("wrap", "constant", "mirror")[i % 3]]
+        _core.pin_kernel("histogram")
+        try:
+            for kind, options, policies in (("median_histogram", {}, (True, False)),
+                                            ("percentile", dict(percentile=97.0), (True,))):
+                for omit in policies:
+                    with _core.Plan(shape, dtype, kind, size, mode=mode, cval=0.5, omit_nan=omit, **options) as plan:
+                        assert plan.algorithm == "histogram"
+                        actual = plan.run_host(values)[rows]
+                    expected = oracle.window_filter(strip, kind, size, mode=mode, cval=0.5, omit_nan=omit,
+                                                    q=options.get("percentile", 50.0))[rows]
+                    np.testing.assert_array_equal(bits(actual), bits(expected), err_msg=str((shape, size, kind, omit)))
+        finally:
+            _core.pin_kernel(None)

@@ -86,3 +86,14 @@ def test_wide_boxes_find_a_tile(tiles) -> None:
         need = 8 * (th + kh - 1 + tz + kd - 1) + 2 * _align16(2 * (support + 64))
         assert need + (2 * support + 16 * 1024 if in_smem else 0) <= smem <= budget
     assert fits > 500
+
+
+def test_flat_windows_share_their_supports(tiles) -> None:
+    """The windows of test_gpu_histogram_wide.py that are walked along the rows have
+    the tiles that give a warp several patches."""
+    from tests.test_gpu_histogram_wide import SIDEWAYS
+
+    for double in (0, 1):
+        windows = [(1, *((1,) * (2 - len(shape)) + shape), 1, *((1,) * (2 - len(size)) + size), -1, double)
+                   for shape, size, _ in SIDEWAYS]
+        assert [t[:2] for t in tiles(windows)] == [tile for _, _, tile in SIDEWAYS]
