@@ -30,10 +30,19 @@ bool robust_tile_configure(Plan& p) {
   const Geom3& g = p.tile.g;
   Tile& t = p.tile.t;
   // 512 outputs per block share a halo; arrays that would leave SMs without a
-  // block take 128.
+  // block take 128. Tiles are 32 columns wide, narrower over arrays of fewer and
+  // wider over arrays of few rows: 32 columns over one of 2 or 3 left the MAD
+  // slower than one window per thread of the general kernel (5 x 5 x 1 over
+  // 400 x 400 x 3: 0.22 ms there, 0.32 in tiles of 32 columns, 0.17 in tiles of 4).
+  auto covering = [](long long n, int most) {
+    int side = 1;
+    while (side < n && side < most) side *= 2;
+    return side;
+  };
   auto shape = [&](int outputs) {
-    t.TW = g.H == 1 ? outputs : 32;
-    t.TH = g.H == 1 ? 1 : outputs / 32;
+    t.TW = covering(g.W, 32);
+    t.TH = covering(g.H, outputs / t.TW);
+    t.TW = covering(g.W, outputs / t.TH);
     t.SW = t.TW + g.kw - 1;
     t.SH = t.TH + g.kh - 1;
     t.tiles_x = (g.W + t.TW - 1) / t.TW;
@@ -43,6 +52,12 @@ bool robust_tile_configure(Plan& p) {
   shape(512);
   if (t.tiles < 4ll * p.sm_count) shape(128);
   if (t.tiles >= (1ll << 31)) return false;
+  // A stack of tiny slices fills few of a block's threads. The general kernel breaks
+  // even at about an eighth of them for the MAD (20,000 slices of 4 x 4, 3 x 3 windows:
+  // 0.11 ms there, 0.14 in tiles), at a sixteenth for clipping and the mode (there 0.55
+  // and 0.24, 0.10 and 0.17 in tiles).
+  const long long threads = t.tiles * std::max(t.TW * t.TH, robust_tile::kT);
+  if (p.n_out * (ra.kind == kRobustMad ? 7 : 14) < threads) return false;
   static const int widths[] = {9, 16, 25, 32, 49, 64, 81, 128};
   int width = 0;
   for (int w : widths)
