@@ -530,12 +530,8 @@ std::vector<Candidate> plan_candidates_impl(Plan& p, int smem_limit) {
   }
   const bool hist_kind = p.r.kind == kMedianHistogram || p.r.kind == kRankHistogram;
   const int width = network_width_for(p.dtype, p.r.count);
-  bool hist_ok = false;
-  if (histogram_supported(p)) {
-    Plan probe = p;  // configuration only, no device resources
-    histogram_configure(probe);
-    hist_ok = histogram_smem(probe) <= (size_t)smem_limit;
-  }
+  Plan hist = p;  // configuration only, no device resources
+  const bool hist_ok = histogram_configure(hist) && histogram_smem(hist) <= (size_t)smem_limit;
   // Rectangular minima / maxima: the separable kernel (its cost does not grow
   // with the window) ahead of everything for windows wider than 5 x 5.
   bool extrema_ok = false, passes_ok = false;
@@ -554,14 +550,12 @@ std::vector<Candidate> plan_candidates_impl(Plan& p, int smem_limit) {
   if (hist_ok) {
     hist_tiles.push_back({Algo::kHistogram, 0, 0});
     if (p.r.count <= 2048 && g.kd == 1 && !line) {
-      Plan probe = p;
-      histogram_configure(probe);
-      const int dw = probe.hist_block_w, dh = probe.hist_block_h;
+      const int dw = hist.hist_block_w, dh = hist.hist_block_h;
       for (auto [tw, th] : {std::pair<int, int>{32, 128}, {128, 64}, {64, 64}}) {
         if (tw == dw && th == dh) continue;
         Plan q = p;
-        histogram_configure(q, tw, th);
-        if (q.hist_block_w == tw && histogram_smem(q) <= (size_t)smem_limit) hist_tiles.push_back({Algo::kHistogram, tw, th});
+        if (histogram_configure(q, tw, th) && histogram_smem(q) <= (size_t)smem_limit)
+          hist_tiles.push_back({Algo::kHistogram, tw, th});
       }
     }
   }
@@ -595,9 +589,9 @@ int apply_candidate_impl(Plan& p, const Candidate& c, int smem_limit) {
   p.algo = c.algo;
   switch (c.algo) {
     case Algo::kHistogram: {
-      histogram_configure(p, c.tw, c.th);
+      const bool ok = histogram_configure(p, c.tw, c.th);
       p.smem_bytes = histogram_smem(p);
-      if (p.smem_bytes > (size_t)smem_limit) return fail(NDF_ERR_UNSUPPORTED, "window too large");
+      if (!ok || p.smem_bytes > (size_t)smem_limit) return fail(NDF_ERR_UNSUPPORTED, "window too large");
       cudaError_t e = histogram_allocate(p);
       if (e != cudaSuccess) {
         cudaGetLastError();

@@ -1601,49 +1601,53 @@ Runs count_runs(const std::vector<uint8_t>& mask, int kd, int kh, int kw) {
 // where a tile has single rows, else 8 columns.
 int patch_width(const Geom3& g, int th) { return th % 4 != 0 && g.kd == 1 ? 32 : 8; }
 
-// Work of a box window's tile in warp instructions (measured on
-// windows from 13 x 13 to 129 x 129 and 9 x 33 x 33): the block sort of the
-// support (13 per sample in shared memory, 29 through a slot, and a share of the
-// passes' scans and barriers per tile), pairs of rows
-// counted per patch, and the ranks looked through, which grow with the support
-// over the window and with the spread of the patch's order statistics (that of
-// windows shifted across the patch, for independent samples, and 1% of the
-// support for a slope).
-double box_cost(const Geom3& g, int tw, int th, int tz, double S, bool in_smem, bool sideways) {
+// The walk over a box window's tile in warp instructions (measured on windows
+// from 13 x 13 to 129 x 129 and 9 x 33 x 33): pairs of rows counted per patch, and
+// the ranks looked through, which grow with the support over the window and with
+// the spread of the patch's order statistics (that of windows shifted across the
+// patch, for independent samples, and 1% of the support for a slope). Patches of one
+// row are walked along it where the windows are so wide that moving them beats
+// counting them again. (Counted anew for every patch, a median over 20,001 samples of
+// a line of 2^20 took 1.01 ms and one of 2 x 10001 over 512 x 2048 11.5 ms, the
+// latter in tiles of at most 128 columns too; walked along rows of up to 1,024
+// columns 0.24 and 1.03.)
+struct BoxWalk {
+  double cost;
+  bool sideways;
+};
+
+BoxWalk box_walk(const Geom3& g, int tw, int th, int tz, double S) {
   const int pw = patch_width(g, th), lines = 32 / pw;
   const bool deep = g.kd > 1;
-  if (sideways && pw != 32) return 1e300;
   const int ph = deep ? 1 : lines, pz = deep ? lines : 1;
   const double outputs = (double)tw * th * tz, volume = (double)g.kd * g.kh * g.kw;
   const double words = (g.kw + pw - 1 + 31) / 32;
   const double pair = 20.0 * words + 25.0;
   const double planes = g.kd + pz - 1;
-  const double all = sideways ? (g.kh + 1) / 2 : planes * (g.kh + ph - 1) / 2;
-  // Moving a patch along its row counts two words of each support row.
-  const double moved = sideways ? g.kh * 65.0 / pair : planes * (2 * ph - 1);
-  double columns = (double)(tw / pw) * ((tz + pz - 1) / pz), steps_all = std::max(1, th / ph);
-  if (sideways) std::swap(columns, steps_all);
-  const double runs = std::min(steps_all, std::max(1.0, kHWarps / columns));
-  const double steps = std::max(1.0, steps_all / runs);
-  const double pairs = std::min(all, moved + all / steps);
   const double shifted = deep ? (double)g.kh * g.kw * (pz - 1) : (double)g.kw * (ph - 1);
   const double moves = std::min(std::sqrt(0.5 * ((double)g.kd * g.kh * (pw - 1) + shifted)), 1.5 * std::sqrt(volume));
   const double ranks = std::min(S, 1.6 * moves * S / volume + 0.01 * S);
-  const double idle = std::max(1.0, kHWarps / (columns * runs));
   const double patches = outputs / 32.0 * (deep ? (double)pz * ((tz + pz - 1) / pz) / tz : 1.0);
-  return (in_smem ? 13.0 : 29.0) * S + 12000.0 + idle * patches * (pairs * pair + 65.0 * (ranks / 32.0 + 2.0) + 250.0);
+  // Patches in `lines` lines of `length`, whose first one costs `all` pairs of rows
+  // and the others `moved`, or `all` too if those are fewer.
+  auto walk = [&](double lines, double length, double all, double moved) {
+    const double runs = std::min(length, std::max(1.0, kHWarps / lines));
+    const double steps = std::max(1.0, length / runs);
+    const double pairs = std::min(all, moved + all / steps);
+    const double idle = std::max(1.0, kHWarps / (lines * runs));
+    return idle * patches * (pairs * pair + 65.0 * (ranks / 32.0 + 2.0) + 250.0);
+  };
+  const double across = tw / pw, columns = across * ((tz + pz - 1) / pz), rows = std::max(1, th / ph);
+  const double down = walk(columns, rows, planes * (g.kh + ph - 1) / 2, planes * (2 * ph - 1));
+  if (pw != 32) return {down, false};
+  // Moving a patch along its row counts two words of each support row.
+  const double right = walk(rows, across, (g.kh + 1) / 2, g.kh * 65.0 / pair);
+  return {std::min(down, right), right < down};
 }
 
-// Whether a tile's patches are walked along its rows: those of one row, where the
-// windows are so wide that moving them beats counting them again. (Counted anew for
-// every patch, a median over 20,001 samples of a line of 2^20 took 1.01 ms and one of
-// 2 x 10001 over 512 x 2048 11.5 ms, the latter in tiles of at most 128 columns too;
-// walked along rows of up to 1,024 columns 0.24 and 1.03.)
-bool walks_sideways(const Geom3& g, int tw, int th, int tz, double S, bool in_smem) {
-  return box_cost(g, tw, th, tz, S, in_smem, true) < box_cost(g, tw, th, tz, S, in_smem, false);
-}
-
-// Pick the output tile by a cost model: for boxes box_cost; for footprints in
+// Pick the output tile by a cost model: for boxes in warp instructions, the walk's
+// and the block sort's (13 per support sample in shared memory, 29 through a slot, and
+// a share of the passes' scans and barriers per tile); for footprints in
 // units of one histogram update per output: vertical steps, the first window
 // of each segment's walk, the column moves, the block sort (about 8 units per
 // support sample) and a global decode when the sorted keys do not fit in
@@ -1686,16 +1690,18 @@ HistChoice choose_tile(const Geom3& g, size_t key_bytes, const Runs& runs = Runs
       }
       return;
     }
+    if (box_smem(g, tw, th, tz, column_map, false) > kSmemBudget) return;
+    // Tiles that an SM takes one after the other, whole ones: small arrays
+    // prefer tiles that leave no SM idle. Two resident blocks overlap.
+    const double tiles = (double)((g.W + tw - 1) / tw * ((g.H + th - 1) / th) * ((g.D + tz - 1) / tz));
+    const double turns = std::ceil(tiles / kBoxSMs);
+    if (turns * (turns > 1 ? 0.75 : 1.0) * (13.0 * (double)S + 12000.0) >= best_cost) return;  // the sort alone
+    const double walk = box_walk(g, tw, th, tz, (double)S).cost;
     for (int in_smem = 1; in_smem >= 0; --in_smem) {
       const size_t smem = box_smem(g, tw, th, tz, column_map, in_smem != 0);
       if (smem > kSmemBudget) continue;
-      // Tiles that an SM takes one after the other, whole ones: small arrays
-      // prefer tiles that leave no SM idle. Two resident blocks overlap.
-      const double tiles = std::ceil((double)g.W / tw) * std::ceil((double)g.H / th) * std::ceil((double)g.D / tz);
-      const double turns = std::ceil(tiles / kBoxSMs);
       const double cost = turns * (smem <= kSmemPair && turns > 1 ? 0.75 : 1.0) *
-                          std::min(box_cost(g, tw, th, tz, (double)S, in_smem != 0, false),
-                                   box_cost(g, tw, th, tz, (double)S, in_smem != 0, true));
+                          ((in_smem ? 13.0 : 29.0) * (double)S + 12000.0 + walk);
       if (cost < best_cost) {
         best_cost = cost;
         best.TW = tw;
@@ -1773,7 +1779,7 @@ HistArgs make_args_core(const Geom3& g, const HistChoice& c, int dtype, const Ru
                                                  ? work_bytes_for(a.SH, a.SZ, a.SW, c.column_map)
                                                  : c.smem - (size_t)axis_map_bytes(a.SH, a.SZ, a.SW, c.column_map));
   a.patch_w = patch_width(g, c.TH);
-  a.sideways = !runs.footprint && walks_sideways(g, c.TW, c.TH, c.TZ, a.S, c.in_smem);
+  a.sideways = !runs.footprint && box_walk(g, c.TW, c.TH, c.TZ, a.S).sideways;
   a.plane_magic = (unsigned int)(((1ull << 32) + a.plane - 1) / (unsigned long long)a.plane);
   a.row_magic = (unsigned int)(((1ull << 32) + a.SW - 1) / (unsigned long long)a.SW);
   a.r = r;
@@ -1863,19 +1869,15 @@ Runs runs_of(const Plan& p) {
 
 }  // namespace
 
-bool histogram_supported(const Plan& p) {
+bool histogram_configure(Plan& p, int tw, int th) {
   if (p.ndim > 3 || p.r.count < 1) return false;
   const int k = p.r.kind;
   if (k != kMedian && k != kMedianNetwork && k != kMedianHistogram && k != kRank &&
       k != kRankHistogram && k != kMin && k != kMax && k != kPercentile)
     return false;
-  HistChoice c = choose_tile(p.tile.g, p.dtype == 0 ? 4 : 8, runs_of(p));
-  return c.TW > 0;
-}
-
-void histogram_configure(Plan& p, int tw, int th) {
   const Runs runs = runs_of(p);
   HistChoice c = choose_tile(p.tile.g, p.dtype == 0 ? 4 : 8, runs, tw, th);
+  if (c.TW == 0) return false;
   p.hist_block_w = c.TW;
   p.hist_block_h = c.TH;
   p.hist_block_d = c.TZ;
@@ -1888,7 +1890,7 @@ void histogram_configure(Plan& p, int tw, int th) {
   p.hist_nv = runs.nv;
   p.hist_nh = runs.nh;
   p.hist_lists.clear();
-  if (runs.footprint && c.TW > 0) {
+  if (runs.footprint) {
     // Support-linear offsets (zz * plane + y * SW + x) of the taps and of
     // the run ends; below the support size, so they fit 16 bits.
     const Geom3& g = p.tile.g;
@@ -1921,6 +1923,7 @@ void histogram_configure(Plan& p, int tw, int th) {
   HistArgs a = make_args(p);
   p.hist_blocks_x = a.tiles_x;
   p.hist_blocks_y = a.tiles / a.tiles_x;
+  return true;
 }
 
 size_t histogram_smem(const Plan& p) { return p.hist_smem; }

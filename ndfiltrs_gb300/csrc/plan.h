@@ -255,9 +255,9 @@ bool boxcar_band_configure(Plan& p, int smem_limit);
 size_t tile_select_smem(const Plan& p, const Tile& t);
 size_t tile_moments_smem(const Plan& p, const Tile& t);
 size_t histogram_smem(const Plan& p);
-bool histogram_supported(const Plan& p);
-// The cost model's tile, or tw x th (an autotuner candidate) when given.
-void histogram_configure(Plan& p, int tw = 0, int th = 0);
+// The cost model's tile, or tw x th (an autotuner candidate) when given. False where
+// the kernel does not take the window.
+bool histogram_configure(Plan& p, int tw = 0, int th = 0);
 cudaError_t histogram_allocate(Plan& p);
 int network_width_for(int dtype, int count);
 bool box_supported(int dtype, int kh, int kw);

@@ -28,11 +28,10 @@ int main() {
           for (int v : {(int)(i / kw / kh), (int)(i / kw % kh), (int)(i % kw)}) p.box_taps.push_back(v);
     }
     p.r.kind = 0;  // median
-    if (!ndf::histogram_supported(p)) {
+    if (!ndf::histogram_configure(p)) {
       std::printf("0 0 0 0 0 0 0\n");
       continue;
     }
-    ndf::histogram_configure(p);
     std::printf("%d %d %d %d %d %zu %d\n", p.hist_block_w, p.hist_block_h, p.hist_block_d, (int)p.hist_sdec,
                 (int)p.hist_in_smem, ndf::histogram_smem(p), p.hist_nf + 2 * p.hist_nv + 2 * p.hist_nh);
   }
