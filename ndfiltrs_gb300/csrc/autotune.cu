@@ -1,7 +1,7 @@
 // Autotuner: the kernel choice of a tileable plan (sliding histogram, box
 // pair kernel, register network or radix select, and their output tiles;
-// the moments tile) measured on the device and cached per (device, dtype,
-// statistic, invalid-value policy, window box, tap count, footprint class).
+// the moments tile) measured on the device and cached per (kernel version, device,
+// dtype, statistic, invalid-value policy, window box, tap count, footprint class).
 //
 // Every candidate computes bit-identical order statistics (and the moments
 // candidates differ only in their tiles), so a cached choice changes speed,
@@ -36,6 +36,11 @@ namespace ndf {
 int fail(int code, const std::string& message);
 
 namespace {
+
+// Version of the kernels behind the families, the first part of every key. Choices
+// that were measured on other kernels are not taken from a file: raise it with a
+// change that can turn one.
+constexpr char kKernelVersion[] = "k2";
 
 struct TuneEntry {
   Candidate c;
@@ -142,6 +147,7 @@ void load_locked(TuneCache& c) {
     std::string key, algo;
     TuneEntry e;
     if (!(fields >> key >> algo >> e.c.tw >> e.c.th >> e.ms)) continue;
+    if (key.compare(0, sizeof(kKernelVersion), std::string(kKernelVersion) + '/') != 0) continue;
     if (!parse_algo(algo, &e.c.algo)) continue;
     c.entries[key] = e;
   }
@@ -201,7 +207,7 @@ std::string key_of(const Plan& p) {
   });
   const Geom3& g = p.tile.g;
   char buf[256];
-  std::snprintf(buf, sizeof(buf), "sm%d%d-%d/%s/%s/%s/d%d%s/%dx%dx%d/V%d/%s", major, minor, p.sm_count,
+  std::snprintf(buf, sizeof(buf), "%s/sm%d%d-%d/%s/%s/%s/d%d%s/%dx%dx%d/V%d/%s", kKernelVersion, major, minor, p.sm_count,
                 p.dtype == 0 ? "f32" : "f64", statistic_class(p.r), p.r.omit ? "omit" : "propagate",
                 p.ndim, g.H == 1 ? "line" : "", g.kd, g.kh, g.kw, p.r.count,
                 p.footprint.empty() ? "box" : "footprint");
