@@ -42,3 +42,21 @@ def test_choices_of_other_kernels_are_not_taken(gpu, tmp_path) -> None:
             assert with_file(stale) == (0, usual)
     finally:
         nf.set_autotune(0, "")
+
+
+def test_box_tiles_follow_the_array(gpu) -> None:
+    """The histogram's tile of a box depends on the array's size, which a choice's
+    key does not hold: boxes have one candidate, nothing to measure, and footprints
+    several."""
+    import ndfiltrs_gb300 as nf
+    from ndfiltrs_gb300 import _core
+
+    disk = np.add.outer(np.arange(-9, 10) ** 2, np.arange(-9, 10) ** 2) <= 81
+    try:
+        nf.set_autotune(2, "")
+        for footprint, entries in ((None, 0), (disk, 1)):
+            with _core.Plan((200, 200), np.float32, "median", (19, 19), footprint=footprint, omit_nan=True) as plan:
+                assert plan.algorithm == "histogram"
+            assert nf.autotune_entries() == entries
+    finally:
+        nf.set_autotune(0, "")
