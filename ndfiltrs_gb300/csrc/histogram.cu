@@ -1534,7 +1534,6 @@ struct HistChoice {
 };
 
 constexpr size_t kSmemBudget = 225 * 1024;
-constexpr double kBoxSMs = 152;
 constexpr size_t kSmemPair = 113 * 1024 - 640;  // two blocks per SM (with 1 KB and the static variables each)
 
 // Run-list entries of a footprint window (0 for a rectangular one).
@@ -1653,7 +1652,7 @@ BoxWalk box_walk(const Geom3& g, int tw, int th, int tz, double S) {
 // support sample) and a global decode when the sorted keys do not fit in
 // shared memory. Or the given tw x th when it fits (an autotuner candidate; 0
 // when it does not).
-HistChoice choose_tile(const Geom3& g, size_t key_bytes, const Runs& runs = Runs{}, int force_tw = 0,
+HistChoice choose_tile(const Geom3& g, size_t key_bytes, int sm_count, const Runs& runs = Runs{}, int force_tw = 0,
                        int force_th = 0) {
   HistChoice best;
   if ((long long)g.kw > kMaxSupport || (long long)g.kh > kMaxSupport || (long long)g.kd > kMaxSupport)
@@ -1694,7 +1693,7 @@ HistChoice choose_tile(const Geom3& g, size_t key_bytes, const Runs& runs = Runs
     // Tiles that an SM takes one after the other, whole ones: small arrays
     // prefer tiles that leave no SM idle. Two resident blocks overlap.
     const double tiles = (double)((g.W + tw - 1) / tw * ((g.H + th - 1) / th) * ((g.D + tz - 1) / tz));
-    const double turns = std::ceil(tiles / kBoxSMs);
+    const double turns = std::ceil(tiles / std::max(1, sm_count));
     if (turns * (turns > 1 ? 0.75 : 1.0) * (13.0 * (double)S + 12000.0) >= best_cost) return;  // the sort alone
     const double walk = box_walk(g, tw, th, tz, (double)S).cost;
     for (int in_smem = 1; in_smem >= 0; --in_smem) {
@@ -1876,7 +1875,7 @@ bool histogram_configure(Plan& p, int tw, int th) {
       k != kRankHistogram && k != kMin && k != kMax && k != kPercentile)
     return false;
   const Runs runs = runs_of(p);
-  HistChoice c = choose_tile(p.tile.g, p.dtype == 0 ? 4 : 8, runs, tw, th);
+  HistChoice c = choose_tile(p.tile.g, p.dtype == 0 ? 4 : 8, p.sm_count, runs, tw, th);
   if (c.TW == 0) return false;
   p.hist_block_w = c.TW;
   p.hist_block_h = c.TH;
@@ -2147,16 +2146,16 @@ extern "C" int ndf_histogram_filter_noalloc(const void* d_in, void* d_out, int32
   r.q_is_max = percentile == 100.0;
   r.pct = nullptr;
   r.cval = dtype == NDF_FLOAT32 ? (double)(float)cval : cval;
-  HistChoice c = choose_tile(g, dtype == 0 ? 4 : 8);
+  int device = 0, sm_count = 0, optin = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+  HistChoice c = choose_tile(g, dtype == 0 ? 4 : 8, sm_count);
   if (c.TW == 0) return noalloc_fail(NDF_ERR_UNSUPPORTED, "window too large for the histogram kernel");
   HistArgs a = make_args_core(g, c, dtype, Runs{}, r);
   if ((size_t)a.slot_bytes > kNoAllocScratchBytes)
     return noalloc_fail(NDF_ERR_MEMORY,
                         "the window's sort slot exceeds the 16 MiB allocation-free scratch");
-  int device = 0, sm_count = 0, optin = 0;
-  cudaError_t e = cudaGetDevice(&device);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return noalloc_fail(NDF_ERR_NO_DEVICE, "no usable CUDA device");

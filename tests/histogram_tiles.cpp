@@ -2,19 +2,20 @@
 // host code chooses it (no device): one line "D H W kd kh kw hole double" per
 // window, "hole" being the flat position of the one missing tap of a footprint
 // (-1: a full box). Reads as "TW TH TZ sdec in_smem smem entries"; TW is 0 where
-// the kernel does not take the window.
+// the kernel does not take the window. An argument gives the device's SMs (152).
 #include <cstdio>
+#include <cstdlib>
 
 #include "../ndfiltrs_gb300/csrc/plan.h"
 
-int main() {
+int main(int argc, char** argv) {
   long long D, H, W, hole;
   int kd, kh, kw, wide;
   while (std::scanf("%lld %lld %lld %d %d %d %lld %d", &D, &H, &W, &kd, &kh, &kw, &hole, &wide) == 8) {
     ndf::Plan p;
     p.dtype = wide;
     p.ndim = D > 1 || kd > 1 ? 3 : 2;
-    p.sm_count = 152;
+    p.sm_count = argc > 1 ? std::atoi(argv[1]) : 152;
     ndf::Geom3& g = p.tile.g;
     g = ndf::Geom3{};
     g.D = D, g.H = H, g.W = W, g.kd = kd, g.kh = kh, g.kw = kw;

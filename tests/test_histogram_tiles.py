@@ -22,9 +22,9 @@ def tiles(tmp_path_factory):
     subprocess.run(["g++", "-std=c++17", "-O1", f"-I{cuda}", str(ROOT / "tests" / "histogram_tiles.cpp"), "-o",
                     str(program), str(library), f"-Wl,-rpath,{library.parent}"], check=True)
 
-    def run(windows):
+    def run(windows, sm_count=152):
         text = "\n".join(" ".join(str(int(v)) for v in w) for w in windows)
-        lines = subprocess.run([str(program)], input=text, capture_output=True, text=True, check=True).stdout.split("\n")
+        lines = subprocess.run([str(program), str(sm_count)], input=text, capture_output=True, text=True, check=True).stdout.split("\n")
         return [tuple(int(v) for v in line.split()) for line in lines if line]
 
     return run
@@ -97,3 +97,11 @@ def test_flat_windows_share_their_supports(tiles) -> None:
         windows = [(1, *((1,) * (2 - len(shape)) + shape), 1, *((1,) * (2 - len(size)) + size), -1, double)
                    for shape, size, _ in SIDEWAYS]
         assert [t[:2] for t in tiles(windows)] == [tile for _, _, tile in SIDEWAYS]
+
+
+def test_tiles_follow_the_sm_count(tiles) -> None:
+    """Small arrays take tiles that leave no SM of the device without one."""
+    windows = [(1, n, n, 1, k, k, -1, 0) for n in (300, 700, 1500) for k in (15, 33)]
+    outputs = {sms: [t[0] * t[1] for t in tiles(windows, sms)] for sms in (19, 152)}
+    assert outputs[19] != outputs[152]
+    assert all(few >= many for few, many in zip(outputs[19], outputs[152]))
