@@ -105,3 +105,14 @@ def test_tiles_follow_the_sm_count(tiles) -> None:
     outputs = {sms: [t[0] * t[1] for t in tiles(windows, sms)] for sms in (19, 152)}
     assert outputs[19] != outputs[152]
     assert all(few >= many for few, many in zip(outputs[19], outputs[152]))
+
+
+def test_deep_windows_sort_through_slots(tiles) -> None:
+    """The cubes of test_gpu_histogram_deep.py have the tiles that they are there
+    for, those of 64 x 512 x 512 among them, and slots in global memory."""
+    from tests.test_gpu_histogram_deep import CUBES
+
+    windows = [(*shape, *size, -1, double) for shape, size, double, _ in CUBES]
+    for (_, _, _, tile), chosen in zip(CUBES, tiles(windows)):
+        assert (chosen[:3], chosen[4]) == (tile, 0)
+    assert tiles([(64, 512, 512, 9, 33, 33, -1, 0)])[0][:5] == (32, 20, 8, 0, 0)
