@@ -30,7 +30,8 @@
 // instructions per output at 65 x 65 whatever the window; patches took the
 // 65 x 65 median of a 4096^2 float32 star field from 6.59 to 3.07 ms and the
 // (9, 33, 33) median of a 64 x 512 x 512 cube from 61.2 to 33.0 ms; sorting a box's
-// support in shared memory, and sharing it among four planes, to 2.42 and 15 ms.
+// support in shared memory, and sharing it among several planes (eight for that
+// cube), to 2.40 and 13.2 ms.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -286,8 +287,8 @@ __device__ __forceinline__ int select_in_word32(unsigned int word, int k) {
 // statistic is usually a few window samples away, within a word or two. A
 // walk longer than kSeqWords words continues as a parallel scan of 16 words
 // per iteration (sixteen sequential words measured 2-5% faster than four,
-// and four faster than one or two, from 13 x 13 to 65 x 65 windows; 32 no
-// faster than 16). Every loop
+// and four faster than one or two, on full windows from 13 x 13 to 65 x 65 when
+// boxes came this way too; 32 no faster than 16). Every loop
 // that contains warp-synchronous operations runs until both segments of the
 // warp are done, so the two halves stay converged.
 constexpr int kSeg = 16;

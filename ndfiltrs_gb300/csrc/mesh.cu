@@ -269,10 +269,10 @@ __device__ void m_within(V v, long long r0, long long r1, double low, double hig
 // on the FP64 pipe, exact sums among them, for bounds that almost never fall
 // within a float32 rounding of a sample. Deviations are taken from a median of
 // the samples, so that |mean| stays near the spread and nothing cancels. With
-// c terms per thread, then a tree, the sums are off by (c + 10) u of their
-// absolute sums, which bounds the error of the limits below; a limit closer to
-// its neighbouring samples than that (or sums out of float32's range) is not
-// decided, and the caller runs the float64 pass. The reference's own roundings
+// c terms per thread, a tree of five levels and up to 16 warps' parts in turn, the
+// sums are off by (c + 21) u of their absolute sums, which bounds the error of the
+// limits below; a limit closer to its neighbouring samples than that (or sums out of
+// float32's range) is not decided, and the caller runs the float64 pass. The reference's own roundings
 // lie below 2^-50 of the center. Every thread of the block gets the same answer.
 template <typename V>
 __device__ bool m_decide(V v, long long q0, long long q1, long long s0, long long s1, int center, double lower,
