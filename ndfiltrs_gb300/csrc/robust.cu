@@ -1,10 +1,12 @@
 // Robust window statistics for float32 inputs, the plan hooks and the
-// dispatch (float64 inputs instantiate in robust_f64.cu).
+// dispatch (float64 inputs instantiate in robust_f64.cu, the windows that the tile
+// kernel marked in robust_marked.cu).
 #include "robust.cuh"
 
 namespace ndf {
 
 cudaError_t launch_robust_f64(const Plan& p, const double* in, double* out, cudaStream_t s);
+cudaError_t launch_robust_marked(const Plan& p, const float* in, float* out, cudaStream_t s);
 cudaError_t launch_robust_tile(const Plan& p, const float* in, float* out, cudaStream_t s);
 bool robust_tile_configure(Plan& p);
 
@@ -29,7 +31,7 @@ cudaError_t launch_robust(const Plan& p, const void* in, void* out, cudaStream_t
   if (p.robust_width > 0) {
     // The tile kernel, then the windows that it left marked.
     cudaError_t e = launch_robust_tile(p, (const float*)in, (float*)out, s);
-    return e != cudaSuccess ? e : launch_robust_t<float>(p, (const float*)in, (float*)out, s, true);
+    return e != cudaSuccess ? e : launch_robust_marked(p, (const float*)in, (float*)out, s);
   }
   if (p.dtype == 0) return launch_robust_t<float>(p, (const float*)in, (float*)out, s);
   return launch_robust_f64(p, (const double*)in, (double*)out, s);

@@ -663,12 +663,14 @@ __device__ double robust_window(Fetch&& fetch, int V, const Reduce& r, const Rob
 }
 
 // MAXV > 0: thread-local arrays; MAXV == 0: per-thread slices of `scratch`.
-// `marked_only` (float32): only the outputs that hold kUndecided.
-template <typename T, int MAXV, bool MERGE>
+// MARKED (float32): only the outputs that hold kUndecided, whose marks a thread loads
+// several at a time. (One kernel for both, with the marks as a switch, ran every
+// output through that loop: 8% more for float64 clipping.)
+template <typename T, int MAXV, bool MERGE, bool MARKED>
 __global__ void __launch_bounds__(kRThreads)
     robust_kernel(const T* __restrict__ in, T* __restrict__ out, const __grid_constant__ GenericArgs a,
                   const long long* __restrict__ taps, const __grid_constant__ RobustArgs ra,
-                  double* __restrict__ scratch, bool marked_only) {
+                  double* __restrict__ scratch) {
   const int rank = a.rank;
   const int V = a.r.count;
   const long long* flat = taps + (long long)V * rank;
@@ -678,74 +680,80 @@ __global__ void __launch_bounds__(kRThreads)
   double* v = MAXV > 0 ? local_v : scratch + tid * 3ll * V;
   double* s = MAXV > 0 ? local_s : v + V;
   double* w = MAXV > 0 ? local_w : s + V;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long first = tid; first < a.n_out; first += kRobustChunk * stride) {
-    unsigned int todo = 0;
-#pragma unroll
-    for (int j = 0; j < kRobustChunk; ++j) {
-      const long long o = first + j * stride;
-      bool mine = o < a.n_out;
-      if constexpr (sizeof(T) == 4) {
-        if (mine && marked_only) mine = __float_as_uint(out[o]) == kUndecided;
-      }
-      todo |= mine ? 1u << j : 0u;
+  auto output = [&](long long o) {
+    long long coord[kMaxGenericRank];
+    long long rem = o;
+    bool interior = true;
+    for (int d = 0; d < rank; ++d) {
+      coord[d] = rem / a.stride[d];
+      rem -= coord[d] * a.stride[d];
+      interior = interior && coord[d] + a.low[d] >= 0 && coord[d] + a.high[d] < a.shape[d];
     }
-    for (; todo; todo &= todo - 1) {
-      const long long o = first + (__ffs((int)todo) - 1) * stride;
-      long long coord[kMaxGenericRank];
-      long long rem = o;
-      bool interior = true;
+    auto fetch = [&](int i) -> double {
+      if (interior) return widen(__ldg(in + o + flat[i]));
+      const long long* tap = taps + (long long)i * rank;
+      long long src = 0;
       for (int d = 0; d < rank; ++d) {
-        coord[d] = rem / a.stride[d];
-        rem -= coord[d] * a.stride[d];
-        interior = interior && coord[d] + a.low[d] >= 0 && coord[d] + a.high[d] < a.shape[d];
+        long long m;
+        if (!map_index(coord[d] + tap[d], a.shape[d], a.mode[d], &m)) return widen(cval);
+        src += m * a.stride[d];
       }
-      auto fetch = [&](int i) -> double {
-        if (interior) return widen(__ldg(in + o + flat[i]));
-        const long long* tap = taps + (long long)i * rank;
-        long long src = 0;
-        for (int d = 0; d < rank; ++d) {
-          long long m;
-          if (!map_index(coord[d] + tap[d], a.shape[d], a.mode[d], &m)) return widen(cval);
-          src += m * a.stride[d];
-        }
-        return widen(__ldg(in + src));
-      };
-      const double result = robust_window<MAXV, MERGE>(fetch, V, a.r, ra, v, s, w);
-      T value;
-      if constexpr (sizeof(T) == 4)
-        value = nan64(result) ? nan_of(0.0f) : __double2float_rn(result);
-      else
-        value = nan64(result) ? nan_of(0.0) : result;
-      out[o] = value;
+      return widen(__ldg(in + src));
+    };
+    const double result = robust_window<MAXV, MERGE>(fetch, V, a.r, ra, v, s, w);
+    T value;
+    if constexpr (sizeof(T) == 4)
+      value = nan64(result) ? nan_of(0.0f) : __double2float_rn(result);
+    else
+      value = nan64(result) ? nan_of(0.0) : result;
+    out[o] = value;
+  };
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  if constexpr (MARKED) {
+    for (long long first = tid; first < a.n_out; first += kRobustChunk * stride) {
+      unsigned int todo = 0;
+#pragma unroll
+      for (int j = 0; j < kRobustChunk; ++j) {
+        const long long o = first + j * stride;
+        todo |= o < a.n_out && __float_as_uint(out[o]) == kUndecided ? 1u << j : 0u;
+      }
+      for (; todo; todo &= todo - 1) output(first + (__ffs((int)todo) - 1) * stride);
     }
+  } else {
+    for (long long o = tid; o < a.n_out; o += stride) output(o);
   }
 }
 
-template <typename T, int MAXV, bool MERGE = false>
-cudaError_t launch_robust_v(const Plan& p, const T* in, T* out, cudaStream_t s, bool marked_only) {
+template <typename T, int MAXV, bool MERGE, bool MARKED>
+cudaError_t launch_robust_v(const Plan& p, const T* in, T* out, cudaStream_t s) {
   const long long blocks = MAXV > 0 ? std::max(1ll, std::min((p.n_out + kRThreads - 1) / kRThreads,
                                                              (long long)std::max(1, p.sm_count) * 16))
                                     : p.robust_threads / kRThreads;
-  robust_kernel<T, MAXV, MERGE><<<(unsigned)blocks, kRThreads, 0, s>>>(in, out, p.generic, p.d_gen_taps, p.robust,
-                                                                        reinterpret_cast<double*>(p.d_scratch), marked_only);
+  robust_kernel<T, MAXV, MERGE, MARKED><<<(unsigned)blocks, kRThreads, 0, s>>>(
+      in, out, p.generic, p.d_gen_taps, p.robust, reinterpret_cast<double*>(p.d_scratch));
   return cudaGetLastError();
 }
 
-template <typename T>
-cudaError_t launch_robust_t(const Plan& p, const T* in, T* out, cudaStream_t s, bool marked_only = false) {
+// MARKED: windows of up to 128 samples.
+template <typename T, bool MARKED = false>
+cudaError_t launch_robust_t(const Plan& p, const T* in, T* out, cudaStream_t s) {
   const int V = p.r.count;
-  if (V <= 32) return launch_robust_v<T, 32>(p, in, out, s, marked_only);
+  if (V <= 32) return launch_robust_v<T, 32, false, MARKED>(p, in, out, s);
   // Windows of 33-256 samples: runs sorted in registers and merged, except
   // for the clipping kinds, whose iterations run faster in the kernel
   // without it (fewer registers).
   const bool clip = p.robust.kind >= kRobustSigmaMean;
-  if (V <= 64) return clip ? launch_robust_v<T, 64, false>(p, in, out, s, marked_only) : launch_robust_v<T, 64, true>(p, in, out, s, marked_only);
+  if (V <= 64)
+    return clip ? launch_robust_v<T, 64, false, MARKED>(p, in, out, s) : launch_robust_v<T, 64, true, MARKED>(p, in, out, s);
   if (V <= 128)
-    return clip ? launch_robust_v<T, 128, false>(p, in, out, s, marked_only) : launch_robust_v<T, 128, true>(p, in, out, s, marked_only);
-  if (V <= 256)
-    return clip ? launch_robust_v<T, 256, false>(p, in, out, s, marked_only) : launch_robust_v<T, 256, true>(p, in, out, s, marked_only);
-  return launch_robust_v<T, 0>(p, in, out, s, marked_only);
+    return clip ? launch_robust_v<T, 128, false, MARKED>(p, in, out, s) : launch_robust_v<T, 128, true, MARKED>(p, in, out, s);
+  if constexpr (MARKED) {
+    return cudaErrorInvalidValue;
+  } else {
+    if (V <= 256)
+      return clip ? launch_robust_v<T, 256, false, false>(p, in, out, s) : launch_robust_v<T, 256, true, false>(p, in, out, s);
+    return launch_robust_v<T, 0, false, false>(p, in, out, s);
+  }
 }
 
 }  // namespace
