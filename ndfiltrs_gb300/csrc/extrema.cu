@@ -335,15 +335,19 @@ int strip_warps(size_t per_warp) {
 // after the other, about 0.6 us each at first, so arrays whose segments would be
 // shorter than twice the window (2.5 times for float64, whose shuffles are
 // double) are faster in passes (31 x 31 on 2000 x 1500: 0.041 against 0.033 ms), except
-// for the short walks of windows of up to 15 rows of float32. So are arrays that fill few
-// of a strip's 64 columns, where the passes' strips of 32 waste less (9 x 3 on 10^6 x 4:
-// 0.262 against 0.200 ms float32, 0.470 against 0.317 float64; on 10^6 x 24 0.263 against
-// 0.308, and 0.471 against 0.417); windows of one column, which need no shuffles, take
-// strips from 2 columns on (30 x 1 on 10^6 x 16: 0.219 against 0.302).
+// for the short walks of windows of up to 15 rows of float32. A float64 walk takes some
+// 25 to 33 us however short, which passes over less than 700,000 outputs undercut for
+// windows of 3 rows or more and up to 64 columns (3 x 54 on 800^2: 32.6 against 28.4,
+// on 300 x 3000 33.2 against 37.6). Passes are faster too over arrays that fill few of a
+// strip's 64 columns, where their strips of 32 waste less (9 x 3 on 10^6 x 4: 0.262
+// against 0.200 ms float32, 0.470 against 0.317 float64; on 10^6 x 24 0.263 against 0.308,
+// and 0.471 against 0.417); windows of one column, which need no shuffles, take strips
+// from 2 columns on (30 x 1 on 10^6 x 16: 0.219 against 0.302).
 int strip_rows(const Plan& p) {
   const Geom3& g = p.tile.g;
   if (g.kh > kStripMax || g.kw > kStripMax || (p.r.omit && p.r.min_count > 1)) return 0;
   if (g.W <= (g.kw == 1 ? 1 : p.dtype == 0 ? 15 : 32)) return 0;
+  if (p.dtype != 0 && p.n_out < 700000 && g.kh >= 3 && g.kw <= 64) return 0;
   const long long key = p.dtype == 0 ? 4 : 8;
   const long long strips = (g.W + kStripWidth - 1) / kStripWidth;
   const size_t per_warp = (size_t)(g.kh * kStripWidth * key);
