@@ -24,6 +24,7 @@
 #pragma once
 
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "moments.cuh"
@@ -36,7 +37,7 @@ constexpr int kRThreads = 128;
 // The output value that marks a window the tile kernel (robust_tile.cuh) left
 // to this one: a NaN whose payload no filter output holds.
 constexpr unsigned int kUndecided = 0x7FD5A11Cu;
-constexpr int kRobustChunk = 8;  // outputs whose marks a thread loads together
+constexpr int kRobustChunk = 16;  // outputs whose marks a thread loads together
 // Phi^-1(0.75), src/robust.rs:11.
 constexpr double kNormalUpperQuartile = 0.6744897501960817;
 
@@ -711,12 +712,21 @@ __global__ void __launch_bounds__(kRThreads)
   const long long stride = (long long)gridDim.x * blockDim.x;
   if constexpr (MARKED) {
     for (long long first = tid; first < a.n_out; first += kRobustChunk * stride) {
+      // All of a chunk in one batch of loads, and at most four of a thread that has no
+      // more (the array's last one is loaded for those beyond).
       unsigned int todo = 0;
+      auto look = [&](auto count) {
+        unsigned int mark[decltype(count)::value];
 #pragma unroll
-      for (int j = 0; j < kRobustChunk; ++j) {
-        const long long o = first + j * stride;
-        todo |= o < a.n_out && __float_as_uint(out[o]) == kUndecided ? 1u << j : 0u;
-      }
+        for (int j = 0; j < count; ++j) mark[j] = __float_as_uint(out[min(first + j * stride, a.n_out - 1)]);
+#pragma unroll
+        for (int j = 0; j < count; ++j)
+          todo |= mark[j] == kUndecided && first + j * stride < a.n_out ? 1u << j : 0u;
+      };
+      if (first + 4 * stride < a.n_out)
+        look(std::integral_constant<int, kRobustChunk>{});
+      else
+        look(std::integral_constant<int, 4>{});
       for (; todo; todo &= todo - 1) output(first + (__ffs((int)todo) - 1) * stride);
     }
   } else {
