@@ -264,9 +264,10 @@ __device__ __forceinline__ int clip_pass(const Column& s, int lo, int hi, const 
   int x = lo, y = hi;
   if (ra.spread == 1) {
     const F mad = mad_spread<F>(s, lo, hi, a, b);
-    if (mad == (F)0) {
-      // Zero spread: only samples equal to the center stay.
-      if (ra.center == 0) return 0;
+    // Zero spread: only samples equal to the center stay. About a mean the test below
+    // decides it where no sample is so close to the mean that it might equal it (data of
+    // few values, most of them alike).
+    if (mad == (F)0 && ra.center != 0) {
       while (x < hi && s[x] != a) ++x;
       while (y > x && s[y - 1] != a) --y;
       *new_lo = x;
