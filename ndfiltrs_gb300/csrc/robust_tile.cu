@@ -33,7 +33,7 @@ bool robust_tile_configure(Plan& p) {
   // block take 128. Tiles are 32 columns wide, narrower over arrays of fewer and
   // wider over arrays of few rows: 32 columns over one of 2 or 3 left the MAD
   // slower than one window per thread of the general kernel (5 x 5 x 1 over
-  // 400 x 400 x 3: 0.22 ms there, 0.32 in tiles of 32 columns, 0.17 in tiles of 4).
+  // 400 x 400 x 3: 0.22 ms there, 0.32 in tiles of 32 columns, 0.064 in tiles of 4).
   auto covering = [](long long n, int most) {
     int side = 1;
     while (side < n && side < most) side *= 2;

@@ -34,7 +34,7 @@
 //
 // Bound now by the min / max pipe of the sort and by the shared-memory loads
 // of the passes over the column. Measured with the filling-in pass (frames of
-// noise with outliers, NaN and infinities): MAD 5 x 5 on 4096^2 7.63 -> 0.74 ms
+// noise with outliers, NaN and infinities): MAD 5 x 5 on 4096^2 7.63 -> 0.71 ms
 // (0.91 with a few float64 operations per output, which cost a third of a 3 x 3
 // MAD), clipped mode 7 x 7 on 2048^2 30.7 -> 0.80 ms.
 #pragma once
@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(kT, min_blocks<N>())
   const bool drop_inf = clip || a.r.drop_inf;
   const uint32_t outside = sample_key<float>((float)a.r.cval, drop_inf);
   if (threadIdx.x == 0) lowest = INT_MAX;
-  if (!stage_tile(keys, maps, smem_raw, in, a, &tmap, z, y0, x0, outside,
+  if (!stage_tile<true>(keys, maps, smem_raw, in, a, &tmap, z, y0, x0, outside,
                   [&](float v) { return sample_key<float>(v, drop_inf); }))
     return;
   __syncthreads();
